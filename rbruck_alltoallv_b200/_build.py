@@ -36,6 +36,7 @@ CUDA_SOURCES = [
     "kernels/grouped_gemm_fp8_pair_sm100.cu",
     "kernels/grouped_gemm_mxfp8_sm100.cu",
     "kernels/fft_transpose.cu",
+    "kernels/reshard.cu",
     "kernels/noalloc.cu",
     "api/c_api.cu",
     "api/tuner_native.cpp",

@@ -79,6 +79,8 @@ def declare_cuda(lib):
     lib.rbv_ctx_set_eager.argtypes = [C.c_void_p, C.c_ulonglong]
     lib.rbv_ctx_set_cooperative.argtypes = [C.c_void_p, C.c_int]
     declare_moe(lib)
+    lib.rbv_reshard_heads.argtypes = [C.c_void_p, C.POINTER(C.c_void_p), C.POINTER(C.c_void_p), C.c_longlong,
+                                      C.c_longlong, C.c_int, C.c_void_p]
     lib.rbv_alltoallv_noalloc.argtypes = [C.c_int, C.c_int, C.POINTER(C.c_void_p), C.POINTER(C.c_void_p), C.c_void_p,
                                           C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]
     lib.rbv_noalloc_status.argtypes = [C.c_void_p]

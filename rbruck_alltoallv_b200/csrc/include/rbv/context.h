@@ -91,6 +91,7 @@ class Context {
   char* peer_heap(int q) const { return peer_[q]; }
   int max_ctas() const { return max_ctas_; }
   int sm_count() const { return sm_count_; }
+  StatusBlock* host_status_dev() const { return host_status_dev_; }   // where kernels note failures for the host
 
   cudaError_t ipc_handle(void* out64);
   cudaError_t connect(const void* handles);  // nproc x 64 bytes, in process order

@@ -113,6 +113,7 @@ class Communicator:
             raise CommError("context creation failed: " + self._lib.rbv_last_error().decode())
         self._lib.rbv_ctx_set_timeout_ms(self._ctx, float(timeout_ms))
         self._bulk = int(os.environ.get("RBV_BULK", "0"))
+        self.tracing = False     # calls prepared from now on report their phase time stamps (enable_trace)
         self._side = None
         if self.nproc > 1:
             self._side = dist.new_group(backend="gloo")
@@ -555,6 +556,7 @@ class Communicator:
     def enable_trace(self, on: bool = True) -> None:
         """Have every following call report its phase time stamps (``status()['phases_us']``)."""
         self._lib.rbv_ctx_set_trace(self._ctx, 1 if on else 0)
+        self.tracing = bool(on)
 
     def set_cooperative(self, mode) -> None:
         """Kernel launch mode: ``None`` / -1 cooperative only where a call needs all its CTAs resident (default),

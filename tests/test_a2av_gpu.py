@@ -491,6 +491,41 @@ def test_ulysses_sequence_head_exchange_round_trip():
         assert torch.equal(back[r], x[r])
 
 
+@pytest.mark.parametrize("P,s_l,H,D,dtype", [
+    (2, 1, 2, 1, torch.uint8),              # pieces of one byte
+    (3, 5, 3, 3, torch.bfloat16),           # pieces of 6 bytes
+    (4, 7, 8, 5, torch.float32),            # pieces of 40 bytes: 8-byte vectors
+    (8, 129, 16, 80, torch.bfloat16),       # rows that no tile divides
+    (16, 700, 16, 64, torch.bfloat16),      # several vectors per thread, a ragged last tile
+    (1, 33, 4, 8, torch.float64)])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_ulysses_both_directions_at_odd_sizes(P, s_l, H, D, dtype, offset):
+    """Plain tensors (one kernel), tensors that start at an odd element, strided tensors and views of the library's own
+    buffers (which take the packed exchange) all give the same bytes."""
+    from rbruck_alltoallv_b200.ops.ulysses import UlyssesExchange
+    ex = UlyssesExchange(get_comm(P), s_l, H, D, dtype=dtype)
+    n = s_l * H * D
+    x = []
+    for r in range(P):
+        raw = torch.randint(0, 120, (n + offset,), device="cuda", dtype=torch.uint8).to(dtype)
+        x.append(raw[offset:].view(s_l, H, D))
+    full = torch.cat(x, dim=0)
+    want = [full[:, r * (H // P):(r + 1) * (H // P), :] for r in range(P)]
+    got = [t.clone() for t in ex.seq_to_head(x)]
+    back = ex.head_to_seq(got)
+    again = ex.head_to_seq(ex.seq_to_head(x))                                            # views of the result buffers
+    strided = [t.permute(2, 0, 1).contiguous().permute(1, 2, 0) for t in got]            # same values, other strides
+    packed = ex.head_to_seq(strided)
+    ex.comm.check()
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+    for res in (back, again, packed):
+        assert all(torch.equal(a, b) for a, b in zip(res, x))
+    held = ex.seq_to_head(x)                                                             # overwritten while it is read
+    got = ex.seq_to_head([t.view(-1).view(s_l, H, D) for t in held])
+    flat = torch.cat([t.reshape(s_l, H, D) for t in want], dim=0)
+    assert all(torch.equal(got[r], flat[:, r * (H // P):(r + 1) * (H // P), :]) for r in range(P))
+
+
 def test_more_than_64_ranks_run_as_persistent_calls():
     """Up to 1024 logical ranks (the size of the reference's largest recorded trace) run through the static kernel,
     which keeps no per-rank tables; one-shot calls of such communicators are refused with a clear message."""
