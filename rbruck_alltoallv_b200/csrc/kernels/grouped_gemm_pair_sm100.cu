@@ -1,15 +1,21 @@
-// Grouped GEMM for the expert FFN on CTA PAIRS (tcgen05 cta_group::2): two CTAs on neighbouring SMs share one
-// 256 x 256 output tile.  Each CTA fetches its own 128 rows of A and its own half (128 of 256 rows) of the B tile, so a
-// k-block costs 32 KB of shared-memory fill per SM instead of the 48 KB of the one-CTA kernel
-// (grouped_gemm_sm100.cu) for the same number of MMAs: a third less traffic between L2 and the SMs, and a pipeline of
-// 6 stages instead of 4 in the same shared memory.  No counterpart exists in the reference (it has no compute kernels).
+// Grouped GEMM for the expert FFN on CTA PAIRS (tcgen05 cta_group::2), weights as the M operand and tokens as the N
+// operand.  Two CTAs on neighbouring SMs share one tile of 256 weight rows by up to 256 tokens.  Each CTA fetches its own
+// 128 weight rows and its own half of the tile's tokens, so a k-block of a full tile costs 32 KB of shared-memory fill
+// per SM.  No counterpart exists in the reference (it has no compute kernels).
 //
 //   C[rows of group g] = epilogue( A[rows of group g] (M_g x K, K-major) * B_g^T (N x K, K-major) )
 //
-// One persistent cluster of two CTAs per SM pair walks a static tile schedule (groups in order, n-major, m fastest):
-//   warp 0    TMA producer, in both CTAs (own A rows, own half of B; bytes counted on a barrier of the rank-0 CTA)
-//   warp 1    TMEM allocation in both CTAs; in the rank-0 CTA one elected thread issues the M256 N256 K16 MMAs
-//   warps 2-5 epilogue, in both CTAs (each drains the 128 accumulator rows in its own TMEM)
+// Why tokens are N: the M of an MMA is fixed (256 for a pair) while its N is any multiple of 32 up to 256, and the token
+// count is the ragged one.  A group of R rows costs ceil(R / 32) * 32 columns, cut into tiles of nearly equal size, where
+// tokens as M cost ceil(R / 256) * 256 rows: a group of 16 decoded tokens ran 16 times the MMAs it needed and fetched 16
+// times the token rows.  Measured on one B200, MoE layer of 8 experts, hidden 4096, FFN 14336: 64 tokens 660 -> 500 us
+// (HBM-bound now: every weight is read once), 8192 tokens 4.89 -> 4.86 ms (bound by the tensor cores under the power cap).
+//
+// One persistent cluster of two CTAs per SM pair walks a static tile schedule (groups in order, weight rows slow, tokens
+// fast, so the token tiles of one weight tile run at the same time and share it in L2):
+//   warp 0    TMA producer, in both CTAs (own weight rows, own half of the tokens; bytes counted in the rank-0 CTA)
+//   warp 1    TMEM allocation in both CTAs; in the rank-0 CTA one elected thread issues the M256 K16 MMAs
+//   warps 2-5 epilogue, in both CTAs (each drains the 128 weight rows in its own TMEM: a lane is an output column)
 // TMEM holds two 128 x 256 fp32 accumulators per CTA, so the epilogue of tile i overlaps the MMAs of tile i + 1.
 // TMA loads carry no cluster multicast.  All waits are bounded; on expiry both CTAs are told, record an error,
 // release their TMEM and return.
@@ -21,6 +27,7 @@
 #include <cstdlib>
 
 #include "kernels/sm100_ptx.cuh"
+#include "kernels/tok_epilogue.cuh"
 #include "rbv/moe.h"
 
 namespace rbv {
@@ -29,18 +36,21 @@ using namespace sm100;
 
 namespace {
 
-constexpr int PM = 256;            // tile rows per pair
-constexpr int HM = 128;            // rows per CTA
-constexpr int PN = 256;            // tile columns
-constexpr int HN = 128;            // rows of the B tile each CTA fetches
+constexpr int PM = 256;            // weight rows (output columns) per pair tile
+constexpr int HM = 128;            // weight rows per CTA
+constexpr int PT = 256;            // most tokens per tile
+constexpr int PU = 32;             // tokens per unit: a tile's token count is a multiple of this
 constexpr int PK = 64;             // one 128-byte swizzle atom of bf16
 constexpr int PSTAGES = 6;
-constexpr int PA_BYTES = HM * PK * 2;   // 16 KB
-constexpr int PB_BYTES = HN * PK * 2;   // 16 KB
-constexpr int PSTAGE_BYTES = PA_BYTES + PB_BYTES;
+constexpr int PW_BYTES = HM * PK * 2;        // 16 KB of weights
+constexpr int PT_BYTES = PT / 2 * PK * 2;    // up to 16 KB of tokens
+constexpr int PSTAGE_BYTES = PW_BYTES + PT_BYTES;
 constexpr int PAIR_THREADS = 192;
 constexpr int PAIR_TMEM_COLS = 512;
 constexpr size_t PAIR_SMEM = (size_t)PSTAGES * PSTAGE_BYTES + 1024 /*alignment slack*/;
+
+// Token boxes of 16, 32, 64 and 128 rows: a CTA's half of a tile is fetched with the smallest that covers it.
+struct PairMaps { CUtensorMap w, tok[4]; };
 
 struct PairParams {
   const int* group_start;
@@ -59,33 +69,39 @@ struct PairParams {
   char* heap[16];
 };
 
-struct PairTile { int m0, n0, b_row, rows; bool valid; };
+struct PairTile { int tok0, ntok, nt, n0, b_row; bool valid; };   // first token row, live tokens, columns, weight rows
 
-// Tile t of the pair schedule: groups in order; inside a group n-major, m fastest.  `rows` = rows of the group from m0 on.
-__device__ __forceinline__ PairTile pair_tile_of(const PairParams& p, int t, const int* s_rows, const int* s_start) {
-  const int ntn = p.N / PN;
-  PairTile r; r.valid = false; r.m0 = 0; r.n0 = 0; r.b_row = 0; r.rows = 0;
-  for (int g = 0; g < p.G; g++) {
-    const int ntm = (s_rows[g] + PM - 1) / PM;
-    const int cnt = ntm * ntn;
-    if (t < cnt) {
-      const int n = t / ntm, m = t - n * ntm;
-      r.m0 = s_start[g] + m * PM; r.n0 = n * PN; r.b_row = g * p.N + n * PN; r.rows = s_rows[g] - m * PM;
-      r.valid = true;
-      return r;
+// Walks the tile schedule; `at(t)` wants non-decreasing t.
+struct PairWalk {
+  int g = 0, before = 0;   // tiles of the groups in front of g
+  __device__ __forceinline__ PairTile at(const PairParams& p, int t, const int* s_rows, const int* s_start) {
+    PairTile r; r.valid = false; r.tok0 = r.ntok = r.nt = r.n0 = r.b_row = 0;
+    for (; g < p.G; g++) {
+      const int units = (s_rows[g] + PU - 1) / PU, ntm = (units + PT / PU - 1) / (PT / PU);
+      const int cnt = ntm * (p.N / PM);
+      if (t - before < cnt) {
+        const int n = (t - before) / ntm, m = (t - before) - n * ntm;
+        const int base = units / ntm, extra = units - base * ntm;     // the first `extra` tiles are one unit larger
+        const int u0 = m * base + min(m, extra), nu = base + (m < extra ? 1 : 0);
+        r.tok0 = s_start[g] + u0 * PU; r.nt = nu * PU; r.ntok = min(s_rows[g] - u0 * PU, r.nt);
+        r.n0 = n * PM; r.b_row = g * p.N + n * PM;
+        r.valid = true;
+        return r;
+      }
+      before += cnt;
     }
-    t -= cnt;
+    return r;
   }
-  return r;
-}
+};
 
-__device__ __forceinline__ float silu_f(float x) { return x / (1.0f + __expf(-x)); }
+// Index of the token box for `half` rows, and its rows.
+__device__ __forceinline__ int tok_box(int half) { return half <= 16 ? 0 : half <= 32 ? 1 : half <= 64 ? 2 : 3; }
+__device__ __forceinline__ uint32_t tok_box_bytes(int half) { return (16u << tok_box(half)) * PK * 2; }
 
 }  // namespace
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
-grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
-                         const PairParams p) {
+grouped_gemm_pair_kernel(const __grid_constant__ PairMaps maps, const __grid_constant__ PairParams p) {
   extern __shared__ uint8_t dyn_smem[];
   uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dyn_smem) + 1023) & ~uintptr_t(1023));
   __shared__ __align__(8) uint64_t full_bar[PSTAGES];    // used in the rank-0 CTA: bytes of both CTAs' loads
@@ -121,23 +137,25 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
   if (warp == 0) {
     // ---------------- TMA producer (both CTAs) ----------------
     if (elect_one()) {
-      tma_prefetch_desc(&tma_a);
-      tma_prefetch_desc(&tma_b);
+      tma_prefetch_desc(&maps.w);
       int stage = 0; uint32_t phase = 0;
       bool ok = true;
+      PairWalk walk;
       for (int t = pair; ok; t += npairs) {
-        const PairTile tl = pair_tile_of(p, t, s_rows, s_start);
+        const PairTile tl = walk.at(p, t, s_rows, s_start);
         if (!tl.valid) break;
-        const int a_row = tl.m0 + (int)rank * HM;
-        const int b_row = tl.b_row + (int)rank * HN;
+        const int half = tl.nt / 2;
+        const CUtensorMap* tok = &maps.tok[tok_box(half)];
+        const uint32_t bytes = 2u * (PW_BYTES + tok_box_bytes(half));
+        const int w_row = tl.b_row + (int)rank * HM;
+        const int t_row = tl.tok0 + (int)rank * half;
         for (int kb = 0; kb < num_kb; kb++) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag)) { ok = false; break; }
-          uint8_t* sa = tiles + (size_t)stage * PSTAGE_BYTES;
-          uint8_t* sb = sa + PA_BYTES;
-          if (leader) mbar_arrive_expect_tx(&full_bar[stage], 2 * PSTAGE_BYTES);
+          uint8_t* sw = tiles + (size_t)stage * PSTAGE_BYTES;
+          if (leader) mbar_arrive_expect_tx(&full_bar[stage], bytes);
           const uint32_t bar0 = mapa_u32(smem_u32(&full_bar[stage]), 0);
-          tma_load_2d_pair(sa, &tma_a, kb * PK, a_row, bar0);
-          tma_load_2d_pair(sb, &tma_b, kb * PK, b_row, bar0);
+          tma_load_2d_pair(sw, &maps.w, kb * PK, w_row, bar0);
+          tma_load_2d_pair(sw + PW_BYTES, tok, kb * PK, t_row, bar0);
           if (++stage == PSTAGES) { stage = 0; phase ^= 1u; }
         }
       }
@@ -146,26 +164,27 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
   } else if (warp == 1) {
     // ---------------- MMA issuer (rank-0 CTA only) ----------------
     if (leader && elect_one()) {
-      const uint32_t idesc = umma_idesc(PM, PN, 1 /*bf16*/);
       int stage = 0; uint32_t phase = 0;
       bool ok = true;
       int i = 0;
+      PairWalk walk;
       for (int t = pair; ok; t += npairs, i++) {
-        const PairTile tl = pair_tile_of(p, t, s_rows, s_start);
+        const PairTile tl = walk.at(p, t, s_rows, s_start);
         if (!tl.valid) break;
+        const uint32_t idesc = umma_idesc(PM, tl.nt, 1 /*bf16*/);
         const int b = i & 1;
         if (!mbar_wait(&tempty_bar[b], (((uint32_t)i >> 1) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
         tc_fence_after_sync();
-        const uint32_t d_tmem = tmem_base + (uint32_t)b * PN;
+        const uint32_t d_tmem = tmem_base + (uint32_t)b * PT;
         for (int kb = 0; kb < num_kb; kb++) {
           if (!mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
           tc_fence_after_sync();
-          const uint8_t* sa = tiles + (size_t)stage * PSTAGE_BYTES;
-          const uint64_t adesc = umma_desc_sw128(sa);
-          const uint64_t bdesc = umma_desc_sw128(sa + PA_BYTES);
+          const uint8_t* sw = tiles + (size_t)stage * PSTAGE_BYTES;
+          const uint64_t wdesc = umma_desc_sw128(sw);
+          const uint64_t tdesc = umma_desc_sw128(sw + PW_BYTES);
           #pragma unroll
           for (int kk = 0; kk < PK / 16; kk++)
-            umma_bf16_pair(d_tmem, adesc + 2u * kk, bdesc + 2u * kk, idesc, (uint32_t)((kb | kk) != 0));
+            umma_bf16_pair(d_tmem, wdesc + 2u * kk, tdesc + 2u * kk, idesc, (uint32_t)((kb | kk) != 0));
           umma_commit_pair(&empty_bar[stage]);   // frees this stage in both CTAs
           if (++stage == PSTAGES) { stage = 0; phase ^= 1u; }
         }
@@ -176,54 +195,35 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid
   } else {
     // ---------------- epilogue (both CTAs): warps 2..5, TMEM lane quarter = warp % 4 ----------------
     const int q = warp & 3;
-    const int row = q * 32 + lane;
     __nv_bfloat16* C = static_cast<__nv_bfloat16*>(p.C);
     bool ok = true;
     int i = 0;
+    PairWalk walk;
     for (int t = pair; ok; t += npairs, i++) {
-      const PairTile tl = pair_tile_of(p, t, s_rows, s_start);
+      const PairTile tl = walk.at(p, t, s_rows, s_start);
       if (!tl.valid) break;
       const int b = i & 1;
       if (!mbar_wait(&tfull_bar[b], ((uint32_t)i >> 1) & 1u, abort_flag)) { ok = false; break; }
       tc_fence_after_sync();
-      const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)b * PN;
-      const bool live = row < tl.rows - (int)rank * HM;
-      __nv_bfloat16* crow = C + (size_t)(tl.m0 + (int)rank * HM + row) * p.ldc;
-      if (p.ret && live) {
-        const unsigned rv = __ldg(p.ret + tl.m0 + (int)rank * HM + row);
-        crow = reinterpret_cast<__nv_bfloat16*>(p.heap[rv >> 24] + p.y2_off) + (size_t)(rv & 0xffffffu) * p.ldc;
-      }
+      const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)b * PT;
+      const int nw = tl.n0 + (int)rank * HM + q * 32;   // first of this warp's 32 columns
       #pragma unroll 1
-      for (int c = 0; c < PN; c += 32) {
+      for (int c = 0; c < tl.nt; c += PU) {
         uint32_t r[32];
         tmem_ld32(taddr + c, r);
+        unsigned rv = 0;   // push mode: where the token of this lane's index goes, handed out by shuffle
+        if (p.ret && c + lane < tl.ntok) rv = __ldg(p.ret + tl.tok0 + c + lane);
         tmem_ld_wait();
+        __nv_bfloat16* rows = C + (size_t)(tl.tok0 + c) * p.ldc;
         if (p.epilogue == 1) {
-          uint32_t o[8];
-          #pragma unroll
-          for (int j = 0; j < 8; j++) {
-            float g0 = __uint_as_float(r[4 * j]), u0 = __uint_as_float(r[4 * j + 1]);
-            float g1 = __uint_as_float(r[4 * j + 2]), u1 = __uint_as_float(r[4 * j + 3]);
-            __nv_bfloat162 v = __floats2bfloat162_rn(silu_f(g0) * u0, silu_f(g1) * u1);
-            o[j] = *reinterpret_cast<uint32_t*>(&v);
-          }
-          if (live) {
-            uint4* dst = reinterpret_cast<uint4*>(crow + (tl.n0 + c) / 2);
-            dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
-            dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
-          }
+          tokepi::store_swiglu(r, rows, p.ldc, nw / 2, tl.ntok - c, lane);
+        } else if (p.ret) {
+          tokepi::store_plain(r, [&](int tok) {
+            const unsigned to = __shfl_sync(0xffffffffu, rv, tok);
+            return reinterpret_cast<__nv_bfloat16*>(p.heap[to >> 24] + p.y2_off) + (size_t)(to & 0xffffffu) * p.ldc;
+          }, nw, tl.ntok - c, lane);
         } else {
-          uint32_t o[16];
-          #pragma unroll
-          for (int j = 0; j < 16; j++) {
-            __nv_bfloat162 v = __floats2bfloat162_rn(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
-            o[j] = *reinterpret_cast<uint32_t*>(&v);
-          }
-          if (live) {
-            uint4* dst = reinterpret_cast<uint4*>(crow + tl.n0 + c);
-            #pragma unroll
-            for (int j = 0; j < 4; j++) dst[j] = make_uint4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
-          }
+          tokepi::store_plain(r, [&](int tok) { return rows + (size_t)tok * p.ldc; }, nw, tl.ntok - c, lane);
         }
       }
       tc_fence_before_sync();
@@ -262,13 +262,13 @@ EncodeTiledFn pair_encode_fn() {
   return fn;
 }
 
-// [rows, K] bf16 row-major, box = 128 rows x 64 elements, 128-byte swizzle
-bool pair_make_map(CUtensorMap* m, const void* base, unsigned long long rows, unsigned long long K) {
+// [rows, K] bf16 row-major, box = box_rows x 64 elements, 128-byte swizzle
+bool pair_make_map(CUtensorMap* m, const void* base, unsigned long long rows, unsigned long long K, unsigned box_rows) {
   EncodeTiledFn fn = pair_encode_fn();
   if (!fn) return false;
   cuuint64_t dims[2] = {K, rows};
   cuuint64_t strides[1] = {K * 2};
-  cuuint32_t box[2] = {(cuuint32_t)PK, (cuuint32_t)HM};
+  cuuint32_t box[2] = {(cuuint32_t)PK, box_rows};
   cuuint32_t estr[2] = {1, 1};
   return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -295,7 +295,7 @@ static int launch_bf16_pair(const void* A, long long a_rows, const void* B, void
                             int max_ctas, void* cuda_stream, const unsigned* ret, const void* const* heaps, int nheaps,
                             unsigned long long y2_off) {
   using namespace rbv;
-  if (G < 1 || G > kMoeMaxGroups || N % PN || K % PK || a_rows < 1 || (ldc % 8)) return (int)cudaErrorInvalidValue;
+  if (G < 1 || G > kMoeMaxGroups || N % PM || K % PK || a_rows < 1 || (ldc % 8)) return (int)cudaErrorInvalidValue;
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C)) & 15)
     return (int)cudaErrorInvalidValue;
   if (ret && (epilogue != 0 || !heaps || nheaps < 1 || nheaps > 16 || (y2_off & 15))) return (int)cudaErrorInvalidValue;
@@ -306,9 +306,10 @@ static int launch_bf16_pair(const void* A, long long a_rows, const void* B, void
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
-  CUtensorMap ma, mb;
-  if (!pair_make_map(&ma, A, (unsigned long long)a_rows, (unsigned long long)K)) return (int)cudaErrorUnknown;
-  if (!pair_make_map(&mb, B, (unsigned long long)G * N, (unsigned long long)K)) return (int)cudaErrorUnknown;
+  PairMaps maps;
+  if (!pair_make_map(&maps.w, B, (unsigned long long)G * N, (unsigned long long)K, HM)) return (int)cudaErrorUnknown;
+  for (int i = 0; i < 4; i++)
+    if (!pair_make_map(&maps.tok[i], A, (unsigned long long)a_rows, (unsigned long long)K, 16u << i)) return (int)cudaErrorUnknown;
   PairParams p;
   p.group_start = group_start; p.group_rows = group_rows; p.G = G; p.N = N; p.K = K; p.ldc = ldc; p.C = C;
   p.error = error_flag; p.epilogue = epilogue;
@@ -322,7 +323,7 @@ static int launch_bf16_pair(const void* A, long long a_rows, const void* B, void
   }
   grid &= ~1;   // whole pairs
   if (grid < 2) return (int)cudaErrorInvalidValue;
-  grouped_gemm_pair_kernel<<<grid, PAIR_THREADS, PAIR_SMEM, static_cast<cudaStream_t>(cuda_stream)>>>(ma, mb, p);
+  grouped_gemm_pair_kernel<<<grid, PAIR_THREADS, PAIR_SMEM, static_cast<cudaStream_t>(cuda_stream)>>>(maps, p);
   return (int)cudaGetLastError();
 }
 

@@ -47,6 +47,36 @@ def test_grouped_gemm_matches_fp32(rows, N, K, pair):
     assert torch.all(out[M:] == 7.0), "rows beyond the last group must stay untouched"
 
 
+@pytest.mark.parametrize("swiglu", [False, True])
+@pytest.mark.parametrize("rows", [[1], [31, 32, 33], [0, 255, 0, 256, 257], [288, 1, 511], [513, 1025], [5] * 64])
+def test_grouped_gemm_token_tiles(rows, swiglu):
+    """Token counts at the edges of the pair kernel's units (32) and tiles (256).  Bound: bf16 rounding of the result
+    (2^-9 relative) plus fp32 accumulation of K = 192 products in another order (192 * 2^-24 of the sum of magnitudes)."""
+    from rbruck_alltoallv_b200.ops.moe import grouped_gemm
+    torch.manual_seed(len(rows) + sum(rows))
+    G, M, N, K = len(rows), sum(rows), 512, 192
+    A = torch.randn(M, K, device="cuda").to(torch.bfloat16)
+    B = (torch.randn(G, N, K, device="cuda") * 0.1).to(torch.bfloat16)
+    gs, gr = _groups(rows, "cuda")
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    n_out = N // 2 if swiglu else N
+    out = torch.full((M + 3, n_out), 7.0, dtype=torch.bfloat16, device="cuda")
+    grouped_gemm(A, B, gs, gr, out=out, swiglu=swiglu, error=err, pair=True)
+    torch.cuda.synchronize()
+    assert err.item() == 0 and torch.all(out[M:] == 7.0)
+    r0 = 0
+    for g, n in enumerate(rows):
+        a, w = A[r0:r0 + n].double(), B[g].double()
+        ref, mag = a @ w.t(), a.abs() @ w.abs().t()
+        slack = mag * 192 * 2.0 ** -24
+        if swiglu:   # silu(g) * u: |d/dg| <= 1.1 |u|, |d/du| <= |g|, and 2^-20 for the fast exponential and division
+            gate, up = ref[:, 0::2], ref[:, 1::2]
+            slack = 1.1 * up.abs() * slack[:, 0::2] + gate.abs() * slack[:, 1::2] + (gate * up).abs() * 2.0 ** -20
+            ref = torch.nn.functional.silu(gate) * up
+        assert ((out[r0:r0 + n].double() - ref).abs() <= ref.abs() * 2.0 ** -8 + slack + 1e-6).all(), f"group {g}"
+        r0 += n
+
+
 @pytest.mark.parametrize("pair", [False, True])
 def test_grouped_gemm_swiglu(pair):
     from rbruck_alltoallv_b200.ops.moe import grouped_gemm, pack_gate_up
@@ -214,6 +244,38 @@ def test_grouped_gemm_mxfp8_scale_paths(scales):
             got = out[r0:r0 + n].float()
             assert (got - ref).abs().max().item() <= 0.01 * ref.abs().max().item() + 1e-3, f"group {g} ({scales})"
     assert torch.all(out[~used] == 7.0), "rows between the groups must stay untouched"
+
+
+@pytest.mark.parametrize("swiglu", [False, True])
+@pytest.mark.parametrize("rows,N", [([1], 128), ([31, 32, 33], 256), ([127, 0, 128, 129], 384), ([160, 97, 300], 640)])
+def test_grouped_gemm_mxfp8_token_tiles(rows, N, swiglu):
+    """Token counts at the edges of the units (32) and tiles (128); N with and without a half-empty last tile.  The
+    operands are exact after quantisation, so the bound is bf16 rounding plus fp32 accumulation of K = 384 products."""
+    from rbruck_alltoallv_b200.ops.moe import (dequantize_rows_mxfp8, dequantize_weight_mxfp8, grouped_gemm_mxfp8,
+                                               quantize_rows_mxfp8, quantize_weight_mxfp8)
+    torch.manual_seed(sum(rows) + N)
+    G, K = len(rows), 384
+    gs, gr, total, start = _groups_aligned(rows, "cuda")
+    Aq, sfa = quantize_rows_mxfp8(torch.randn(total, K, device="cuda").to(torch.bfloat16))
+    Bq, sfb = quantize_weight_mxfp8(torch.randn(G, N, K, device="cuda") * 0.1)
+    A, B = dequantize_rows_mxfp8(Aq, sfa).double(), dequantize_weight_mxfp8(Bq, sfb).double()
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    n_out = N // 2 if swiglu else N
+    out = torch.full((total, n_out), 7.0, dtype=torch.bfloat16, device="cuda")
+    grouped_gemm_mxfp8(Aq, sfa, Bq, sfb, gs, gr, out=out, swiglu=swiglu, error=err)
+    torch.cuda.synchronize()
+    assert err.item() == 0
+    untouched = torch.ones(total, dtype=torch.bool, device="cuda")
+    for g, n in enumerate(rows):
+        a, w, r0 = A[start[g]:start[g] + n], B[g], start[g]
+        untouched[r0:r0 + n] = False
+        ref, slack = a @ w.t(), (a.abs() @ w.abs().t()) * 384 * 2.0 ** -24
+        if swiglu:
+            gate, up = ref[:, 0::2], ref[:, 1::2]
+            slack = 1.1 * up.abs() * slack[:, 0::2] + gate.abs() * slack[:, 1::2] + (gate * up).abs() * 2.0 ** -20
+            ref = torch.nn.functional.silu(gate) * up
+        assert ((out[r0:r0 + n].double() - ref).abs() <= ref.abs() * 2.0 ** -8 + slack + 1e-6).all(), f"group {g}"
+    assert torch.all(out[untouched] == 7.0), "rows between the groups must stay untouched"
 
 
 def test_grouped_gemm_mxfp8_refuses_unaligned_groups():
