@@ -30,6 +30,7 @@ CUDA_SOURCES = [
     "kernels/a2av_eager.cu",
     "kernels/a2av_static.cu",
     "kernels/moe_kernels.cu",
+    "kernels/moe_local.cu",
     "kernels/grouped_gemm_sm100.cu",
     "kernels/grouped_gemm_pair_sm100.cu",
     "kernels/grouped_gemm_fp8_sm100.cu",

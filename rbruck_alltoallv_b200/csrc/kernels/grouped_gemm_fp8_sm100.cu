@@ -285,14 +285,15 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_
 
 // Row-wise 1 x 128 quantisation of bf16 activations to e4m3: out[row, k] = x[row, k] / scale, scale = amax / 448.
 // Sixteen lanes per (row, 128-column block), eight bf16 (one 16-byte load) per lane, four blocks per half-warp in
-// flight before the first reduction; scales are stored transposed, [K / 128][rows].
+// flight before the first reduction; scales are stored transposed, [K / 128][rows].  `used` (optional, device): only
+// the first *used rows hold anything.
 __global__ void __launch_bounds__(256)
 quantize_rows_kernel(const __nv_bfloat16* __restrict__ x, long long rows, int K, int ldx, uint8_t* __restrict__ out,
-                     float* __restrict__ scale_t) {
+                     float* __restrict__ scale_t, const int* __restrict__ used) {
   constexpr int kUnroll = 4;
   const int lane16 = threadIdx.x & 15;
   const unsigned kblocks = (unsigned)(K / 128);
-  const unsigned nblk = (unsigned)(rows * kblocks);                       // < 2^31, checked by the caller
+  const unsigned nblk = (unsigned)((used ? min(rows, (long long)__ldg(used)) : rows) * kblocks);   // < 2^31, checked by the caller
   const unsigned groups = (gridDim.x * blockDim.x) >> 4;                  // half-warps in the grid
   const unsigned g0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 4;
   const unsigned which = g0 & 1u;   // the two half-warps of a warp take neighbouring blocks; the loop is warp-uniform
@@ -409,6 +410,11 @@ extern "C" int rbv_grouped_gemm_fp8(const void* A, const float* a_scale_t, long 
 
 extern "C" int rbv_quantize_rows_fp8(const void* x_bf16, long long rows, int K, int ldx, void* out_fp8, float* scale_t,
                                      void* cuda_stream) {
+  return rbv_quantize_used_rows_fp8(x_bf16, rows, nullptr, K, ldx, out_fp8, scale_t, cuda_stream);
+}
+
+extern "C" int rbv_quantize_used_rows_fp8(const void* x_bf16, long long rows, const int* used, int K, int ldx,
+                                          void* out_fp8, float* scale_t, void* cuda_stream) {
   using namespace rbv;
   if (K % 128 || rows < 1 || (ldx % 8) || (reinterpret_cast<uintptr_t>(x_bf16) & 15) ||
       (reinterpret_cast<uintptr_t>(out_fp8) & 7))
@@ -419,6 +425,6 @@ extern "C" int rbv_quantize_rows_fp8(const void* x_bf16, long long rows, int K, 
   if (grid > 148 * 8) grid = 148 * 8;
   if (grid < 1) grid = 1;
   quantize_rows_kernel<<<(int)grid, 256, 0, static_cast<cudaStream_t>(cuda_stream)>>>(
-      static_cast<const __nv_bfloat16*>(x_bf16), rows, K, ldx, static_cast<uint8_t*>(out_fp8), scale_t);
+      static_cast<const __nv_bfloat16*>(x_bf16), rows, K, ldx, static_cast<uint8_t*>(out_fp8), scale_t, used);
   return (int)cudaGetLastError();
 }

@@ -10,6 +10,7 @@
 #include <cstdint>
 
 #include "api/ctx_internal.h"
+#include "kernels/moe_router.cuh"
 #include "kernels/mx_quant.cuh"
 #include "kernels/primitives.cuh"
 #include "rbv/device_types.h"
@@ -31,44 +32,12 @@ __global__ void moe_route_kernel(const float* __restrict__ logits, int T, int E,
   const int lane = threadIdx.x & 31;
   const int warps = (gridDim.x * blockDim.x) >> 5;
   for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < T; t += warps) {
-    const float* row = logits + (size_t)t * E;
-    float v[kMoeMaxExperts / 32];
-    float mx = -INFINITY;
-    #pragma unroll
-    for (int j = 0; j < kMoeMaxExperts / 32; j++) {
-      int e = j * 32 + lane;
-      v[j] = e < E ? row[e] : -INFINITY;
-      mx = fmaxf(mx, v[j]);
-    }
-    #pragma unroll
-    for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    // top-2 by (value, lower index wins ties)
-    float best[2]; int bi[2];
-    #pragma unroll
-    for (int k = 0; k < 2; k++) {
-      float bv = -INFINITY; int be = 0x7fffffff;
-      #pragma unroll
-      for (int j = 0; j < kMoeMaxExperts / 32; j++) {
-        int e = j * 32 + lane;
-        bool taken = (k == 1 && e == bi[0]);
-        if (e < E && !taken && (v[j] > bv || (v[j] == bv && e < be))) { bv = v[j]; be = e; }
-      }
-      #pragma unroll
-      for (int o = 16; o; o >>= 1) {
-        float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-        int oe = __shfl_xor_sync(0xffffffffu, be, o);
-        if (ov > bv || (ov == bv && oe < be)) { bv = ov; be = oe; }
-      }
-      best[k] = bv; bi[k] = be;
-    }
-    // softmax probabilities of the two winners, renormalised: p_k / (p_0 + p_1)
-    const float p0 = __expf(best[0] - mx), p1 = __expf(best[1] - mx);
-    const float inv = 1.0f / (p0 + p1);
+    const Top2 top = route_token(logits + (size_t)t * E, E, lane);
     if (lane == 0) {
-      topk_idx[2 * t] = bi[0]; topk_idx[2 * t + 1] = bi[1];
-      topk_w[2 * t] = p0 * inv; topk_w[2 * t + 1] = p1 * inv;
-      atomicAdd(&s_hist[bi[0]], 1);
-      atomicAdd(&s_hist[bi[1]], 1);
+      topk_idx[2 * t] = top.e[0]; topk_idx[2 * t + 1] = top.e[1];
+      topk_w[2 * t] = top.w[0]; topk_w[2 * t + 1] = top.w[1];
+      atomicAdd(&s_hist[top.e[0]], 1);
+      atomicAdd(&s_hist[top.e[1]], 1);
     }
   }
   __syncthreads();

@@ -1,0 +1,309 @@
+// MoE router, dispatch and combine of a communicator with one rank: the experts of every token live on this GPU, so
+// there is no histogram to gather and nobody to wait for; the end of a kernel is its completion.
+//
+//   route     softmax + top-2, the row's place among its expert's rows, and (by the last CTA to finish) the layout
+//   dispatch  every token is read once and stored to the rows of its two experts, as bf16, MXFP8 or block-scaled fp8
+//   combine   gate-weighted sum of a token's two result rows
+//
+// A layer call over a handful of tokens is a chain of launches and of memory latencies: the general path takes a memset,
+// a router, a one-CTA exchange of the histogram with itself, a one-CTA layout kernel, and one warp per row that first
+// draws its place from a counter and then walks the whole row.  Here places are drawn while routing, rows are cut into
+// pieces so that a few tokens already occupy every SM, and a piece is requested from memory before its place is known.
+#include <cuda_bf16.h>
+#include <cuda_fp8.h>
+#include <cuda_runtime.h>
+
+#include <cstdint>
+
+#include "api/ctx_internal.h"
+#include "kernels/moe_router.cuh"
+#include "kernels/mx_quant.cuh"
+#include "kernels/primitives.cuh"
+#include "rbv/device_types.h"
+#include "rbv/moe.h"
+
+namespace rbv {
+namespace {
+
+constexpr int kRouteWarps = 8;
+
+struct RouteLocalArgs {
+  const float* logits;
+  int T, E, align;
+  int* topk_idx;            // [T, 2]
+  float* topk_w;            // [T, 2]
+  int* place;               // [T, 2]: index of the row among its expert's rows
+  int* scratch;             // [E + 1], zero on entry, left zero: rows per expert, CTAs that have finished
+  int *dst_base, *group_start, *group_rows, *totals;
+  char* heap[kMaxProcs];    // for the failure note only
+  unsigned long long ctrl_off;
+  StatusBlock* host_status;
+};
+
+// One warp per token.
+__global__ void __launch_bounds__(kRouteWarps * 32) moe_route_local_kernel(const __grid_constant__ RouteLocalArgs a) {
+  __shared__ int s_rows[kMoeMaxExperts], s_base[kMoeMaxExperts];
+  __shared__ int s_last;
+  const int tid = threadIdx.x, lane = tid & 31;
+  for (int i = tid; i < a.E; i += blockDim.x) s_rows[i] = 0;
+  __syncthreads();
+  const int t = blockIdx.x * kRouteWarps + (tid >> 5);
+  Top2 top{};
+  int at0 = 0, at1 = 0;
+  if (t < a.T) {
+    top = route_token(a.logits + (size_t)t * a.E, a.E, lane);
+    if (lane == 0) {
+      at0 = atomicAdd(&s_rows[top.e[0]], 1);
+      at1 = atomicAdd(&s_rows[top.e[1]], 1);
+    }
+  }
+  __syncthreads();
+  for (int i = tid; i < a.E; i += blockDim.x)
+    if (s_rows[i]) s_base[i] = atomicAdd(&a.scratch[i], s_rows[i]);
+  __syncthreads();
+  if (t < a.T && lane == 0) {
+    reinterpret_cast<int2*>(a.topk_idx)[t] = make_int2(top.e[0], top.e[1]);
+    reinterpret_cast<float2*>(a.topk_w)[t] = make_float2(top.w[0], top.w[1]);
+    reinterpret_cast<int2*>(a.place)[t] = make_int2(s_base[top.e[0]] + at0, s_base[top.e[1]] + at1);
+  }
+  if (tid == 0) {
+    __threadfence();
+    s_last = atomicAdd(&a.scratch[a.E], 1) == (int)gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  // layout: the experts' rows one after the other, each expert starting at a multiple of `align` rows
+  __threadfence();
+  for (int e = tid; e < a.E; e += blockDim.x) {
+    s_rows[e] = __ldcg(&a.scratch[e]);
+    a.scratch[e] = 0;
+  }
+  __syncthreads();
+  for (int e = tid; e < a.E; e += blockDim.x) {
+    int base = 0;
+    for (int e2 = 0; e2 < e; e2++) base += (s_rows[e2] + a.align - 1) / a.align * a.align;
+    a.dst_base[e] = base;
+    a.group_start[e] = base;
+    a.group_rows[e] = s_rows[e];
+  }
+  if (tid == 0) {
+    a.scratch[a.E] = 0;
+    a.totals[0] = a.totals[1] = 2 * a.T;
+    // like every call on a communicator that failed earlier and was not reset, say so
+    CtrlBlock* my = reinterpret_cast<CtrlBlock*>(a.heap[0] + a.ctrl_off);
+    if (dev::ld_relaxed_sys(&my->abort_flag))
+      dev::note_failure(a.heap, 1, 0, a.ctrl_off, a.host_status, RBV_ERR_ABORTED, 0, 0, 0);
+  }
+}
+
+enum { ROWS_BF16 = 0, ROWS_MX = 1, ROWS_FP8 = 2 };
+
+struct DispatchLocalArgs {
+  const uint4* x;           // [T, H] bf16
+  int T, H, segs;           // segs: pieces per row
+  const int* topk_idx;
+  const int* place;
+  const int* dst_base;
+  int* slot;                // [T, 2] out: the rows
+  unsigned* ret;            // optional: return address of every row (token * 2 + k)
+  void* rows;               // [capacity, H] bf16 or e4m3
+  void* scales;             // MXFP8: words in atom order [H / 128][capacity / 128][128]; fp8: fp32 [H / 128][capacity]
+  int capacity;
+  int* error;
+};
+
+// One warp per (token, piece of U * 256 columns).
+template <int MODE, int U>
+__global__ void __launch_bounds__(128) moe_dispatch_local_kernel(const __grid_constant__ DispatchLocalArgs a) {
+  const int lane = threadIdx.x & 31;
+  const long long item = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
+  const int t = (int)(item / a.segs), seg = (int)(item - (long long)t * a.segs);
+  if (t >= a.T) return;
+  const int nvec = a.H / 8, first = seg * (U * 32) + lane;
+  uint4 raw[U];
+  #pragma unroll
+  for (int u = 0; u < U; u++) {
+    raw[u] = make_uint4(0u, 0u, 0u, 0u);
+    if (first + u * 32 < nvec) raw[u] = __ldg(a.x + (size_t)t * nvec + first + u * 32);
+  }
+  const int2 e = reinterpret_cast<const int2*>(a.topk_idx)[t], at = reinterpret_cast<const int2*>(a.place)[t];
+  const int pos[2] = {a.dst_base[e.x] + at.x, a.dst_base[e.y] + at.y};
+  const bool fits[2] = {pos[0] < a.capacity, pos[1] < a.capacity};
+  if (seg == 0 && lane < 2) {
+    const int k = lane;
+    a.slot[2 * t + k] = k ? pos[1] : pos[0];
+    if (!(k ? fits[1] : fits[0])) atomicCAS(a.error, 0, (4 << 8) | ((k ? e.y : e.x) & 0xff));
+    else if (a.ret) a.ret[k ? pos[1] : pos[0]] = (unsigned)(2 * t + k);
+  }
+  #pragma unroll
+  for (int u = 0; u < U; u++) {
+    const int vec = first + u * 32;
+    const bool in = vec < nvec;
+    if (MODE == ROWS_BF16) {
+      uint4* rows = static_cast<uint4*>(a.rows);
+      #pragma unroll
+      for (int k = 0; k < 2; k++)
+        if (in && fits[k]) rows[(size_t)pos[k] * nvec + vec] = raw[u];
+      continue;
+    }
+    // quantised where it is read, exactly as rbv_quantize_rows_mxfp8 / rbv_quantize_rows_fp8 do: a lane holds 8 columns,
+    // 4 lanes a block of 32, 16 lanes a block of 128
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw[u]);
+    float2 v[4];
+    float m = 0.0f;
+    #pragma unroll
+    for (int j = 0; j < 4; j++) {
+      v[j] = __bfloat1622float2(h[j]);
+      m = fmaxf(m, fmaxf(fabsf(v[j].x), fabsf(v[j].y)));
+    }
+    m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
+    m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
+    float inv;
+    unsigned word = 0;
+    float scale = 0.0f;
+    if (MODE == ROWS_MX) {
+      const int ex = mx_exponent(m);
+      inv = mx_inv_scale(ex);
+      word = (unsigned)(ex + 127) << (8 * ((lane & 15) >> 2));
+      word |= __shfl_xor_sync(0xffffffffu, word, 4);
+      word |= __shfl_xor_sync(0xffffffffu, word, 8);
+    } else {
+      m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 4));
+      m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 8));
+      scale = m > 0.0f ? m / 448.0f : 1.0f;
+      inv = 1.0f / scale;
+    }
+    unsigned q[4];
+    #pragma unroll
+    for (int j = 0; j < 4; j++)
+      q[j] = __nv_cvt_float2_to_fp8x2(make_float2(v[j].x * inv, v[j].y * inv), __NV_SATFINITE, __NV_E4M3);
+    #pragma unroll
+    for (int k = 0; k < 2; k++) {
+      if (!in || !fits[k]) continue;
+      const size_t r = (size_t)pos[k];
+      static_cast<uint2*>(a.rows)[r * nvec + vec] = make_uint2(q[0] | (q[1] << 16), q[2] | (q[3] << 16));
+      if ((lane & 15) == 0) {
+        const size_t kb = (size_t)(vec / 16);
+        if (MODE == ROWS_MX)
+          static_cast<unsigned*>(a.scales)[(kb * (size_t)(a.capacity / 128) + r / 128) * 128 + (r % 32) * 4 + (r % 128) / 32] = word;
+        else
+          static_cast<float*>(a.scales)[kb * (size_t)a.capacity + r] = scale;
+      }
+    }
+  }
+}
+
+struct CombineLocalArgs {
+  uint4* out;               // [T, H] bf16
+  const uint4* y;           // result rows of H bf16
+  int T, H, segs;
+  const int* slot;          // [T, 2] rows of y, or null: rows 2 t and 2 t + 1
+  const float* topk_w;
+};
+
+// One warp per (token, piece of U * 256 columns): all loads of a piece before its first store.
+template <int U>
+__global__ void __launch_bounds__(128) moe_combine_local_kernel(const __grid_constant__ CombineLocalArgs a) {
+  const int lane = threadIdx.x & 31;
+  const long long item = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
+  const int t = (int)(item / a.segs), seg = (int)(item - (long long)t * a.segs);
+  if (t >= a.T) return;
+  const int nvec = a.H / 8, first = seg * (U * 32) + lane;
+  const int2 row = a.slot ? reinterpret_cast<const int2*>(a.slot)[t] : make_int2(2 * t, 2 * t + 1);
+  const float2 w = reinterpret_cast<const float2*>(a.topk_w)[t];
+  uint4 r[2][U];
+  #pragma unroll
+  for (int u = 0; u < U; u++)
+    if (first + u * 32 < nvec) {
+      r[0][u] = dev::ld_cg_v4(a.y + (size_t)row.x * nvec + first + u * 32);
+      r[1][u] = dev::ld_cg_v4(a.y + (size_t)row.y * nvec + first + u * 32);
+    }
+  #pragma unroll
+  for (int u = 0; u < U; u++)
+    if (first + u * 32 < nvec) {
+      const __nv_bfloat162* h0 = reinterpret_cast<const __nv_bfloat162*>(&r[0][u]);
+      const __nv_bfloat162* h1 = reinterpret_cast<const __nv_bfloat162*>(&r[1][u]);
+      uint4 v;
+      __nv_bfloat162* o = reinterpret_cast<__nv_bfloat162*>(&v);
+      #pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const float2 f0 = __bfloat1622float2(h0[j]), f1 = __bfloat1622float2(h1[j]);
+        o[j] = __floats2bfloat162_rn(fmaf(w.y, f1.x, fmaf(w.x, f0.x, 0.0f)), fmaf(w.y, f1.y, fmaf(w.x, f0.y, 0.0f)));
+      }
+      a.out[(size_t)t * nvec + first + u * 32] = v;
+    }
+}
+
+// Pieces of 1024 columns (four 16-byte loads in flight per lane and operand) once they make 16 warps per SM, pieces of
+// 256 columns below that, where latency and idle SMs count and not bytes in flight.
+bool long_pieces(int T, int H, int sms) { return (long long)T * ((H + 1023) / 1024) >= 16ll * sms; }
+unsigned piece_grid(int T, int H, bool lng, int* segs) {
+  *segs = (H + (lng ? 1023 : 255)) / (lng ? 1024 : 256);
+  return (unsigned)(((long long)T * *segs + 3) / 4);
+}
+
+bool one_rank(rbv_ctx_t ctx) { return ctx && ctx->c && ctx->c->nproc() == 1 && ctx->c->P() == 1; }
+
+}  // namespace
+}  // namespace rbv
+
+using namespace rbv;
+
+extern "C" {
+
+int rbv_moe_route_local(rbv_ctx_t ctx, const float* logits, int T, int E, int align, int* topk_idx, float* topk_w,
+                        int* place, int* scratch, int* dst_base, int* group_start, int* group_rows, int* totals,
+                        void* stream) {
+  if (!one_rank(ctx) || E < 2 || E > kMoeMaxExperts || align < 1 || T < 1) return (int)cudaErrorInvalidValue;
+  const Context& c = *ctx->c;
+  RouteLocalArgs a{};
+  a.logits = logits; a.T = T; a.E = E; a.align = align;
+  a.topk_idx = topk_idx; a.topk_w = topk_w; a.place = place; a.scratch = scratch;
+  a.dst_base = dst_base; a.group_start = group_start; a.group_rows = group_rows; a.totals = totals;
+  a.heap[0] = c.heap(); a.ctrl_off = c.layout().ctrl_off; a.host_status = c.host_status_dev();
+  moe_route_local_kernel<<<(T + kRouteWarps - 1) / kRouteWarps, kRouteWarps * 32, 0, static_cast<cudaStream_t>(stream)>>>(a);
+  return (int)cudaGetLastError();
+}
+
+int rbv_moe_dispatch_local(rbv_ctx_t ctx, const void* x, int T, int H, const int* topk_idx, const int* place,
+                           const int* dst_base, int* slot, unsigned* ret, int format, void* rows, void* scales,
+                           long long capacity_rows, int* error_flag, void* stream) {
+  if (!one_rank(ctx) || T < 1 || 2ll * T >= (1ll << 24) || H % 8 || capacity_rows > 0x7fffffffll) return (int)cudaErrorInvalidValue;
+  if (format != ROWS_BF16 && (H % 128 || !scales)) return (int)cudaErrorInvalidValue;
+  if (format == ROWS_MX && capacity_rows % 128) return (int)cudaErrorInvalidValue;
+  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(rows)) & 15) return (int)cudaErrorMisalignedAddress;
+  DispatchLocalArgs a;
+  a.x = static_cast<const uint4*>(x); a.T = T; a.H = H;
+  a.topk_idx = topk_idx; a.place = place; a.dst_base = dst_base; a.slot = slot; a.ret = ret;
+  a.rows = rows; a.scales = scales; a.capacity = (int)capacity_rows; a.error = error_flag;
+  const bool lng = long_pieces(T, H, ctx->c->sm_count());
+  const unsigned grid = piece_grid(T, H, lng, &a.segs);
+  const cudaStream_t st = static_cast<cudaStream_t>(stream);
+#define RBV_LAUNCH(MODE) \
+  if (lng) moe_dispatch_local_kernel<MODE, 4><<<grid, 128, 0, st>>>(a); else moe_dispatch_local_kernel<MODE, 1><<<grid, 128, 0, st>>>(a)
+  switch (format) {
+    case ROWS_BF16: RBV_LAUNCH(ROWS_BF16); break;
+    case ROWS_MX: RBV_LAUNCH(ROWS_MX); break;
+    case ROWS_FP8: RBV_LAUNCH(ROWS_FP8); break;
+    default: return (int)cudaErrorInvalidValue;
+  }
+#undef RBV_LAUNCH
+  return (int)cudaGetLastError();
+}
+
+int rbv_moe_combine_local(rbv_ctx_t ctx, void* out, int T, int H, const int* slot, const float* topk_w, const void* y,
+                          void* stream) {
+  if (!one_rank(ctx) || T < 1 || H % 8) return (int)cudaErrorInvalidValue;
+  if ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(y)) & 15) return (int)cudaErrorMisalignedAddress;
+  CombineLocalArgs a;
+  a.out = static_cast<uint4*>(out); a.y = static_cast<const uint4*>(y); a.T = T; a.H = H;
+  a.slot = slot; a.topk_w = topk_w;
+  const bool lng = long_pieces(T, H, ctx->c->sm_count());
+  const unsigned grid = piece_grid(T, H, lng, &a.segs);
+  const cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (lng) moe_combine_local_kernel<4><<<grid, 128, 0, st>>>(a);
+  else moe_combine_local_kernel<1><<<grid, 128, 0, st>>>(a);
+  return (int)cudaGetLastError();
+}
+
+}  // extern "C"

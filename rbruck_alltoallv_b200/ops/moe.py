@@ -60,15 +60,16 @@ def grouped_gemm(A: torch.Tensor, B: torch.Tensor, group_start: torch.Tensor, gr
     return out
 
 
-def quantize_rows_fp8(x: torch.Tensor):
-    """bf16 [rows, K] -> (e4m3 bytes [rows, K], scales [K // 128, rows]); one scale per row and 128-wide K block."""
+def quantize_rows_fp8(x: torch.Tensor, used: Optional[torch.Tensor] = None):
+    """bf16 [rows, K] -> (e4m3 bytes [rows, K], scales [K // 128, rows]); one scale per row and 128-wide K block.  With
+    ``used`` (int32 CUDA tensor) only the first ``used[0]`` rows are quantised, the others are left undefined."""
     lib = _native.cuda_lib()
     assert x.dtype == torch.bfloat16 and x.dim() == 2 and x.stride(1) == 1 and x.shape[1] % 128 == 0
     rows, K = x.shape
     q = torch.empty(rows, K, dtype=torch.uint8, device=x.device)
     sc = torch.empty(K // 128, rows, dtype=torch.float32, device=x.device)
     st = torch.cuda.current_stream(x.device).cuda_stream
-    rc = lib.rbv_quantize_rows_fp8(_p(x), rows, K, x.stride(0), _p(q), _p(sc), C.c_void_p(st))
+    rc = lib.rbv_quantize_used_rows_fp8(_p(x), rows, _p(used), K, x.stride(0), _p(q), _p(sc), C.c_void_p(st))
     if rc:
         raise RuntimeError(f"quantisation launch failed (CUDA error {rc})")
     return q, sc
@@ -323,6 +324,11 @@ class MoEExpertParallel:
         self.group_rows = torch.zeros(self.El, dtype=i32, device=dev)
         self.totals = torch.zeros(2, dtype=i32, device=dev)
         self.error = torch.zeros(4, dtype=i32, device=dev)
+        self.place = torch.empty(tokens, 2, dtype=i32, device=dev)             # one rank: see _route_and_dispatch_local
+        self.route_scratch = torch.zeros(self.E + 1, dtype=i32, device=dev)
+        if self.P == 1 and self.fp8 and not self.mx and hidden % 128 == 0:
+            self.xq8 = torch.empty(self.cap, hidden, dtype=torch.uint8, device=dev)
+            self.xs8 = torch.empty(hidden // 128, self.cap, dtype=torch.float32, device=dev)
         # Streamed dispatch (bf16 path): rows travel expert by expert, every landed row bumps its expert's counter on
         # the owner, and the first grouped GEMM, launched on a second stream next to the dispatch, starts an expert as
         # soon as its rows are complete.  Opt-in (``overlap=True`` or RBV_MOE_OVERLAP=1): measured on B200 with the
@@ -378,26 +384,17 @@ class MoEExpertParallel:
         st = C.c_void_p(torch.cuda.current_stream(self.dev).cuda_stream)
         if out is None:
             out = torch.empty_like(x)
-        self._check(lib.rbv_moe_route(_p(logits), T, self.E, _p(self.topk_idx), _p(self.topk_w), _p(self.hist), st),
-                    "router")
-        self._gather.launch()
-        if self.overlap:
-            return self._forward_streamed(x, out, st)
-        # the MXFP8 GEMM wants every expert's rows to start at a multiple of 128 rows (its scale atoms)
-        self._check(lib.rbv_moe_layout_aligned(_p(self.hist_all), self.P, self.E, self.me, _p(self.dst_base),
-                                               _p(self.group_start), _p(self.group_rows), _p(self.cursor),
-                                               _p(self.totals), 128 if self.mx else 1, st), "layout")
-        if self.qdispatch:
-            self._check(lib.rbv_moe_dispatch_mx(ctx, _p(x), T, H, _p(self.topk_idx), _p(self.dst_base),
-                                                _p(self.cursor), _p(self.slot), self.xrecv_off, self.sfrow_off,
-                                                self.ret_off if self.push else 0, self.cap, self.E,
-                                                _p(self.error[0:1]), st), "dispatch")
-            self._check(lib.rbv_moe_scale_atoms(_p(self.sfrow), _p(self.xs), self.cap, H // 128, st), "scale layout")
+        local = self.P == 1 and not self.overlap
+        fp8_rows = None
+        if local:
+            fp8_rows = self._route_and_dispatch_local(x, logits, st)
         else:
-            self._check(lib.rbv_moe_dispatch_ret(ctx, _p(x), T, H, _p(self.topk_idx), _p(self.dst_base),
-                                                 _p(self.cursor), _p(self.slot), self.xrecv_off,
-                                                 self.ret_off if self.push else 0, self.cap, self.E,
-                                                 _p(self.error[0:1]), st), "dispatch")
+            self._check(lib.rbv_moe_route(_p(logits), T, self.E, _p(self.topk_idx), _p(self.topk_w), _p(self.hist), st),
+                        "router")
+            self._gather.launch()
+            if self.overlap:
+                return self._forward_streamed(x, out, st)
+            self._layout_and_dispatch(x, st)
         if self.mx:
             # activations are quantised once (by the dispatch, or here); the first GEMM's epilogue (SwiGLU) hands the
             # second GEMM its operand already quantised, so the bf16 intermediate never exists
@@ -422,11 +419,11 @@ class MoEExpertParallel:
                 grouped_gemm_mxfp8(hq, hs, self.w2_q, self.w2_s, self.group_start, self.group_rows, out=self.y,
                                    error=self.error[2:3])
         elif self.fp8:
-            # activations are quantised row-wise (1 x 128 blocks) right before each GEMM
-            xq, xs = quantize_rows_fp8(self.xrecv)
+            # activations are quantised row-wise (1 x 128 blocks), by the dispatch or right before each GEMM
+            xq, xs = fp8_rows or quantize_rows_fp8(self.xrecv, self.totals)
             grouped_gemm_fp8(xq, xs, self.w13_q, self.w13_s, self.group_start, self.group_rows, out=self.h, swiglu=True,
                              error=self.error[1:2])
-            hq, hs = quantize_rows_fp8(self.h)
+            hq, hs = quantize_rows_fp8(self.h, self.totals)
             grouped_gemm_fp8(hq, hs, self.w2_q, self.w2_s, self.group_start, self.group_rows, out=self.y,
                              error=self.error[2:3])
         else:
@@ -439,13 +436,54 @@ class MoEExpertParallel:
             else:
                 grouped_gemm(self.h, self.w2, self.group_start, self.group_rows, out=self.y, swiglu=False,
                              error=self.error[2:3])
-        if self.push:
+        if local:
+            self._check(lib.rbv_moe_combine_local(ctx, _p(out), T, H, None if self.push else _p(self.slot),
+                                                  _p(self.topk_w), _p(self.y2 if self.push else self.y), st), "combine")
+        elif self.push:
             self._check(lib.rbv_moe_combine_pushed(ctx, _p(out), T, H, _p(self.topk_w), _p(self.y2),
                                                    _p(self.error[3:4]), st), "combine")
         else:
             self._check(lib.rbv_moe_combine(ctx, _p(out), T, H, _p(self.topk_idx), _p(self.topk_w), _p(self.slot),
                                             self.y_off, self.E, _p(self.error[3:4]), st), "combine")
         return out
+
+    def _layout_and_dispatch(self, x, st):
+        lib, ctx, T, H = self.lib, self.comm._ctx, self.T, self.H
+        # the MXFP8 GEMM wants every expert's rows to start at a multiple of 128 rows (its scale atoms)
+        self._check(lib.rbv_moe_layout_aligned(_p(self.hist_all), self.P, self.E, self.me, _p(self.dst_base),
+                                               _p(self.group_start), _p(self.group_rows), _p(self.cursor),
+                                               _p(self.totals), 128 if self.mx else 1, st), "layout")
+        if self.qdispatch:
+            self._check(lib.rbv_moe_dispatch_mx(ctx, _p(x), T, H, _p(self.topk_idx), _p(self.dst_base),
+                                                _p(self.cursor), _p(self.slot), self.xrecv_off, self.sfrow_off,
+                                                self.ret_off if self.push else 0, self.cap, self.E,
+                                                _p(self.error[0:1]), st), "dispatch")
+            self._check(lib.rbv_moe_scale_atoms(_p(self.sfrow), _p(self.xs), self.cap, H // 128, st), "scale layout")
+        else:
+            self._check(lib.rbv_moe_dispatch_ret(ctx, _p(x), T, H, _p(self.topk_idx), _p(self.dst_base),
+                                                 _p(self.cursor), _p(self.slot), self.xrecv_off,
+                                                 self.ret_off if self.push else 0, self.cap, self.E,
+                                                 _p(self.error[0:1]), st), "dispatch")
+
+    def _route_and_dispatch_local(self, x, logits, st):
+        """Router, layout and dispatch with every expert on this GPU (``csrc/kernels/moe_local.cu``): two launches.  Rows
+        leave the dispatch in the format the first GEMM reads; returns them and their scales for block-scaled fp8."""
+        lib, ctx, T, H = self.lib, self.comm._ctx, self.T, self.H
+        if x.data_ptr() % 16:                 # a view that starts inside a 16-byte vector
+            x = x.clone()
+        self._check(lib.rbv_moe_route_local(ctx, _p(logits), T, self.E, 128 if self.mx else 1, _p(self.topk_idx),
+                                            _p(self.topk_w), _p(self.place), _p(self.route_scratch), _p(self.dst_base),
+                                            _p(self.group_start), _p(self.group_rows), _p(self.totals), st), "router")
+        if self.qdispatch:
+            fmt, rows, scales = 1, self.xq, self.xs
+        elif self.fp8 and not self.mx and H % 128 == 0:
+            fmt, rows, scales = 2, self.xq8, self.xs8
+        else:
+            fmt, rows, scales = 0, self.xrecv, None
+        self._check(lib.rbv_moe_dispatch_local(ctx, _p(x), T, H, _p(self.topk_idx), _p(self.place), _p(self.dst_base),
+                                               _p(self.slot), _p(self.ret) if self.push else None, fmt, _p(rows),
+                                               _p(scales), self.cap, _p(self.error[0:1]), st), "dispatch")
+        return (rows, scales) if fmt == 2 else None
 
     def _forward_streamed(self, x, out, st):
         lib, ctx, T, H = self.lib, self.comm._ctx, self.T, self.H

@@ -489,3 +489,46 @@ def test_moe_layer_streamed_dispatch_matches_reference(overlap):
             assert (out.float() - ref).abs().max().item() <= 0.02 * ref.abs().max().item() + 1e-3, (overlap, rep)
     finally:
         comm.close()
+
+
+@pytest.mark.parametrize("fp8", [False, True, "mx"], ids=["bf16", "fp8", "mxfp8"])
+@pytest.mark.parametrize("tokens,hidden,experts", [(1, 128, 2), (7, 384, 4), (129, 1152, 8), (2500, 1024, 64)])
+def test_moe_one_rank_route_and_dispatch(tokens, hidden, experts, fp8):
+    """Places, layout and rows of the one-rank kernels against torch: every routed row in its expert's range, once, in the
+    format the GEMM reads (the separate quantisers are the oracle), with ties in the logits and a view that starts at an
+    odd element."""
+    from rbruck_alltoallv_b200.ops.moe import MoEExpertParallel, quantize_rows_fp8, quantize_rows_mxfp8, mx_from_atoms
+    from rbruck_alltoallv_b200.parallel.comm import Communicator
+    if fp8 is False:
+        hidden = (hidden + 255) // 256 * 256     # the bf16 GEMM's columns
+    comm = Communicator(nranks=1, heap_bytes=64 << 20, arena_bytes=1 << 20)
+    layer = MoEExpertParallel(comm, experts, hidden, 128, tokens, fp8=fp8)
+    torch.manual_seed(tokens)
+    x = torch.randn(tokens * hidden + 1, device="cuda").to(torch.bfloat16)[1:].view(tokens, hidden)
+    logits = torch.randint(0, 6, (tokens, experts), device="cuda").float()
+    for _ in range(2):                       # the second pass starts from what the first one left
+        layer.forward(x, logits)
+    layer.check()
+    order = torch.argsort(-logits - 1e-3 * (experts - torch.arange(experts, device="cuda")) / experts, dim=1, stable=True)[:, :2]
+    idx = layer.topk_idx.long()
+    assert torch.equal(idx, order)
+    rows = torch.bincount(idx.view(-1), minlength=experts)
+    assert torch.equal(layer.group_rows.long(), rows)
+    align = 128 if fp8 == "mx" else 1
+    padded = (rows + align - 1) // align * align
+    start = torch.cumsum(padded, 0) - padded
+    assert torch.equal(layer.group_start.long(), start)
+    slot = layer.slot.long()
+    assert ((slot >= start[idx]) & (slot < (start + rows)[idx])).all() and slot.unique().numel() == 2 * tokens
+    both = slot.view(-1)
+    src = x.clone().repeat_interleave(2, dim=0)
+    if fp8 is False:
+        assert torch.equal(layer.xrecv[both], src)
+    elif fp8 == "mx":
+        q, sf = quantize_rows_mxfp8(src)
+        assert torch.equal(layer.xq[both], q)
+        assert torch.equal(mx_from_atoms(layer.xs, layer.cap)[:, both], mx_from_atoms(sf, 2 * tokens))
+    else:
+        q, sc = quantize_rows_fp8(src)
+        assert torch.equal(layer.xq8[both], q) and torch.equal(layer.xs8[:, both], sc)
+    comm.close()
