@@ -12,17 +12,29 @@
 //   A: sfa[K / 128][ceil(a_rows / 128)][128]        B: sfb[G][K / 128][N / 128][128]
 // so that a tile's scales are one 512-byte TMA box per operand and K block.  For the atoms of A to coincide with tiles,
 // every group must start at a multiple of 128 rows (checked in the kernel; the MoE layout pads experts accordingly).
-// Two CTAs on neighbouring SMs share a 256 x 128 tile.  Per K block (128 bytes of K) each CTA fetches by TMA (no
-// multicast; bytes counted on a barrier of the rank-0 CTA) its own 128 rows of A, its own 64 of the 128 weight rows,
-// the scale atom of its A rows and the scale atom of the tile's 128 weight rows.  The rank-0 CTA copies the scales of
-// both CTAs from shared memory into TMEM (tcgen05.cp.32x128b.warpx4, 4 + 4 columns per stage) and issues four MMAs
-// (M 256, N 128, K 32), each naming its scale byte in the instruction descriptor.  TMEM: two 128-column accumulators
-// (the epilogue of tile i overlaps the MMAs of tile i + 1) and 8 columns of scales per pipeline stage.
-// Epilogues: bf16; SwiGLU to bf16; SwiGLU followed by the MXFP8 quantiser of the next GEMM's operand (each thread owns a
-// row of the tile, so the scale of a 32-block needs no other thread); and, for the down GEMM of the MoE layer, bf16 rows
-// stored straight into the buffers of the GPUs the tokens came from (the return all-to-all, overlapped with the MMAs
-// of the other tiles).  All waits are bounded; on expiry both CTAs are told, record an error, release their TMEM and
-// return.
+// Weight rows are the M operand and tokens the N operand (the token count is the ragged one, and the M of an MMA is
+// fixed): two CTAs on neighbouring SMs share a tile of 256 weight rows by up to 256 tokens.  Tiles start at multiples of
+// 64 tokens, so that a tile's token scales start at an even TMEM column of one of three atoms, and hold a multiple of 32.
+// Per K block (128 bytes of K) each CTA fetches by TMA (no multicast; bytes counted on a barrier of the rank-0 CTA) its
+// own 128 weight rows, its own half of the tile's tokens, the scale atom of its weight rows and the one to three scale
+// atoms of the tile's tokens.  The rank-0 CTA copies the scales of both CTAs from shared memory into TMEM
+// (tcgen05.cp.32x128b.warpx4, 4 + 12 columns per stage) and issues four MMAs (M 256, K 32), each naming its scale byte in
+// the instruction descriptor.
+// TMEM: three slots of 128 columns for accumulators and 16 columns of scales per stage.  Two tiles of 256 tokens do not
+// fit beside the scales, so they take slots 0, 1 and 1, 2 in turn; the epilogue takes the slot that they share into
+// registers first and hands it back at once, and the next tile, whose other slot was free all along, starts a TMEM read
+// later.  Tiles of up to 128 tokens alternate between slots 0 and 2.
+// Why this tile: per K block an SM's shared memory takes the stage's 34 KB from L2 and gives the MMAs 128 weight rows and
+// half the tokens for each 32 bytes of K; the more tokens an MMA has, the less of that is weights.  Measured on one B200,
+// 8 experts, hidden 4096, FFN 14336, up / down GEMM in us, against 256 tokens (as M) by 128 weight rows: 64 tokens
+// 218 / 122 -> 178 / 105, 1000 tokens 268 / 154 -> 245 / 154, 2000 tokens 456 / 224 -> 423 / 195, 8192 tokens 2098 / 1052
+// -> 1534 / 712.  On the way: 128 tokens by 256 weight rows 531 / 270 at 2000 tokens, 192 by 256 455 / 238, two MMAs of
+// 128 tokens each instead of one of 256 443 / 205.
+// Epilogues: bf16; SwiGLU to bf16; SwiGLU followed by the MXFP8 quantiser of the next GEMM's operand (32 tokens at a time
+// change hands through shared memory, so that eight lanes hold the 32 values that share a scale); and, for the down GEMM
+// of the MoE layer, bf16 rows stored straight into the buffers of the GPUs the tokens came from (the return all-to-all,
+// overlapped with the MMAs of the other tiles).  All waits are bounded; on expiry both CTAs are told, record an error,
+// release their TMEM and return.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
@@ -32,6 +44,7 @@
 
 #include "kernels/mx_quant.cuh"
 #include "kernels/sm100_ptx.cuh"
+#include "kernels/tok_epilogue.cuh"
 #include "rbv/moe.h"
 
 namespace rbv {
@@ -40,20 +53,31 @@ using namespace sm100;
 
 namespace {
 
-constexpr int XM = 256;                 // tile rows per pair
-constexpr int XHM = 128;                // rows per CTA
-constexpr int XN = 128;                 // tile columns
-constexpr int XHB = 64;                 // weight rows each CTA fetches
+constexpr int XM = 256;                 // weight rows (output columns) per pair tile
+constexpr int XHM = 128;                // weight rows per CTA
+constexpr int XT = 256;                 // most tokens per tile
+constexpr int XSUB = 128;               // tokens (columns) per accumulator slot
+constexpr int XU = 32;                  // a tile's token count is a multiple of this
+constexpr int XS = 64;                  // a tile starts at a multiple of this many tokens of its group
 constexpr int XK = 128;                 // bytes of K per pipeline stage (one 128-byte swizzle row, four scale blocks)
-constexpr int XSTAGES = 8;
-constexpr int XA_TILE = XHM * XK;       // 16 KB
-constexpr int XB_TILE = XHB * XK;       // 8 KB
-constexpr int XSF_TILE = 512;           // 128 scale words
-constexpr int XSTAGE = XA_TILE + XB_TILE + 2 * XSF_TILE;   // 25 KB
+constexpr int XSTAGES = 6;
+constexpr int XW_TILE = XHM * XK;       // 16 KB of weights
+constexpr int XT_TILE = XT / 2 * XK;    // up to 16 KB of tokens
+constexpr int XSF_TILE = 512;           // an atom: 128 scale words
+constexpr int XSTAGE = XW_TILE + XT_TILE + 4 * XSF_TILE;   // 34 KB
 constexpr int XTHREADS = 192;           // TMA warp, MMA warp, 4 epilogue warps
-constexpr int XACC_COLS = 2 * XN;       // two accumulators
-constexpr int XSF_COLS = 8;             // TMEM columns of scales per stage: 4 for A, 4 for B
-constexpr size_t XSMEM = (size_t)XSTAGES * XSTAGE + 1024;
+constexpr int XACCS = 3;                // accumulator slots
+constexpr int XACC_COLS = XACCS * XSUB;
+constexpr int XSF_COLS = 16;            // TMEM columns of scales per stage: 4 for the weights, 12 for the tokens
+static_assert(XACC_COLS + XSTAGES * XSF_COLS <= 512, "TMEM");
+// quantising epilogue: two buffers of 32 tokens x 64 outputs; rows 80 floats apart, so that the even lanes' token and the
+// odd lanes' token fall into different halves of the banks
+constexpr int XQ_LD = 80;
+constexpr int XQ_BUF = XU * XQ_LD * 4;  // 10 KB
+constexpr size_t XSMEM = (size_t)XSTAGES * XSTAGE + 2 * XQ_BUF + 1024;
+
+// Token boxes of 16, 32, 64 and 128 rows: a CTA's half of a tile is fetched with the smallest that covers it.
+struct MxMaps { CUtensorMap w, sfw, sft, tok[4]; };
 
 struct MxParams {
   const int* group_start;
@@ -72,25 +96,51 @@ struct MxParams {
   char* heap[16];
 };
 
-struct XTile { int g, m0, n0, rows; bool valid; };
+struct XTile { int g, tok0, ntok, nt, n0; bool valid; };   // group, first token row, live tokens, columns, first weight row
 
-__device__ __forceinline__ XTile xtile_of(const MxParams& p, int t, const int* s_rows, const int* s_start) {
-  const int ntn = p.N / XN;
-  XTile r; r.valid = false; r.g = 0; r.m0 = 0; r.n0 = 0; r.rows = 0;
-  for (int g = 0; g < p.G; g++) {
-    const int ntm = (s_rows[g] + XM - 1) / XM;
-    const int cnt = ntm * ntn;
-    if (t < cnt) {
-      const int n = t / ntm, m = t - n * ntm;
-      r.g = g; r.m0 = s_start[g] + m * XM; r.n0 = n * XN; r.rows = s_rows[g] - m * XM; r.valid = true;
-      return r;
+// Walks the tile schedule (groups in order, weight rows slow, tokens fast); `at(t)` wants non-decreasing t.
+struct MxWalk {
+  int g = 0, before = 0;   // tiles of the groups in front of g
+  __device__ __forceinline__ XTile at(const MxParams& p, int t, const int* s_rows, const int* s_start) {
+    XTile r; r.valid = false; r.g = r.tok0 = r.ntok = r.nt = r.n0 = 0;
+    const int ntn = (p.N + XM - 1) / XM;     // N is a multiple of 128: the last tile may be half empty
+    for (; g < p.G; g++) {
+      const int units = (s_rows[g] + XS - 1) / XS, ntm = (units + XT / XS - 1) / (XT / XS);
+      const int cnt = ntm * ntn;
+      if (t - before < cnt) {
+        const int n = (t - before) / ntm, m = (t - before) - n * ntm;
+        const int base = units / ntm, extra = units - base * ntm;     // the first `extra` tiles are one unit larger
+        const int u0 = m * base + min(m, extra), nu = base + (m < extra ? 1 : 0);
+        r.g = g; r.tok0 = s_start[g] + u0 * XS; r.n0 = n * XM;
+        r.ntok = min(s_rows[g] - u0 * XS, nu * XS); r.nt = (r.ntok + XU - 1) / XU * XU;
+        r.valid = true;
+        return r;
+      }
+      before += cnt;
     }
-    t -= cnt;
+    return r;
   }
-  return r;
-}
+};
 
-__device__ __forceinline__ float silu_x(float x) { return x / (1.0f + __expf(-x)); }
+__device__ __forceinline__ int mx_tok_box(int half) { return half <= 16 ? 0 : half <= 32 ? 1 : half <= 64 ? 2 : 3; }
+__device__ __forceinline__ uint32_t mx_tok_box_bytes(int half) { return (16u << mx_tok_box(half)) * XK; }
+
+// Accumulator slots of the tiles of one CTA pair, in order; every role walks the same sequence.
+struct MxSlots {
+  unsigned odd = 0;            // which of the two places the next tile takes
+  uint32_t phases = 0;         // bit s: parity of the uses of slot s so far
+  int first, count;            // slots of the current tile
+  __device__ __forceinline__ void next(const XTile& t) {
+    count = t.nt > XSUB ? 2 : 1;
+    first = odd ? (count == 2 ? 1 : 2) : 0;
+    odd ^= 1u;
+  }
+  __device__ __forceinline__ uint32_t phase(int slot) const { return (phases >> slot) & 1u; }
+  __device__ __forceinline__ void used(int slot) { phases ^= 1u << slot; }
+};
+
+// Scale atoms that cover the tokens of a tile: tok0 is a multiple of 64, and group starts of 128.
+__device__ __forceinline__ int mx_tok_atoms(const XTile& t) { return ((t.tok0 & 127) + t.nt + 127) / 128; }
 
 // Instruction descriptor of the block-scaled kinds: e4m3 x e4m3, K-major operands, UE8M0 scales; the scale byte each
 // operand uses (0..3 inside its TMEM word) is added per MMA.
@@ -114,6 +164,19 @@ __device__ __forceinline__ void tmem_cp_scales_pair(uint32_t taddr, uint64_t sde
   asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(sdesc) : "memory");
 }
 
+// The four epilogue warps: barrier, and barrier with a vote.
+__device__ __forceinline__ void epi_barrier() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+__device__ __forceinline__ bool epi_all(bool pred) {
+  uint32_t all;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %1, 0;\n\t"
+      "bar.red.and.pred q, 1, 128, p;\n\t"
+      "selp.b32 %0, 1, 0, q;\n\t}"
+      : "=r"(all) : "r"((uint32_t)pred) : "memory");
+  return all != 0;
+}
+
 __device__ __forceinline__ void umma_mxf8_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                                uint32_t tsfa, uint32_t tsfb, uint32_t accumulate) {
   asm volatile(
@@ -127,15 +190,13 @@ __device__ __forceinline__ void umma_mxf8_pair(uint32_t d_tmem, uint64_t a_desc,
 }  // namespace
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(XTHREADS, 1)
-grouped_gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
-                          const __grid_constant__ CUtensorMap tma_sfa, const __grid_constant__ CUtensorMap tma_sfb,
-                          const MxParams p) {
+grouped_gemm_mxfp8_kernel(const __grid_constant__ MxMaps maps, const __grid_constant__ MxParams p) {
   extern __shared__ uint8_t dyn_smem[];
   uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dyn_smem) + 1023) & ~uintptr_t(1023));
   __shared__ __align__(8) uint64_t full_bar[XSTAGES];    // rank-0 CTA: operand and scale bytes of both CTAs
   __shared__ __align__(8) uint64_t empty_bar[XSTAGES];   // each CTA: its stage has been read by the MMAs
-  __shared__ __align__(8) uint64_t tfull_bar[2];         // each CTA: accumulator b is complete
-  __shared__ __align__(8) uint64_t tempty_bar[2];        // rank-0 CTA: both CTAs have drained accumulator b
+  __shared__ __align__(8) uint64_t tfull_bar[XACCS];     // each CTA: the accumulator is complete
+  __shared__ __align__(8) uint64_t tempty_bar[XACCS];    // rank-0 CTA: both CTAs have taken the accumulator
   __shared__ uint32_t tmem_base_s;
   __shared__ int s_rows[kMoeMaxGroups], s_start[kMoeMaxGroups];
   __shared__ int s_abort, s_bad;
@@ -149,7 +210,7 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tma_a, const __gri
   if (tid == 0) {
     s_bad = 0;
     for (int s = 0; s < XSTAGES; s++) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-    for (int b = 0; b < 2; b++) { mbar_init(&tfull_bar[b], 1); mbar_init(&tempty_bar[b], 8); }
+    for (int b = 0; b < XACCS; b++) { mbar_init(&tfull_bar[b], 1); mbar_init(&tempty_bar[b], 8); }
     s_abort = 0;
     mbar_fence_init();
   }
@@ -176,28 +237,33 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tma_a, const __gri
   if (warp == 0) {
     // ---------------- TMA producer (both CTAs) ----------------
     if (elect_one()) {
-      tma_prefetch_desc(&tma_a);
-      tma_prefetch_desc(&tma_b);
-      tma_prefetch_desc(&tma_sfa);
-      tma_prefetch_desc(&tma_sfb);
+      tma_prefetch_desc(&maps.w);
+      tma_prefetch_desc(&maps.sfw);
+      tma_prefetch_desc(&maps.sft);
       int stage = 0; uint32_t phase = 0;
       bool ok = true;
       const int nb128 = p.N / 128;
+      MxWalk walk;
       for (int t = first_tile; ok; t += npairs) {
-        const XTile tl = xtile_of(p, t, s_rows, s_start);
+        const XTile tl = walk.at(p, t, s_rows, s_start);
         if (!tl.valid) break;
-        const int a_row = tl.m0 + (int)rank * XHM;
-        const int b_row = tl.g * p.N + tl.n0 + (int)rank * XHB;
+        const int half = tl.nt / 2;
+        const CUtensorMap* tok = &maps.tok[mx_tok_box(half)];
+        const int atoms = mx_tok_atoms(tl);
+        const uint32_t bytes = 2u * (XW_TILE + mx_tok_box_bytes(half) + (uint32_t)(1 + atoms) * XSF_TILE);
+        const int n_row = tl.n0 + (int)rank * XHM;
         for (int kb = 0; kb < num_kb; kb++) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag)) { ok = false; break; }
-          uint8_t* sa = tiles + (size_t)stage * XSTAGE;
-          if (leader) mbar_arrive_expect_tx(&full_bar[stage], 2 * XSTAGE);
+          uint8_t* sw = tiles + (size_t)stage * XSTAGE;
+          if (leader) mbar_arrive_expect_tx(&full_bar[stage], bytes);
           const uint32_t bar0 = mapa_u32(smem_u32(&full_bar[stage]), 0);
-          tma_load_2d_pair(sa, &tma_a, kb * XK, a_row, bar0);
-          tma_load_2d_pair(sa + XA_TILE, &tma_b, kb * XK, b_row, bar0);
-          tma_load_2d_pair(sa + XA_TILE + XB_TILE, &tma_sfa, 0, kb * p.a_row_blocks + a_row / 128, bar0);
-          tma_load_2d_pair(sa + XA_TILE + XB_TILE + XSF_TILE, &tma_sfb, 0,
-                           (tl.g * num_kb + kb) * nb128 + tl.n0 / 128, bar0);
+          // (rows of a half-empty last tile belong to the next expert or lie outside: computed, never stored)
+          tma_load_2d_pair(sw, &maps.w, kb * XK, tl.g * p.N + n_row, bar0);
+          tma_load_2d_pair(sw + XW_TILE, tok, kb * XK, tl.tok0 + (int)rank * half, bar0);
+          tma_load_2d_pair(sw + XW_TILE + XT_TILE, &maps.sfw, 0, (tl.g * num_kb + kb) * nb128 + n_row / 128, bar0);
+          for (int j = 0; j < atoms; j++)
+            tma_load_2d_pair(sw + XW_TILE + XT_TILE + (1 + j) * XSF_TILE, &maps.sft, 0,
+                             kb * p.a_row_blocks + tl.tok0 / 128 + j, bar0);
           if (++stage == XSTAGES) { stage = 0; phase ^= 1u; }
         }
       }
@@ -206,138 +272,152 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tma_a, const __gri
   } else if (warp == 1) {
     // ---------------- MMA issuer (rank-0 CTA only) ----------------
     if (leader && elect_one()) {
-      const uint32_t idesc = umma_idesc_block_scaled(XM, XN);
       int stage = 0; uint32_t phase = 0;
       bool ok = true;
-      int i = 0;
-      for (int t = first_tile; ok; t += npairs, i++) {
-        const XTile tl = xtile_of(p, t, s_rows, s_start);
+      MxSlots slots;
+      MxWalk walk;
+      for (int t = first_tile; ok; t += npairs) {
+        const XTile tl = walk.at(p, t, s_rows, s_start);
         if (!tl.valid) break;
-        const int b = i & 1;
-        if (!mbar_wait(&tempty_bar[b], (((uint32_t)i >> 1) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
+        slots.next(tl);
+        for (int s = slots.first; s < slots.first + slots.count && ok; s++) {
+          ok = mbar_wait(&tempty_bar[s], slots.phase(s) ^ 1u, abort_flag);
+          slots.used(s);
+        }
+        if (!ok) break;
         tc_fence_after_sync();
-        const uint32_t d_tmem = tmem_base + (uint32_t)b * XN;
+        const uint32_t idesc = umma_idesc_block_scaled(XM, tl.nt);
+        const uint32_t d_tmem = tmem_base + (uint32_t)slots.first * XSUB;
+        const int atoms = mx_tok_atoms(tl);
+        const uint32_t sf_shift = (uint32_t)(tl.tok0 & 127) / 32;   // TMEM column of the tile's first token: 0 or 2
+        auto copy_scales = [&](int st) {
+          const uint8_t* sf = tiles + (size_t)st * XSTAGE + XW_TILE + XT_TILE;
+          const uint32_t to = tmem_base + XACC_COLS + (uint32_t)st * XSF_COLS;
+          tmem_cp_scales_pair(to, desc_rows16(sf));
+          for (int j = 0; j < atoms; j++) tmem_cp_scales_pair(to + 4u + 4u * (uint32_t)j, desc_rows16(sf + (1 + j) * XSF_TILE));
+        };
+        // The scales of the next K block are copied in front of the MMAs of this one when they are there already, so that
+        // the copies (which MMAs have to wait for) run beside MMAs.
+        bool copied = false;
         for (int kb = 0; kb < num_kb; kb++) {
-          if (!mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
-          tc_fence_after_sync();
-          const uint8_t* sa = tiles + (size_t)stage * XSTAGE;
-          const uint64_t adesc = umma_desc_sw128(sa);
-          const uint64_t bdesc = umma_desc_sw128(sa + XA_TILE);
-          const uint32_t tsfa = tmem_base + XACC_COLS + (uint32_t)stage * XSF_COLS;
-          const uint32_t tsfb = tsfa + 4;
-          tmem_cp_scales_pair(tsfa, desc_rows16(sa + XA_TILE + XB_TILE));
-          tmem_cp_scales_pair(tsfb, desc_rows16(sa + XA_TILE + XB_TILE + XSF_TILE));
+          if (!copied) {
+            if (!mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
+            tc_fence_after_sync();
+            copy_scales(stage);
+          }
+          const int next = stage + 1 == XSTAGES ? 0 : stage + 1;
+          const uint32_t next_phase = next ? phase : phase ^ 1u;
+          copied = kb + 1 < num_kb && mbar_try_wait(&full_bar[next], next_phase);
+          if (copied) {
+            tc_fence_after_sync();
+            copy_scales(next);
+          }
+          const uint8_t* sw = tiles + (size_t)stage * XSTAGE;
+          const uint64_t wdesc = umma_desc_sw128(sw);
+          const uint32_t tsfw = tmem_base + XACC_COLS + (uint32_t)stage * XSF_COLS;
+          const uint64_t tdesc = umma_desc_sw128(sw + XW_TILE);
           #pragma unroll
           for (int kk = 0; kk < XK / 32; kk++)
-            umma_mxf8_pair(d_tmem, adesc + 2u * kk, bdesc + 2u * kk, with_scale_ids(idesc, kk, kk), tsfa, tsfb,
+            umma_mxf8_pair(d_tmem, wdesc + 2u * kk, tdesc + 2u * kk, with_scale_ids(idesc, kk, kk), tsfw, tsfw + 4 + sf_shift,
                            (uint32_t)((kb | kk) != 0));
           umma_commit_pair(&empty_bar[stage]);   // frees this stage (operands and scales) in both CTAs
-          if (++stage == XSTAGES) { stage = 0; phase ^= 1u; }
+          stage = next; phase = next_phase;
         }
-        if (ok) umma_commit_pair(&tfull_bar[b]);
+        for (int s = slots.first; s < slots.first + slots.count && ok; s++) umma_commit_pair(&tfull_bar[s]);
       }
       if (!ok) { s_abort = 1; st_cluster_u32(peer_abort, 1); atomicExch(p.error, 2); }
     }
   } else {
     // ---------------- epilogue (both CTAs): warps 2..5, TMEM lane quarter = warp % 4 ----------------
     const int q = warp & 3;
-    const int row = q * 32 + lane;
+    const bool odd = (lane & 1) != 0;
+    float* const qbuf = reinterpret_cast<float*>(tiles + (size_t)XSTAGES * XSTAGE);
     __nv_bfloat16* C = static_cast<__nv_bfloat16*>(p.C);
     const uint32_t tempty0 = mapa_u32(smem_u32(&tempty_bar[0]), 0);
     bool ok = true;
-    int i = 0;
-    for (int t = first_tile; ok; t += npairs, i++) {
-      const XTile tl = xtile_of(p, t, s_rows, s_start);
+    unsigned chunk = 0;   // 32-token chunks so far: which of the two shared buffers
+    MxSlots slots;
+    MxWalk walk;
+    for (int t = first_tile; ok; t += npairs) {
+      const XTile tl = walk.at(p, t, s_rows, s_start);
       if (!tl.valid) break;
-      const int b = i & 1;
-      if (!mbar_wait(&tfull_bar[b], ((uint32_t)i >> 1) & 1u, abort_flag)) { ok = false; break; }
-      tc_fence_after_sync();
-      const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)b * XN;
-      const int my_m0 = tl.m0 + (int)rank * XHM;
-      const bool live = row < tl.rows - (int)rank * XHM;
-      __nv_bfloat16* crow = C + (size_t)(my_m0 + row) * p.ldc;
-      if (p.ret && live) {
-        const unsigned rv = __ldg(p.ret + my_m0 + row);
-        crow = reinterpret_cast<__nv_bfloat16*>(p.heap[rv >> 24] + p.y2_off) + (size_t)(rv & 0xffffffu) * p.ldc;
-      }
-      if (p.epilogue == 3) {
-        // SwiGLU, then the quantiser of the next GEMM's A operand, fused: the 64 outputs of this thread's row are two
-        // blocks of 32; each gets its power-of-two scale from the row's own values (no other thread is involved)
-        uint8_t* qrow = static_cast<uint8_t*>(p.C) + (size_t)(my_m0 + row) * p.ldc + tl.n0 / 2;
-        uint32_t sbytes = 0;
-        #pragma unroll 1
-        for (int half = 0; half < 2; half++) {
-          float o[32];
+      const int n_cta = tl.n0 + (int)rank * XHM;     // this CTA's first output column
+      const bool inside = n_cta < p.N;
+      const int nw = n_cta + q * 32;
+      // tokens c .. c + 31 of the tile
+      auto store_chunk = [&](const uint32_t (&r)[32], int c) {
+        const int live = inside ? tl.ntok - c : 0;
+        unsigned rv = 0;   // push mode: where the token of this lane's index goes, handed out by shuffle
+        if (p.ret && c + lane < tl.ntok) rv = __ldg(p.ret + tl.tok0 + c + lane);
+        if (p.epilogue == 3) {
+          // SwiGLU, then the quantiser of the next GEMM's operand: 32 tokens x 64 outputs of this CTA go through shared
+          // memory, after which 16 lanes hold a token's 64 outputs, four each, and 8 lanes the 32 that share a scale.
+          // The 64 (token, 4-wide) pieces of a warp are read before the other buffer is used again one barrier later.
+          float* buf = qbuf + (chunk++ & 1u) * (XU * XQ_LD);
           #pragma unroll
-          for (int cc = 0; cc < 2; cc++) {
-            uint32_t r[32];
-            tmem_ld32(taddr + half * 64 + cc * 32, r);
-            tmem_ld_wait();
-            #pragma unroll
-            for (int j = 0; j < 16; j++)
-              o[cc * 16 + j] = silu_x(__uint_as_float(r[2 * j])) * __uint_as_float(r[2 * j + 1]);
-          }
-          float m = 0.0f;
+          for (int k = 0; k < 32; k += 2)
+            buf[(k + (odd ? 1 : 0)) * XQ_LD + q * 16 + (lane >> 1)] = tokepi::swiglu_pair(r, k, odd);
+          epi_barrier();
           #pragma unroll
-          for (int j = 0; j < 32; j++) m = fmaxf(m, fabsf(o[j]));
-          const int e = mx_exponent(m);
-          const float inv = mx_inv_scale(e);
-          sbytes |= (uint32_t)(e + 127) << (8 * half);
-          uint32_t w[8];
-          #pragma unroll
-          for (int j = 0; j < 8; j++) {
-            const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(o[4 * j] * inv, o[4 * j + 1] * inv), __NV_SATFINITE, __NV_E4M3);
-            const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(o[4 * j + 2] * inv, o[4 * j + 3] * inv), __NV_SATFINITE, __NV_E4M3);
-            w[j] = lo | (hi << 16);
-          }
-          if (live) {
-            uint4* dst = reinterpret_cast<uint4*>(qrow + half * 32);
-            dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
-            dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
-          }
-        }
-        if (live) {
-          const unsigned R = (unsigned)(my_m0 + row);
-          uint32_t* word = p.sf_out + ((size_t)(tl.n0 / 256) * p.a_row_blocks + R / 128) * 128 + (R % 32) * 4 + (R % 128) / 32;
-          *reinterpret_cast<uint16_t*>(reinterpret_cast<uint8_t*>(word) + ((tl.n0 / 64) & 3)) = (uint16_t)sbytes;
-        }
-      } else
-      #pragma unroll 1
-      for (int c = 0; c < XN; c += 32) {
-        uint32_t r[32];
-        tmem_ld32(taddr + c, r);
-        tmem_ld_wait();
-        if (p.epilogue & 1) {
-          uint32_t o[8];
-          #pragma unroll
-          for (int j = 0; j < 8; j++) {
-            float g0 = __uint_as_float(r[4 * j]), u0 = __uint_as_float(r[4 * j + 1]);
-            float g1 = __uint_as_float(r[4 * j + 2]), u1 = __uint_as_float(r[4 * j + 3]);
-            __nv_bfloat162 v = __floats2bfloat162_rn(silu_x(g0) * u0, silu_x(g1) * u1);
-            o[j] = *reinterpret_cast<uint32_t*>(&v);
-          }
-          if (live) {
-            uint4* dst = reinterpret_cast<uint4*>(crow + (tl.n0 + c) / 2);
-            dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
-            dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
+          for (int u = 0; u < 4; u++) {
+            const int tok = u * 8 + q * 2 + (lane >> 4), l16 = lane & 15;
+            const float4 o = *reinterpret_cast<const float4*>(buf + tok * XQ_LD + l16 * 4);
+            float m = fmaxf(fmaxf(fabsf(o.x), fabsf(o.y)), fmaxf(fabsf(o.z), fabsf(o.w)));
+            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
+            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
+            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 4));
+            const int e = mx_exponent(m);
+            const float inv = mx_inv_scale(e);
+            const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(o.x * inv, o.y * inv), __NV_SATFINITE, __NV_E4M3);
+            const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(o.z * inv, o.w * inv), __NV_SATFINITE, __NV_E4M3);
+            if (tok < live) {
+              const unsigned R = (unsigned)(tl.tok0 + c + tok);
+              const int n_out = n_cta / 2;
+              *reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(p.C) + (size_t)R * p.ldc + n_out + l16 * 4) = lo | (hi << 16);
+              if ((l16 & 7) == 0) {
+                uint32_t* word = p.sf_out + ((size_t)(n_out / 128) * p.a_row_blocks + R / 128) * 128 + (R % 32) * 4 + (R % 128) / 32;
+                reinterpret_cast<uint8_t*>(word)[(n_out / 32 & 3) + (l16 >> 3)] = (uint8_t)(e + 127);
+              }
+            }
           }
         } else {
-          uint32_t o[16];
-          #pragma unroll
-          for (int j = 0; j < 16; j++) {
-            __nv_bfloat162 v = __floats2bfloat162_rn(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
-            o[j] = *reinterpret_cast<uint32_t*>(&v);
-          }
-          if (live) {
-            uint4* dst = reinterpret_cast<uint4*>(crow + tl.n0 + c);
-            #pragma unroll
-            for (int j = 0; j < 4; j++) dst[j] = make_uint4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
+          __nv_bfloat16* rows = C + (size_t)(tl.tok0 + c) * p.ldc;
+          if (p.epilogue == 1) {
+            tokepi::store_swiglu(r, rows, p.ldc, nw / 2, live, lane);
+          } else if (p.ret) {
+            tokepi::store_plain(r, [&](int tok) {
+              const unsigned to = __shfl_sync(0xffffffffu, rv, tok);
+              return reinterpret_cast<__nv_bfloat16*>(p.heap[to >> 24] + p.y2_off) + (size_t)(to & 0xffffffu) * p.ldc;
+            }, nw, live, lane);
+          } else {
+            tokepi::store_plain(r, [&](int tok) { return rows + (size_t)tok * p.ldc; }, nw, live, lane);
           }
         }
+      };
+      slots.next(tl);
+      for (int i = 0; i < slots.count; i++) {
+        // of two slots the one that the next tile wants, slot 1, goes first
+        const int b = slots.count == 2 ? (i == 0 ? 1 : slots.first == 0 ? 0 : 2) : slots.first;
+        const int s = b - slots.first;       // tokens s * 128 ...
+        // (the four epilogue warps meet at a named barrier when they quantise: they leave the loop together, see the vote)
+        const bool got_it = mbar_wait(&tfull_bar[b], slots.phase(b), abort_flag);
+        slots.used(b);
+        if (p.epilogue == 3 ? !epi_all(got_it) : !got_it) { ok = false; break; }
+        tc_fence_after_sync();
+        const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)b * XSUB;
+        const int n = min(tl.nt - s * XSUB, XSUB);
+        uint32_t r[XSUB / 32][32];
+        #pragma unroll
+        for (int k = 0; k < XSUB / 32; k++)
+          if (k * 32 < n) tmem_ld32(taddr + k * 32, r[k]);
+        tmem_ld_wait();
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(tempty0 + 8u * (uint32_t)b);   // 4 warps x 2 CTAs
+        #pragma unroll
+        for (int k = 0; k < XSUB / 32; k++)
+          if (k * 32 < n) store_chunk(r[k], s * XSUB + k * 32);
       }
-      tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(tempty0 + 8u * (uint32_t)b);   // 4 warps x 2 CTAs
     }
     if (!ok && lane == 0) { s_abort = 1; st_cluster_u32(peer_abort, 1); atomicExch(p.error, 3); }
   }
@@ -469,7 +549,7 @@ static int launch_mxfp8(const void* A, const void* sfa, long long a_rows, const 
                         const void* const* heaps = nullptr, int nheaps = 0, unsigned long long y2_off = 0) {
   using namespace rbv;
   if (ret && (epilogue != 0 || !heaps || nheaps < 1 || nheaps > 16 || (y2_off & 15))) return (int)cudaErrorInvalidValue;
-  if (G < 1 || G > kMoeMaxGroups || N % XN || K % XK || a_rows < 1 || (ldc % 8)) return (int)cudaErrorInvalidValue;
+  if (G < 1 || G > kMoeMaxGroups || N % 128 || K % XK || a_rows < 1 || (ldc % 8)) return (int)cudaErrorInvalidValue;
   if (epilogue == 3 && (!sf_out || N % 256 || ldc % 16 || (reinterpret_cast<uintptr_t>(sf_out) & 15)))
     return (int)cudaErrorInvalidValue;
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C)) & 15)
@@ -483,11 +563,12 @@ static int launch_mxfp8(const void* A, const void* sfa, long long a_rows, const 
     configured = true;
   }
   const unsigned long long nrb = (unsigned long long)((a_rows + 127) / 128), nkb = (unsigned long long)(K / XK);
-  CUtensorMap ma, mb, msa, msb;
-  if (!make_map_mx(&ma, A, (unsigned long long)a_rows, (unsigned long long)K, XHM)) return (int)cudaErrorUnknown;
-  if (!make_map_mx(&mb, B, (unsigned long long)G * N, (unsigned long long)K, XHB)) return (int)cudaErrorUnknown;
-  if (!make_map_atoms(&msa, sfa, nkb * nrb)) return (int)cudaErrorUnknown;
-  if (!make_map_atoms(&msb, sfb, (unsigned long long)G * nkb * (unsigned long long)(N / 128))) return (int)cudaErrorUnknown;
+  MxMaps maps;
+  if (!make_map_mx(&maps.w, B, (unsigned long long)G * N, (unsigned long long)K, XHM)) return (int)cudaErrorUnknown;
+  for (int i = 0; i < 4; i++)
+    if (!make_map_mx(&maps.tok[i], A, (unsigned long long)a_rows, (unsigned long long)K, 16u << i)) return (int)cudaErrorUnknown;
+  if (!make_map_atoms(&maps.sft, sfa, nkb * nrb)) return (int)cudaErrorUnknown;
+  if (!make_map_atoms(&maps.sfw, sfb, (unsigned long long)G * nkb * (unsigned long long)(N / 128))) return (int)cudaErrorUnknown;
   MxParams p;
   p.group_start = group_start; p.group_rows = group_rows; p.G = G; p.N = N; p.K = K; p.ldc = ldc;
   p.a_row_blocks = (int)nrb;
@@ -502,7 +583,7 @@ static int launch_mxfp8(const void* A, const void* sfa, long long a_rows, const 
   }
   grid &= ~1;   // whole pairs
   if (grid < 2) return (int)cudaErrorInvalidValue;
-  grouped_gemm_mxfp8_kernel<<<grid, XTHREADS, XSMEM, static_cast<cudaStream_t>(cuda_stream)>>>(ma, mb, msa, msb, p);
+  grouped_gemm_mxfp8_kernel<<<grid, XTHREADS, XSMEM, static_cast<cudaStream_t>(cuda_stream)>>>(maps, p);
   return (int)cudaGetLastError();
 }
 

@@ -247,9 +247,11 @@ def test_grouped_gemm_mxfp8_scale_paths(scales):
 
 
 @pytest.mark.parametrize("swiglu", [False, True])
-@pytest.mark.parametrize("rows,N", [([1], 128), ([31, 32, 33], 256), ([127, 0, 128, 129], 384), ([160, 97, 300], 640)])
+@pytest.mark.parametrize("rows,N", [([1], 128), ([31, 32, 33], 256), ([127, 0, 128, 129], 384), ([160, 97, 300], 640),
+                                     ([191, 192, 193, 257], 256), ([500, 321, 64, 65], 512),
+                                     ([255, 1025, 256], 2304)])
 def test_grouped_gemm_mxfp8_token_tiles(rows, N, swiglu):
-    """Token counts at the edges of the units (32) and tiles (128); N with and without a half-empty last tile.  The
+    """Token counts at the edges of the units (32), tile starts (64), accumulators (128) and tiles (256); N with and without a half-empty last tile.  The
     operands are exact after quantisation, so the bound is bf16 rounding plus fp32 accumulation of K = 384 products."""
     from rbruck_alltoallv_b200.ops.moe import (dequantize_rows_mxfp8, dequantize_weight_mxfp8, grouped_gemm_mxfp8,
                                                quantize_rows_mxfp8, quantize_weight_mxfp8)
