@@ -52,6 +52,10 @@ int rbv_grouped_gemm_fp8(const void* A, const float* a_scale_t, long long a_rows
 int rbv_grouped_gemm_fp8_pair(const void* A, const float* a_scale_t, long long a_rows, const void* B,
                               const float* b_scale, void* C, const int* group_start, const int* group_rows, int G,
                               int N, int K, int ldc, int epilogue, int* error_flag, int max_ctas, void* cuda_stream);
+/* Behind rbv_grouped_gemm_fp8_pair for few rows per group: 256 weight rows by 32 to 128 tokens per tile. */
+int rbv_grouped_gemm_fp8_tok(const void* A, const float* a_scale_t, long long a_rows, const void* B,
+                             const float* b_scale, void* C, const int* group_start, const int* group_rows, int G,
+                             int N, int K, int ldc, int epilogue, int* error_flag, int max_ctas, void* cuda_stream);
 /* MXFP8 variant: e4m3 operands with one UE8M0 (power-of-two) scale per 32 elements along K on both operands, applied
  * by the tensor core (tcgen05.mma.kind::mxf8f6f4.block_scale) on CTA pairs.  Scales are packed four to a uint32 (the
  * four 32-blocks of one 128-wide K block, lowest byte first); the words of 128 consecutive rows form one 512-byte atom

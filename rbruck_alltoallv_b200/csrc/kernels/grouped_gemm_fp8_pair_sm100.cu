@@ -354,6 +354,14 @@ extern "C" int rbv_grouped_gemm_fp8_pair(const void* A, const float* a_scale_t, 
                                          int G, int N, int K, int ldc, int epilogue, int* error_flag, int max_ctas,
                                          void* cuda_stream) {
   using namespace rbv;
+  // Few tokens per group: tokens as the N operand (grouped_gemm_fp8_tok_sm100.cu).  Only the device knows the groups'
+  // rows; the host knows the rows of A, of which the MoE layer, whose buffer is sized for twice the average load, uses
+  // half.  Measured on one B200, 8 experts, hidden 4096, FFN 14336, up / down GEMM, this kernel against that one:
+  // 25 rows per expert 314 / 222 against 170 / 100 us, 125 rows 333 / 222 against 274 / 144, 250 rows 410 / 261 against
+  // 405 / 188, 500 rows 669 / 372 against 757 / 368.
+  if (a_rows <= 384ll * G)
+    return rbv_grouped_gemm_fp8_tok(A, a_scale_t, a_rows, B, b_scale, C, group_start, group_rows, G, N, K, ldc, epilogue,
+                                    error_flag, max_ctas, cuda_stream);
   if (G < 1 || G > kMoeMaxGroups || N % QN || K % QK || a_rows < 1 || (ldc % 8)) return (int)cudaErrorInvalidValue;
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C)) & 15)
     return (int)cudaErrorInvalidValue;

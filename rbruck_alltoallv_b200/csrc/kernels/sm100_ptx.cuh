@@ -124,6 +124,16 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
       : "r"(taddr)
       : "memory");
 }
+// 16 TMEM lanes x 16 columns in the shape of an MMA fragment: lane l of the warp gets, for each group g of 8 columns,
+// columns 8 g + 2 (l % 4) and + 1 of TMEM lane l / 4 in r[4 g], r[4 g + 1], and of TMEM lane l / 4 + 8 in r[4 g + 2],
+// r[4 g + 3].  `taddr` names the first of the 16 lanes (0 or 16 of the warp's quarter).
+__device__ __forceinline__ void tmem_ld_frag16(uint32_t taddr, uint32_t* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+      : "r"(taddr)
+      : "memory");
+}
 __device__ __forceinline__ void tmem_ld_wait() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }

@@ -150,6 +150,38 @@ def test_grouped_gemm_fp8_block_scaled(rows, N, K, pair):
         r0 += n
 
 
+@pytest.mark.parametrize("swiglu", [False, True])
+@pytest.mark.parametrize("rows,N", [([1], 128), ([31, 32, 33], 256), ([63, 0, 64, 65, 97], 384), ([127, 128, 129, 300], 640), ([900], 256)])
+def test_grouped_gemm_fp8_token_tiles(rows, N, swiglu):
+    """Token counts at the edges of the pair kernel's units (32) and tiles (128); N with and without a half-empty last
+    tile.  The operands are exact after quantisation, so the bound is bf16 rounding plus fp32 accumulation of K = 640
+    products and their scaling."""
+    from rbruck_alltoallv_b200.ops.moe import (dequantize_rows_fp8, dequantize_weight_blocks_fp8, grouped_gemm_fp8,
+                                               quantize_rows_fp8, quantize_weight_blocks_fp8)
+    torch.manual_seed(sum(rows) + N)
+    G, M, K = len(rows), sum(rows), 640
+    gs, gr = _groups(rows, "cuda")
+    Aq, sa = quantize_rows_fp8(torch.randn(M, K, device="cuda").to(torch.bfloat16))
+    Bq, sb = quantize_weight_blocks_fp8(torch.randn(G, N, K, device="cuda") * 0.1)
+    A, B = dequantize_rows_fp8(Aq, sa).double(), dequantize_weight_blocks_fp8(Bq, sb).double()
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    n_out = N // 2 if swiglu else N
+    out = torch.full((M + 3, n_out), 7.0, dtype=torch.bfloat16, device="cuda")
+    grouped_gemm_fp8(Aq, sa, Bq, sb, gs, gr, out=out, swiglu=swiglu, error=err, pair=True)
+    torch.cuda.synchronize()
+    assert err.item() == 0 and torch.all(out[M:] == 7.0)
+    r0 = 0
+    for g, n in enumerate(rows):
+        a, w = A[r0:r0 + n], B[g]
+        ref, slack = a @ w.t(), (a.abs() @ w.abs().t()) * 640 * 2.0 ** -24
+        if swiglu:
+            gate, up = ref[:, 0::2], ref[:, 1::2]
+            slack = 1.1 * up.abs() * slack[:, 0::2] + gate.abs() * slack[:, 1::2] + (gate * up).abs() * 2.0 ** -20
+            ref = torch.nn.functional.silu(gate) * up
+        assert ((out[r0:r0 + n].double() - ref).abs() <= ref.abs() * 2.0 ** -8 + slack + 1e-6).all(), f"group {g}"
+        r0 += n
+
+
 @pytest.mark.parametrize("pair", [False, True])
 def test_grouped_gemm_fp8_coarse_scales(pair):
     """Scales that are constant along K: the whole tile is accumulated in TMEM and scaled once."""
