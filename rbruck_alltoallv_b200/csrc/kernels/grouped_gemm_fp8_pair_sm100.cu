@@ -16,6 +16,7 @@
 
 #include <cstdint>
 
+#include "kernels/pdl.cuh"
 #include "kernels/sm100_ptx.cuh"
 #include "rbv/moe.h"
 
@@ -107,8 +108,10 @@ grouped_gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __
     s_abort = 0;
     mbar_fence_init();
   }
-  for (int i = tid; i < p.G; i += blockDim.x) { s_rows[i] = p.group_rows[i]; s_start[i] = p.group_start[i]; }
   if (warp == 1) { tmem_alloc_pair(&tmem_base_s, 512); tmem_relinquish_pair(); }
+  pdl_trigger();
+  pdl_wait();
+  for (int i = tid; i < p.G; i += blockDim.x) { s_rows[i] = p.group_rows[i]; s_start[i] = p.group_start[i]; }
   tc_fence_before_sync();
   __syncthreads();
   cluster_sync_all();
@@ -386,6 +389,5 @@ extern "C" int rbv_grouped_gemm_fp8_pair(const void* A, const float* a_scale_t, 
   }
   grid &= ~1;   // whole pairs
   if (grid < 2) return (int)cudaErrorInvalidValue;
-  grouped_gemm_fp8_pair_kernel<<<grid, QTHREADS, QSMEM, static_cast<cudaStream_t>(cuda_stream)>>>(ma, mb, p);
-  return (int)cudaGetLastError();
+  return (int)launch_dependent(grouped_gemm_fp8_pair_kernel, grid, QTHREADS, QSMEM, static_cast<cudaStream_t>(cuda_stream), ma, mb, p);
 }

@@ -18,6 +18,7 @@
 
 #include <cstdint>
 
+#include "kernels/pdl.cuh"
 #include "kernels/sm100_ptx.cuh"
 #include "rbv/moe.h"
 
@@ -290,6 +291,8 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_
 __global__ void __launch_bounds__(256)
 quantize_rows_kernel(const __nv_bfloat16* __restrict__ x, long long rows, int K, int ldx, uint8_t* __restrict__ out,
                      float* __restrict__ scale_t, const int* __restrict__ used) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int kUnroll = 4;
   const int lane16 = threadIdx.x & 15;
   const unsigned kblocks = (unsigned)(K / 128);
@@ -424,7 +427,7 @@ extern "C" int rbv_quantize_used_rows_fp8(const void* x_bf16, long long rows, co
   long long grid = (nblk + 63) / 64;   // 16 half-warps per block, four blocks of columns each
   if (grid > 148 * 8) grid = 148 * 8;
   if (grid < 1) grid = 1;
-  quantize_rows_kernel<<<(int)grid, 256, 0, static_cast<cudaStream_t>(cuda_stream)>>>(
-      static_cast<const __nv_bfloat16*>(x_bf16), rows, K, ldx, static_cast<uint8_t*>(out_fp8), scale_t, used);
-  return (int)cudaGetLastError();
+  return (int)launch_dependent(quantize_rows_kernel, (unsigned)grid, 256, 0, static_cast<cudaStream_t>(cuda_stream),
+                               static_cast<const __nv_bfloat16*>(x_bf16), rows, K, ldx, static_cast<uint8_t*>(out_fp8),
+                               scale_t, used);
 }

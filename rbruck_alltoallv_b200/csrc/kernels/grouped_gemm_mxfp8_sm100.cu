@@ -43,6 +43,7 @@
 #include <cstdint>
 
 #include "kernels/mx_quant.cuh"
+#include "kernels/pdl.cuh"
 #include "kernels/sm100_ptx.cuh"
 #include "kernels/tok_epilogue.cuh"
 #include "rbv/moe.h"
@@ -214,12 +215,14 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ MxMaps maps, const __grid_cons
     s_abort = 0;
     mbar_fence_init();
   }
+  if (warp == 1) { tmem_alloc_pair(&tmem_base_s, 512); tmem_relinquish_pair(); }
   __syncthreads();
+  pdl_trigger();
+  pdl_wait();
   for (int i = tid; i < p.G; i += blockDim.x) {
     s_rows[i] = p.group_rows[i]; s_start[i] = p.group_start[i];
     if (s_rows[i] > 0 && (s_start[i] & 127)) s_bad = 1;   // the scale atoms of A would not coincide with the tiles
   }
-  if (warp == 1) { tmem_alloc_pair(&tmem_base_s, 512); tmem_relinquish_pair(); }
   tc_fence_before_sync();
   __syncthreads();
   cluster_sync_all();
@@ -583,8 +586,8 @@ static int launch_mxfp8(const void* A, const void* sfa, long long a_rows, const 
   }
   grid &= ~1;   // whole pairs
   if (grid < 2) return (int)cudaErrorInvalidValue;
-  grouped_gemm_mxfp8_kernel<<<grid, XTHREADS, XSMEM, static_cast<cudaStream_t>(cuda_stream)>>>(maps, p);
-  return (int)cudaGetLastError();
+  return (int)launch_dependent(grouped_gemm_mxfp8_kernel, grid, XTHREADS, XSMEM, static_cast<cudaStream_t>(cuda_stream),
+                               maps, p);
 }
 
 extern "C" int rbv_grouped_gemm_mxfp8(const void* A, const void* sfa, long long a_rows, const void* B, const void* sfb,

@@ -26,6 +26,7 @@
 #include <cstdint>
 #include <cstdlib>
 
+#include "kernels/pdl.cuh"
 #include "kernels/sm100_ptx.cuh"
 #include "kernels/tok_epilogue.cuh"
 #include "rbv/moe.h"
@@ -123,8 +124,10 @@ grouped_gemm_pair_kernel(const __grid_constant__ PairMaps maps, const __grid_con
     s_abort = 0;
     mbar_fence_init();
   }
-  for (int i = tid; i < p.G; i += blockDim.x) { s_rows[i] = p.group_rows[i]; s_start[i] = p.group_start[i]; }
   if (warp == 1) { tmem_alloc_pair(&tmem_base_s, PAIR_TMEM_COLS); tmem_relinquish_pair(); }
+  pdl_trigger();
+  pdl_wait();
+  for (int i = tid; i < p.G; i += blockDim.x) { s_rows[i] = p.group_rows[i]; s_start[i] = p.group_start[i]; }
   tc_fence_before_sync();
   __syncthreads();
   cluster_sync_all();   // barriers of both CTAs are initialised before anything is signalled across
@@ -323,8 +326,8 @@ static int launch_bf16_pair(const void* A, long long a_rows, const void* B, void
   }
   grid &= ~1;   // whole pairs
   if (grid < 2) return (int)cudaErrorInvalidValue;
-  grouped_gemm_pair_kernel<<<grid, PAIR_THREADS, PAIR_SMEM, static_cast<cudaStream_t>(cuda_stream)>>>(maps, p);
-  return (int)cudaGetLastError();
+  return (int)launch_dependent(grouped_gemm_pair_kernel, grid, PAIR_THREADS, PAIR_SMEM,
+                               static_cast<cudaStream_t>(cuda_stream), maps, p);
 }
 
 extern "C" int rbv_grouped_gemm_bf16_pair(const void* A, long long a_rows, const void* B, void* C,

@@ -18,6 +18,7 @@
 #include "api/ctx_internal.h"
 #include "kernels/moe_router.cuh"
 #include "kernels/mx_quant.cuh"
+#include "kernels/pdl.cuh"
 #include "kernels/primitives.cuh"
 #include "rbv/device_types.h"
 #include "rbv/moe.h"
@@ -45,6 +46,7 @@ __global__ void __launch_bounds__(kRouteWarps * 32) moe_route_local_kernel(const
   __shared__ int s_rows[kMoeMaxExperts], s_base[kMoeMaxExperts];
   __shared__ int s_last;
   const int tid = threadIdx.x, lane = tid & 31;
+  pdl_trigger();
   for (int i = tid; i < a.E; i += blockDim.x) s_rows[i] = 0;
   __syncthreads();
   const int t = blockIdx.x * kRouteWarps + (tid >> 5);
@@ -115,6 +117,8 @@ struct DispatchLocalArgs {
 // One warp per (token, piece of U * 256 columns).
 template <int MODE, int U>
 __global__ void __launch_bounds__(128) moe_dispatch_local_kernel(const __grid_constant__ DispatchLocalArgs a) {
+  pdl_trigger();
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const long long item = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
   const int t = (int)(item / a.segs), seg = (int)(item - (long long)t * a.segs);
@@ -204,6 +208,8 @@ struct CombineLocalArgs {
 // One warp per (token, piece of U * 256 columns): all loads of a piece before its first store.
 template <int U>
 __global__ void __launch_bounds__(128) moe_combine_local_kernel(const __grid_constant__ CombineLocalArgs a) {
+  pdl_trigger();
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const long long item = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
   const int t = (int)(item / a.segs), seg = (int)(item - (long long)t * a.segs);
@@ -279,16 +285,11 @@ int rbv_moe_dispatch_local(rbv_ctx_t ctx, const void* x, int T, int H, const int
   const bool lng = long_pieces(T, H, ctx->c->sm_count());
   const unsigned grid = piece_grid(T, H, lng, &a.segs);
   const cudaStream_t st = static_cast<cudaStream_t>(stream);
-#define RBV_LAUNCH(MODE) \
-  if (lng) moe_dispatch_local_kernel<MODE, 4><<<grid, 128, 0, st>>>(a); else moe_dispatch_local_kernel<MODE, 1><<<grid, 128, 0, st>>>(a)
-  switch (format) {
-    case ROWS_BF16: RBV_LAUNCH(ROWS_BF16); break;
-    case ROWS_MX: RBV_LAUNCH(ROWS_MX); break;
-    case ROWS_FP8: RBV_LAUNCH(ROWS_FP8); break;
-    default: return (int)cudaErrorInvalidValue;
-  }
-#undef RBV_LAUNCH
-  return (int)cudaGetLastError();
+  auto* kernel = lng ? moe_dispatch_local_kernel<ROWS_BF16, 4> : moe_dispatch_local_kernel<ROWS_BF16, 1>;
+  if (format == ROWS_MX) kernel = lng ? moe_dispatch_local_kernel<ROWS_MX, 4> : moe_dispatch_local_kernel<ROWS_MX, 1>;
+  else if (format == ROWS_FP8) kernel = lng ? moe_dispatch_local_kernel<ROWS_FP8, 4> : moe_dispatch_local_kernel<ROWS_FP8, 1>;
+  else if (format != ROWS_BF16) return (int)cudaErrorInvalidValue;
+  return (int)launch_dependent(kernel, grid, 128, 0, st, a);
 }
 
 int rbv_moe_combine_local(rbv_ctx_t ctx, void* out, int T, int H, const int* slot, const float* topk_w, const void* y,
@@ -301,9 +302,7 @@ int rbv_moe_combine_local(rbv_ctx_t ctx, void* out, int T, int H, const int* slo
   const bool lng = long_pieces(T, H, ctx->c->sm_count());
   const unsigned grid = piece_grid(T, H, lng, &a.segs);
   const cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (lng) moe_combine_local_kernel<4><<<grid, 128, 0, st>>>(a);
-  else moe_combine_local_kernel<1><<<grid, 128, 0, st>>>(a);
-  return (int)cudaGetLastError();
+  return (int)launch_dependent(lng ? moe_combine_local_kernel<4> : moe_combine_local_kernel<1>, grid, 128, 0, st, a);
 }
 
 }  // extern "C"

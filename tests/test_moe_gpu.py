@@ -566,3 +566,39 @@ def test_moe_one_rank_route_and_dispatch(tokens, hidden, experts, fp8):
         q, sc = quantize_rows_fp8(src)
         assert torch.equal(layer.xq8[both], q) and torch.equal(layer.xs8[:, both], sc)
     comm.close()
+
+
+@pytest.mark.parametrize("fp8", [False, True, "mx"], ids=["bf16", "fp8", "mxfp8"])
+def test_moe_layer_back_to_back_and_captured(fp8):
+    """The layer's kernels may start while the one before is still running: passes in a row over changing inputs, and the
+    same passes replayed from a CUDA graph, equal passes that were waited for one by one."""
+    from rbruck_alltoallv_b200.ops.moe import MoEExpertParallel
+    from rbruck_alltoallv_b200.parallel.comm import Communicator
+    T, H, E = 300, 512, 8
+    comm = Communicator(nranks=1, heap_bytes=64 << 20, arena_bytes=1 << 20)
+    layer = MoEExpertParallel(comm, E, H, 256, T, fp8=fp8)
+    torch.manual_seed(0)
+    xs = [torch.randn(T, H, device="cuda").to(torch.bfloat16) for _ in range(6)]
+    ls = [torch.randn(T, E, device="cuda") for _ in range(6)]
+    want = []
+    for x, l in zip(xs, ls):
+        want.append(layer.forward(x, l).clone())
+        torch.cuda.synchronize()
+    outs = [torch.empty_like(x) for x in xs]
+    for x, l, o in zip(xs, ls, outs):
+        layer.forward(x, l, out=o)
+    layer.check()
+    assert all(torch.equal(a, b) for a, b in zip(outs, want))
+    x, l, o = xs[0].clone(), ls[0].clone(), outs[0]
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        layer.forward(x, l, out=o)
+        layer.forward(o, l, out=o)
+    for i in range(3):
+        x.copy_(xs[i])
+        l.copy_(ls[i])
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(o, layer.forward(want[i], ls[i]))
+    del graph
+    comm.close()
