@@ -29,6 +29,7 @@ CUDA_SOURCES = [
     "kernels/a2av_kernel.cu",
     "kernels/a2av_eager.cu",
     "kernels/a2av_static.cu",
+    "kernels/a2av_local.cu",
     "kernels/moe_kernels.cu",
     "kernels/moe_local.cu",
     "kernels/grouped_gemm_sm100.cu",

@@ -108,6 +108,7 @@ int rbv_alltoallv(rbv_ctx_t ctx, int algo, int n, int r, int r2, int b, int b2, 
     ca.bytes_hint = bytes_hint;
     CallOptions opt;
     opt.grid = grid; opt.chunk_bytes = chunk_bytes; opt.flags = flags;
+    opt.allow_static = ctx->allow_static;
     opt.eager_max_bytes = ctx->eager;
     int rc = ctx->c->alltoallv(s, type_size, ca, opt, static_cast<cudaStream_t>(cuda_stream));
     if (rc) g_err = ctx->c->last_error();

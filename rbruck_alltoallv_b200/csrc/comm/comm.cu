@@ -245,6 +245,12 @@ int Context::alltoallv(const AlgoSpec& spec, int ts, const CallArgs& ca, const C
 }
 
 int Context::launch(const Prepared& pc, cudaStream_t stream) {
+  if (pc.is_local) {   // takes no part in the call numbering: it uses no flag, table or cell that a call number guards
+    const cudaError_t e = a2av_local_launch(pc.la, pc.grid, stream);
+    if (e == cudaSuccess) return 0;
+    last_error_ = std::string("kernel launch failed: ") + cudaGetErrorString(e);
+    return RBV_ERR_BAD_ARG;
+  }
   // cooperative_mode_: 1 always cooperative, 0 never (in-place calls excepted), -1 only for calls that need it
   const bool coop = cooperative_mode_ > 0 || (cooperative_mode_ < 0 && pc.cooperative);
   // The host passes the call number along (one trip to device memory less before the first byte moves).  A launch
@@ -294,6 +300,7 @@ int Context::prepare(const AlgoSpec& spec_in, int ts, const CallArgs& ca, const 
   const bool eager = opt.eager_max_bytes > 0;
   const unsigned long long emax = (opt.eager_max_bytes + 7) & ~7ull;
   out->is_static = false;
+  out->is_local = false;
   out->cooperative = true;
   if (eager) {
     if (inplace) { last_error_ = "the eager protocol does not take in-place calls"; return RBV_ERR_BAD_ARG; }
@@ -467,6 +474,35 @@ int Context::prepare(const AlgoSpec& spec_in, int ts, const CallArgs& ca, const 
   } else {
     ka.sendcounts = ca.sendcounts; ka.recvcounts = ca.recvcounts;
     ka.sdispls = ca.sdispls; ka.rdispls = ca.rdispls;
+  }
+
+  // A direct schedule among ranks of this process needs neither the exchange of counts nor the arrival counts of the
+  // dynamic kernel.  That kernel keeps the calls that ask for something of its own: a trace, the bulk-copy engine, an
+  // injected fault, `static` resolution switched off.
+  if (nproc_ == 1 && !eager && !inplace && !trace_ && absent_rank_ < 0 && bulk_mode_ == 0 && opt.allow_static &&
+      dp->plan.ncells == 0) {
+    LocalArgs& la = out->la;
+    std::memset(&la, 0, offsetof(LocalArgs, inl));
+    la.P = P_; la.type_size = ts;
+    la.inline_meta = (ka.flags & CALL_META_INLINE) ? 1 : 0;
+    if (la.inline_meta) la.inl = ka.inl;
+    la.chunk_bytes = align_up(opt.chunk_bytes, 16);
+    la.sendcounts = ka.sendcounts; la.recvcounts = ka.recvcounts;
+    la.sdispls = ka.sdispls; la.rdispls = ka.rdispls;
+    for (int r = 0; r < P_; r++) {
+      la.sendbuf[r] = static_cast<const char*>(ca.sendbufs[r]);
+      la.recvbuf[r] = static_cast<char*>(ca.recvbufs[r]);
+    }
+    la.heap[0] = heap_; la.ctrl_off = lay_.ctrl_off; la.host_status = host_status_dev_;
+    // one CTA per SM, or per chunk (2 KB and more) where the host knows that there are fewer
+    int grid = sm_count_;
+    if (send_bytes >= 0) grid = (int)std::min<long long>(grid, (long long)n + send_bytes / 2048);
+    if (opt.grid > 0) grid = std::min(opt.grid, sm_count_);
+    out->grid = std::max(1, grid);
+    out->eager = false;
+    out->cooperative = false;
+    out->is_local = true;
+    return 0;
   }
 
   // --- launch shape ---

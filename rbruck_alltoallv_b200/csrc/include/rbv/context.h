@@ -71,6 +71,9 @@ struct Prepared {
   bool is_static = false;       // runs the static kernel with `sa`; `ka` is unused then
   bool cooperative = true;      // launch mode this call needs (false: a plain launch is safe)
   StaticArgs sa;
+  unsigned static_items = 0;    // all items of the table, those that others lead to included
+  bool is_local = false;        // runs the local kernel with `la`; `ka` is unused then
+  LocalArgs la;
   void* owned_meta = nullptr;   // device copy of host count arrays that did not fit the kernel parameters
   void* owned_items = nullptr;  // device copy of the precomputed work-item table (eager protocol)
 };
@@ -227,6 +230,8 @@ cudaError_t a2av_launch(const KernelArgs& args, int grid, bool cooperative, cuda
 // implemented in kernels/a2av_static.cu
 cudaError_t a2av_static_configure(int occupancy, int* max_ctas_per_sm);
 cudaError_t a2av_static_launch(const StaticArgs& args, int grid, int occupancy, bool cooperative, cudaStream_t stream);
+// implemented in kernels/a2av_local.cu
+cudaError_t a2av_local_launch(const LocalArgs& args, int grid, cudaStream_t stream);
 // implemented in kernels/a2av_eager.cu
 cudaError_t a2av_eager_launch(const KernelArgs& args, int grid, bool cooperative, cudaStream_t stream);
 

@@ -219,6 +219,25 @@ struct KernelArgs {
   EagerItem inl_items[kInlineEagerItems];   // the first items of the table behind `items` (when there is one)
 };
 
+// Arguments of the local kernel (a2av_local.cu): a direct exchange among ranks of one process.  Counts and displacements
+// as in KernelArgs, for all P ranks.
+struct LocalArgs {
+  int P, type_size;
+  int inline_meta;                  // counts and displacements are in `inl`, not behind the pointers
+  int pad;
+  unsigned long long chunk_bytes;   // 0: chosen by the kernel from the counts
+  const int* sendcounts;
+  const int* recvcounts;            // may be null (no truncation check)
+  const long long* sdispls;
+  const long long* rdispls;
+  const char* sendbuf[kMaxRanks];
+  char* recvbuf[kMaxRanks];
+  char* heap[1];                    // for failure notes
+  unsigned long long ctrl_off;
+  StatusBlock* host_status;
+  InlineMeta inl;
+};
+
 constexpr int kInlineItems = 128;  // the first items of a static call travel in the kernel parameters
 
 // One received block (or a piece of it) that the static kernel copies on, once everything has arrived, from the

@@ -473,6 +473,31 @@ def test_functional_api_with_automatic_choice():
             assert torch.equal(got[s * n:(s + 1) * n], torch.arange(d * n, (d + 1) * n, dtype=torch.int32) + 1000 * s)
 
 
+@pytest.mark.parametrize("device_counts", [False, True])
+@pytest.mark.parametrize("P,ts,shape", [(1, 4, "even"), (2, 1, "one"), (3, 8, "holes"), (8, 2, "zero"), (9, 4, "holes"),
+                                        (16, 2, "one"), (23, 1, "holes"), (64, 4, "even"), (64, 1, "holes")])
+def test_direct_one_shot_calls_of_one_process(P, ts, shape, device_counts):
+    """Count matrices at the edges of the local kernel: nothing to send, one block only, empty blocks between others,
+    blocks of one byte up to several rounds of chunks, counts as kernel parameters (P * P <= 64) and in memory; the
+    dynamic kernel, asked for by switching static resolution off, gives the same bytes."""
+    rng = np.random.default_rng(P * 10 + ts)
+    counts = np.zeros((P, P), dtype=np.int64)
+    if shape == "even":
+        counts[:] = 37
+    elif shape == "one":
+        counts[P - 1, 0] = (5 << 20) // ts + 3
+    elif shape == "holes":
+        counts = rng.integers(0, 3000, (P, P)) * rng.integers(0, 2, (P, P))
+    comm = get_comm(P)
+    for on in (1, 0):
+        comm._lib.rbv_ctx_set_static(comm._ctx, on)
+        try:
+            for kw in ({}, {"chunk_bytes": 100}, {"grid": 3}, {"with_recvcounts": False, "packed": False}):
+                run_case(P, "spreadout", ts, counts, device_counts=device_counts, **kw)
+        finally:
+            comm._lib.rbv_ctx_set_static(comm._ctx, 1)
+
+
 def test_ulysses_sequence_head_exchange_round_trip():
     from rbruck_alltoallv_b200.ops.ulysses import UlyssesExchange
     P, s_l, H, D = 4, 24, 8, 16
