@@ -164,7 +164,7 @@ void* rbv_prepare(rbv_ctx_t ctx, int algo, int n, int r, int r2, int b, int b2, 
 // 0 dynamic rendezvous kernel, 1 eager kernel, 2 static rendezvous kernel; out3 = grid, cooperative launch needed, items
 int rbv_prepared_info(void* prepared, long long* out3) {
   const Prepared* pc = static_cast<Prepared*>(prepared);
-  if (out3) { out3[0] = pc->grid; out3[1] = pc->cooperative ? 1 : 0; out3[2] = pc->is_static ? pc->sa.nitems : pc->ka.nitems; }
+  if (out3) { out3[0] = pc->grid; out3[1] = pc->cooperative ? 1 : 0; out3[2] = pc->is_static ? pc->static_items : pc->ka.nitems; }
   return pc->is_static ? 2 : (pc->eager ? 1 : 0);
 }
 int rbv_launch(rbv_ctx_t ctx, void* prepared, void* cuda_stream) {

@@ -649,6 +649,7 @@ namespace {
 // the byte count is cut into a whole number of rounds: with 64 KB chunks and 1.8 rounds a tenth of the warps would
 // work alone at the end.  Measured on B200: with fewer, larger chunks most warps idle and a 4 MB exchange takes
 // twice as long.
+constexpr unsigned long long kRelayChunk = 8 << 10;   // see prepare_static
 unsigned long long chunk_for(double work, int max_ctas) {
   const double warps = 1.0 * max_ctas * (kThreads / 32);
   const double rounds = std::max(1.0, std::ceil(work / (warps * 64.0 * 1024)));
@@ -712,16 +713,36 @@ int Context::prepare_static(const DevPlan* dp, int ts, const CallArgs& ca, const
     if (first_el) *first_el = f;
     return (unsigned long long)n * ts;
   };
+  // One process: the warp that stores a chunk into a staging cell also executes the hop that forwards it, which wants
+  // every cell to be written once, and read at most once and after that.
+  bool relay = nproc_ == 1 && ncells > 0 && !dp->has_parts;
+  if (relay) {
+    std::vector<unsigned char> state((size_t)P * ncells, 0);   // 0 empty, 1 written, 2 read
+    auto step = [&](int rank, int cell, unsigned char want) {
+      unsigned char& c = state[(size_t)rank * ncells + cell];
+      if (c++ != want) relay = false;
+    };
+    for (const Op& o : dp->h_ops) {
+      if (o.src_cell >= 0) step(o.src, o.src_cell, 1);
+      if (o.dst_cell >= 0) step(o.dst, o.dst_cell, 0);
+    }
+  }
+  constexpr unsigned kNoItem = ~0u;
+  std::vector<unsigned> stored(relay ? (size_t)P * ncells : 0, kNoItem);   // per cell: the item that stores its chunk 0
+  std::vector<unsigned> pred;                                             // per item: the item whose chunk it forwards
   // ---- chunk size: the same on every process (receivers count chunks), so it is derived from the busiest process ----
   unsigned long long chunk = opt.chunk_bytes;
   if (!chunk) {
     std::vector<double> work(nproc_, 0.0);
     for (const Op& o : dp->plan.ops) work[o.src / L] += (double)slice_bytes(o, nullptr);
     chunk = chunk_for(*std::max_element(work.begin(), work.end()), static_max_ctas_);
+    // What the resident warps have stored but not yet forwarded should still be in L2 when they read it.  Measured, 2
+    // layers, blocks up to 4 MB: chunks of 64 KB 167 us, 32 KB 155, 16 KB 144, 8 KB 138, 4 KB 156.
+    if (relay) chunk = std::min<unsigned long long>(chunk, kRelayChunk);
   }
   chunk = align_up(chunk, 16);
   const unsigned long long fpc = ncells > 0 ? lay_.flags_per_rank / (unsigned long long)ncells : 0;
-  if (ncells > 0) chunk = std::max<unsigned long long>(chunk, align_up((stride + fpc - 1) / fpc, 16));
+  if (ncells > 0 && !relay) chunk = std::max<unsigned long long>(chunk, align_up((stride + fpc - 1) / fpc, 16));
   if (chunk > 0xffffffffull) chunk = 0xfffffff0ull;
   auto nchunks = [&](unsigned long long bytes) { return (bytes + chunk - 1) / chunk; };
 
@@ -755,6 +776,7 @@ int Context::prepare_static(const DevPlan* dp, int ts, const CallArgs& ca, const
         const int lsrc = o.src - first, dproc = o.dst / L, ldst = o.dst - dproc * L;
         const unsigned long long off = k * chunk;
         StaticItem it{};
+        unsigned from = kNoItem;
         it.len = (unsigned)std::min<unsigned long long>(chunk, bytes - off);
         it.dst_rank = o.dst;
         unsigned fl = 0;
@@ -765,6 +787,10 @@ int Context::prepare_static(const DevPlan* dp, int ts, const CallArgs& ca, const
         } else {
           it.src = stage_addr(proc_, lsrc, o.src_cell) + off;
           it.wait_flag = (unsigned)((unsigned long long)lsrc * lay_.flags_per_rank + (unsigned long long)o.src_cell * fpc + k);
+          if (relay) {
+            it.wait_flag = kNoFlag;
+            from = stored[(size_t)lsrc * ncells + o.src_cell] + (unsigned)k;   // (the chunks of an op are consecutive items)
+          }
           fl |= ITEM_SRC_STAGE;
         }
         if (o.dst_cell < 0) {
@@ -774,15 +800,40 @@ int Context::prepare_static(const DevPlan* dp, int ts, const CallArgs& ca, const
         } else {
           it.dst = stage_addr(dproc, ldst, o.dst_cell) + off;
           it.signal_flag = (unsigned)((unsigned long long)ldst * lay_.flags_per_rank + (unsigned long long)o.dst_cell * fpc + k);
+          if (relay) {
+            it.signal_flag = kNoFlag;
+            if (k == 0) stored[(size_t)ldst * ncells + o.dst_cell] = (unsigned)items.size();
+          }
           fl |= ITEM_DST_STAGE;
         }
         if (dproc != proc_) fl |= ITEM_REMOTE;
         if (o.flags & kOpSelf) fl |= ITEM_SELF;
         it.flags = (unsigned short)(fl | (std::min<unsigned>(op_key_index(o), 255u) << 8));
         items.push_back(it);
+        if (relay) pred.push_back(from);
       }
     g0 = g1;
   }
+  // Chains: an item that stores a cell chunk leads to the one that forwards it.  The heads keep plan order and are what
+  // the warps are dealt; the others lie behind them.
+  size_t heads = items.size();
+  if (relay) {
+    std::vector<unsigned> at(items.size());
+    heads = 0;
+    for (size_t i = 0; i < items.size(); i++)
+      if (pred[i] == kNoItem) at[i] = (unsigned)heads++;
+    unsigned tail = (unsigned)heads;
+    for (size_t i = 0; i < items.size(); i++)
+      if (pred[i] != kNoItem) {
+        at[i] = tail++;
+        items[pred[i]].signal_flag = at[i];
+        items[pred[i]].flags |= ITEM_NEXT;
+      }
+    std::vector<StaticItem> sorted(items.size());
+    for (size_t i = 0; i < items.size(); i++) sorted[at[i]] = items[i];
+    items.swap(sorted);
+  }
+
   // chunks that land in the receive buffers of this process's ranks, from every process
   std::vector<unsigned long long> expect(L, 0);
   for (const Op& o : dp->plan.ops)
@@ -823,7 +874,8 @@ int Context::prepare_static(const DevPlan* dp, int ts, const CallArgs& ca, const
   std::memset(&sa, 0, sizeof sa);
   sa.P = P; sa.L = L; sa.nproc = nproc_; sa.proc = proc_;
   sa.flags = trace_ ? (unsigned)CALL_TRACE : 0u;
-  sa.nitems = (unsigned)items.size();
+  sa.nitems = (unsigned)heads;
+  out->static_items = (unsigned)items.size();
   sa.expect = static_cast<const unsigned long long*>(out->owned_items);
   sa.items = reinterpret_cast<const StaticItem*>(static_cast<char*>(out->owned_items) + head);
   sa.drain = reinterpret_cast<const DrainItem*>(static_cast<char*>(out->owned_items) + head + items_bytes);
@@ -840,14 +892,15 @@ int Context::prepare_static(const DevPlan* dp, int ts, const CallArgs& ca, const
   // warps of a few.  Several processes: 16 items per CTA (see the kernel).
   const bool spread = static_spread_ && nproc_ == 1;
   int grid = opt.grid > 0 ? opt.grid
-                          : (int)(spread ? items.size() : (items.size() + warps_per_cta - 1) / warps_per_cta);
+                          : (int)(spread ? heads : (heads + warps_per_cta - 1) / warps_per_cta);
   out->grid = std::max(1, std::min(grid, static_max_ctas_));
   out->is_static = true;
   out->eager = false;
   // Only items that forward a staged chunk wait for other items; those come later in the list than what they wait
   // for, on every process.  With one round of items per warp that order cannot block as long as CTAs start in index
   // order; several rounds per warp need all CTAs resident.
-  out->cooperative = ncells > 0 && items.size() > (size_t)out->grid * warps_per_cta;
+  // (Where a warp forwards what it stored itself nobody waits.)
+  out->cooperative = ncells > 0 && !relay && items.size() > (size_t)out->grid * warps_per_cta;
   return 0;
 }
 

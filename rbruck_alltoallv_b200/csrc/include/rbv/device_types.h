@@ -154,12 +154,13 @@ struct alignas(16) StaticItem {
   unsigned short flags;     // ITEM_* bits | key index << 8
   unsigned wait_flag;       // chunk flag of this process to wait for (index at parity 0), kNoFlag: none
   unsigned signal_flag;     // chunk flag on the destination's process to raise, kNoFlag: the chunk counts as an
-                            // arrival in dst_rank's receive buffer instead
+                            // arrival in dst_rank's receive buffer instead.  With ITEM_NEXT: index of the item that
+                            // forwards this chunk, which the same warp executes next (nobody waits for a flag)
 };
 static_assert(sizeof(StaticItem) == 32, "two 16-byte loads per item");
 constexpr unsigned kNoFlag = 0xffffffffu;
 enum ItemFlags : unsigned short {
-  ITEM_SRC_STAGE = 1, ITEM_DST_STAGE = 2, ITEM_REMOTE = 4, ITEM_SELF = 8,
+  ITEM_SRC_STAGE = 1, ITEM_DST_STAGE = 2, ITEM_REMOTE = 4, ITEM_SELF = 8, ITEM_NEXT = 16,
 };
 
 struct InlineMeta {
@@ -253,7 +254,7 @@ struct alignas(16) DrainItem {
 struct StaticArgs {
   int P, L, nproc, proc;
   unsigned flags;                       // CALL_TRACE
-  unsigned nitems;
+  unsigned nitems;                      // items dealt to warps (those that others lead to with ITEM_NEXT lie behind them)
   unsigned seq_hint, use_seq_hint;      // as in KernelArgs
   const StaticItem* items;              // issue order; item c is handled by warp c mod (warps in the grid)
   const unsigned long long* expect;     // [L] chunks that land in each local rank's receive buffer per call

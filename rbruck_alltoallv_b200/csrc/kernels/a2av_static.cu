@@ -20,7 +20,10 @@
 // Completion is the same as in the dynamic kernel (a2av_kernel.cu): chunks that land in a receive buffer are
 // tallied per CTA and added to the receiver's arrival counter behind one fence; the receiver's target for the
 // call was counted on the host.  When one process hosts every rank nothing is tallied or waited for: every delivery
-// is a store of this very launch, so the end of the kernel is the completion.  All waits are bounded.
+// is a store of this very launch, so the end of the kernel is the completion; and the warp that has stored a chunk into
+// a staging cell forwards it itself, hop by hop (ITEM_NEXT), so that no hop waits for a flag or a fence and a forwarded
+// chunk is read back from L2 (measured on one B200: radix-2 Bruck, 8 ranks, blocks up to 1 KB 8.4 -> 6.2 us; two-layer,
+// blocks up to 4 MB 165 -> 137 us).  All waits are bounded.
 #include <cuda_runtime.h>
 
 #include "kernels/primitives.cuh"
@@ -95,7 +98,11 @@ __global__ void __launch_bounds__(kThreads, MINB) a2av_static_kernel(const __gri
 
   bool alive = true;
   unsigned ready = 1u << a.proc;   // processes known to have entered this call
-  for (unsigned c = gwarp; c < a.nitems; c += nwarps) {
+  unsigned next = kNoFlag;         // the item that forwards what this warp has just stored
+  for (unsigned dealt = gwarp; next != kNoFlag || dealt < a.nitems;) {
+    const unsigned c = next != kNoFlag ? next : dealt;
+    if (next == kNoFlag) dealt += nwarps;
+    next = kNoFlag;
     union { uint4 q[2]; StaticItem it; } u;
     if (c < (unsigned)kInlineItems) {
       u.it = a.inl[c];
@@ -134,8 +141,11 @@ __global__ void __launch_bounds__(kThreads, MINB) a2av_static_kernel(const __gri
       char* dst = reinterpret_cast<char*>(it.dst) + ((it.flags & ITEM_DST_STAGE) ? (size_t)parity * a.lay.arena_bytes : 0);
       dev::group_copy(dst, src, it.len, lane, 32);
     }
-    __syncwarp();
-    if (lane == 0) {
+    __syncwarp();   // (also orders these stores before the loads of the warp's other lanes, when it forwards them)
+    if (it.flags & ITEM_NEXT) {
+      next = it.signal_flag;
+      if (trace && lane == 0) atomicMax(&tb->kend[kidx], dev::globaltimer());
+    } else if (lane == 0) {
       if (it.signal_flag == kNoFlag) { if (multi) atomicAdd(&s_arrived[it.dst_rank], 1u); }
       else if (ok) dev::signal_store(flag_of(a, dproc, parity, it.signal_flag), flagv, remote);
       if (trace) atomicMax(&tb->kend[kidx], dev::globaltimer());

@@ -498,6 +498,20 @@ def test_direct_one_shot_calls_of_one_process(P, ts, shape, device_counts):
             comm._lib.rbv_ctx_set_static(comm._ctx, 1)
 
 
+@pytest.mark.parametrize("chunk_bytes", [0, 16, 400])
+@pytest.mark.parametrize("algo,kw", [("rbruck", dict(r=2)), ("tuna2", dict(r=3, b=1)), ("ttpl_bt_s1", dict(n=4, r=2)),
+                                     ("ttpl_bt", dict(n=2, r=2)), ("merge", dict(n=4))])
+def test_persistent_relays_of_one_process(algo, kw, chunk_bytes):
+    """A warp forwards the chunks it stored itself: chains of one to several hops, empty blocks, blocks of one element and
+    blocks of several chunks, repeated so that both parities of the staging cells are used."""
+    rng = np.random.default_rng(chunk_bytes)
+    counts = rng.integers(0, 900, (8, 8)) * rng.integers(0, 2, (8, 8))
+    counts[0, 7] = 1
+    counts[3, 4] = 20000
+    call = run_case(8, algo, 1, counts, persistent=True, launches=3, chunk_bytes=chunk_bytes, **kw)
+    assert call.kind == "static" and not call.cooperative
+
+
 def test_ulysses_sequence_head_exchange_round_trip():
     from rbruck_alltoallv_b200.ops.ulysses import UlyssesExchange
     P, s_l, H, D = 4, 24, 8, 16
