@@ -239,8 +239,8 @@ __global__ void __launch_bounds__(kThreads, 1) a2av_eager_kernel(const __grid_co
         const size_t off = (size_t)k * chunk;
         if (off < bytes) {
           const size_t len = min(chunk, bytes - off);
-          dev::group_copy(a.heap[a.proc] + a.recvoff[lsrc] + (size_t)rdispls[(size_t)lsrc * P + o.origin] * ts + off,
-                          a.sendbuf[lsrc] + (size_t)sdispls[(size_t)lsrc * P + o.dest] * ts + off, len, lane, 32);
+          dev::warp_copy(a.heap[a.proc] + a.recvoff[lsrc] + (size_t)rdispls[(size_t)lsrc * P + o.origin] * ts + off,
+                          a.sendbuf[lsrc] + (size_t)sdispls[(size_t)lsrc * P + o.dest] * ts + off, len, lane);
         }
         if (trace && lane == 0) atomicMax(&tb->kend[kidx], dev::globaltimer());
         continue;

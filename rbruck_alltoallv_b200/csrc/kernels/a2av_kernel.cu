@@ -397,9 +397,9 @@ __global__ void __launch_bounds__(kThreads, 1) a2av_kernel(const __grid_constant
           }
           r = __shfl_sync(0xffffffffu, r, 0);
           if (r != dev::WAIT_OK) { ok = false; alive = false; }
-          else if (len > body) dev::group_copy(dst + off + body, src + off + body, len - body, lane, 32);
+          else if (len > body) dev::warp_copy(dst + off + body, src + off + body, len - body, lane);
         } else {
-          dev::group_copy(dst + off, src + off, len, lane, 32);
+          dev::warp_copy(dst + off, src + off, len, lane);
         }
       }
       __syncwarp();

@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(kThreads, MINB) a2av_static_kernel(const __gri
     if (ok && it.len) {
       const char* src = reinterpret_cast<const char*>(it.src) + ((it.flags & ITEM_SRC_STAGE) ? (size_t)parity * a.lay.arena_bytes : 0);
       char* dst = reinterpret_cast<char*>(it.dst) + ((it.flags & ITEM_DST_STAGE) ? (size_t)parity * a.lay.arena_bytes : 0);
-      dev::group_copy(dst, src, it.len, lane, 32);
+      dev::warp_copy<MINB == 1 ? 8 : 4>(dst, src, it.len, lane);
     }
     __syncwarp();   // (also orders these stores before the loads of the warp's other lanes, when it forwards them)
     if (it.flags & ITEM_NEXT) {
@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(kThreads, MINB) a2av_static_kernel(const __gri
       if (all_ok)
         for (unsigned c = warp; c < a.ndrain; c += warps_per_cta) {
           const DrainItem di = a.drain[c];
-          dev::group_copy(reinterpret_cast<char*>(di.dst), reinterpret_cast<const char*>(di.src), di.len, lane, 32);
+          dev::warp_copy(reinterpret_cast<char*>(di.dst), reinterpret_cast<const char*>(di.src), di.len, lane);
         }
     }
     __syncthreads();

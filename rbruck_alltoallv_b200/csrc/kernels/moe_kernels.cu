@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(kMoeThreads) moe_dispatch_kernel(const __grid_
     char* dst = c.heap[owner] + a.xrecv_off + (size_t)pos * row_bytes;
     if (a.ret_off && lane == 0)
       reinterpret_cast<unsigned*>(c.heap[owner] + a.ret_off)[pos] = ((unsigned)c.proc << 24) | (unsigned)r;
-    dev::group_copy(dst, a.x + (size_t)(r >> 1) * row_bytes, row_bytes, lane, 32);
+    dev::warp_copy(dst, a.x + (size_t)(r >> 1) * row_bytes, row_bytes, lane);
   }
   // completion: the last CTA tells every process that this rank's rows are in place, then waits for all ranks
   __syncthreads();
@@ -470,8 +470,7 @@ __global__ void __launch_bounds__(kMoeThreads) moe_dispatch_streamed_kernel(cons
     const int owner = e / a.El;
     if (lane == 0) a.slot[r] = pos;
     if (pos < a.capacity_rows)
-      dev::group_copy(c.heap[owner] + a.xrecv_off + (size_t)pos * row_bytes, a.x + (size_t)(r >> 1) * row_bytes, row_bytes,
-                      lane, 32);
+      dev::warp_copy(c.heap[owner] + a.xrecv_off + (size_t)pos * row_bytes, a.x + (size_t)(r >> 1) * row_bytes, row_bytes, lane);
     else if (lane == 0) moe_fail(c, 4, e);
     __syncwarp();
     // the row counts as landed once its stores are visible on the owner (a row that did not fit is counted too,

@@ -1,4 +1,4 @@
-// Device primitives: system-scope signal / bounded wait, CTA-wide byte copy for arbitrary alignment.
+// Device primitives: system-scope signal / bounded wait, byte copies of arbitrary alignment.
 //
 // Every wait is bounded by a %globaltimer deadline and also leaves when the context's abort flag
 // is raised; it never traps.  On expiry the caller records a status and the kernel runs to its
@@ -76,7 +76,7 @@ __device__ __forceinline__ WaitResult wait_ge(const T* p, T target, const WaitCf
   }
 }
 
-// ---- CTA-wide copy ---------------------------------------------------------------------------
+// ---- copies ---------------------------------------------------------------------------
 __device__ __forceinline__ uint4 ld_cg_v4(const uint4* p) {
   uint4 v;
   asm volatile("ld.global.cg.v4.u32 {%0,%1,%2,%3}, [%4];"
@@ -93,110 +93,107 @@ __device__ __forceinline__ unsigned char ld_cg_u8(const unsigned char* p) {
   return (unsigned char)v;
 }
 
-template <int WO>
-__device__ __forceinline__ uint4 shift_words(const uint4& a, const uint4& b, unsigned bits) {
-  // the 16 bytes that start WO words + bits/8 bytes into the 32-byte pair (a, b)
-  const unsigned w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-  uint4 o;
-  o.x = __funnelshift_r(w[WO + 0], w[WO + 1], bits);
-  o.y = __funnelshift_r(w[WO + 1], w[WO + 2], bits);
-  o.z = __funnelshift_r(w[WO + 2], w[WO + 3], bits);
-  o.w = __funnelshift_r(w[WO + 3], w[WO + 4], bits);
-  return o;
+// The 16 bytes that start `sh` (0..15) bytes into the 32-byte pair (a, b).
+__device__ __forceinline__ uint4 shift16(const uint4& a, const uint4& b, unsigned sh) {
+  unsigned w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+  #pragma unroll
+  for (int i = 0; i < 6; i++) w[i] = (sh & 8u) ? w[i + 2] : w[i];
+  #pragma unroll
+  for (int i = 0; i < 5; i++) w[i] = (sh & 4u) ? w[i + 1] : w[i];
+  const unsigned bits = (sh & 3u) * 8u;
+  return make_uint4(__funnelshift_r(w[0], w[1], bits), __funnelshift_r(w[1], w[2], bits),
+                    __funnelshift_r(w[2], w[3], bits), __funnelshift_r(w[3], w[4], bits));
 }
 
-// Source and destination differ in their phase inside a 16-byte vector: output vector i is cut out of the
-// aligned source vectors i and i + 1.  Vector i + 1 is what the next lane loads as its own vector i, so it comes
-// by shuffle; only the last lane of a warp (and the lane that holds the last vector) loads it.  That keeps the
-// traffic from L2 at one vector per vector written.  All lanes of a warp must call this together, with
-// consecutive `tid` in consecutive lanes and `nt` a multiple of 32.
-template <int WO>
-__device__ __forceinline__ void copy_shifted(uint4* d, const uint4* s, size_t nvec, unsigned bits,
-                                             unsigned tid, unsigned nt) {
-  constexpr int U = 4;
-  const bool last_lane = (tid & 31u) == 31u;
-  for (size_t base = 0; base < nvec; base += (size_t)U * nt) {   // same trip count for every lane
-    uint4 a[U], b[U];
+// Output vectors [base, base + 32 V) of a warp's copy, those of them that lie in [0, nvec).  s is aligned; output vector i
+// is source vector i (sh = 0) or is cut out of source vectors i and i + 1 at byte sh, where vector i + 1 comes by shuffle
+// from the lane that loaded it.  ALL: the range lies inside.  `between` runs when the loads have been issued.
+template <int V, bool ALL, typename F>
+__device__ __forceinline__ void copy_round(uint4* o, const uint4* s, long long base, long long nvec, unsigned sh, unsigned lane,
+                                           F&& between) {
+  const long long i0 = base + lane, end = nvec + (sh ? 1 : 0);   // a shifted copy also reads the vector behind the last
+  uint4 v[V], more = make_uint4(0u, 0u, 0u, 0u);
+  #pragma unroll
+  for (int j = 0; j < V; j++) {
+    if (!ALL) v[j] = more;
+    if (ALL || (i0 + j * 32 >= 0 && i0 + j * 32 < end)) v[j] = ld_cg_v4(s + i0 + j * 32);
+  }
+  if (sh && lane == 0 && base + V * 32 < end) more = ld_cg_v4(s + base + V * 32);
+  between();
+  if (sh == 0) {
     #pragma unroll
-    for (int j = 0; j < U; j++) {
-      const size_t i = base + (size_t)j * nt + tid;
-      a[j] = make_uint4(0u, 0u, 0u, 0u);
-      b[j] = a[j];
-      if (i < nvec) {
-        a[j] = ld_cg_v4(s + i);
-        if (last_lane || i + 1 >= nvec) b[j] = ld_cg_v4(s + i + 1);
-      }
-    }
-    #pragma unroll
-    for (int j = 0; j < U; j++) {
-      const size_t i = base + (size_t)j * nt + tid;
-      uint4 n;
-      n.x = __shfl_down_sync(0xffffffffu, a[j].x, 1);
-      n.y = __shfl_down_sync(0xffffffffu, a[j].y, 1);
-      n.z = __shfl_down_sync(0xffffffffu, a[j].z, 1);
-      n.w = __shfl_down_sync(0xffffffffu, a[j].w, 1);
-      if (!(last_lane || i + 1 >= nvec)) b[j] = n;
-      if (i < nvec) st_v4(d + i, shift_words<WO>(a[j], b[j], bits));
-    }
+    for (int j = 0; j < V; j++)
+      if (ALL || (i0 + j * 32 >= 0 && i0 + j * 32 < nvec)) st_v4(o + i0 + j * 32, v[j]);
+    return;
+  }
+  #pragma unroll
+  for (int j = 0; j < V; j++) {
+    // the next vector: of the next lane, and for the last lane of lane 0's next one
+    const uint4 give = lane == 0 ? (j + 1 < V ? v[j + 1 < V ? j + 1 : j] : more) : v[j];
+    uint4 next;
+    next.x = __shfl_sync(0xffffffffu, give.x, (lane + 1) & 31u);
+    next.y = __shfl_sync(0xffffffffu, give.y, (lane + 1) & 31u);
+    next.z = __shfl_sync(0xffffffffu, give.z, (lane + 1) & 31u);
+    next.w = __shfl_sync(0xffffffffu, give.w, (lane + 1) & 31u);
+    if (ALL || (i0 + j * 32 >= 0 && i0 + j * 32 < nvec)) st_v4(o + i0 + j * 32, shift16(v[j], next, sh));
   }
 }
 
-// Copies n bytes with a group of nt threads (tid = index in the group: a warp or a whole CTA).
-// dst and src may have any alignment, relative to each other too: stores are 16-byte aligned
-// vectors, loads are aligned vectors re-assembled with funnel shifts when the two phases differ.
-// Loads bypass L1 (the source may have been written by another GPU).  The caller synchronises.
-__device__ __forceinline__ void group_copy(char* dst, const char* src, size_t n, unsigned tid, unsigned nt) {
+// Copies n bytes with one warp.  dst and src may have any alignment, relative to each other too; stores are 16-byte
+// aligned vectors.  Loads bypass L1 (the source may have been written by another GPU).  All lanes call it together.
+//
+// Bound by the latency of memory for short blocks and by the bytes in flight for long ones, so that every load of a round
+// is issued before anything is stored: the bytes in front of and behind the vectors, and up to U vectors per lane whatever
+// the alignment.  (Bytes, the vectors in front of the first line, and the rest one after the other cost a block three
+// trips to memory, and a misaligned copy, which blocks of bf16 elements usually are, had four vectors per lane in
+// flight.)  Measured on one B200, persistent calls of 8 ranks: Zipf blocks up to 64 KB 6.1 -> 4.65 us; blocks up to 4 MB
+// of bf16, direct 103 -> 94 us, two-layer 137 -> 117 us.  A short rest takes a round of its own size: with the
+// instructions of a full one Bruck over blocks of up to 1 KB took 10.0 instead of 6.2 us.  U = 16 moves long blocks
+// another 7 % faster in a2av_local.cu and nothing else (a2av_static.cu: two-layer 117 -> 123 us).
+// The first vector of every round lies on a 128-byte line of the destination (blocks of 1 KB and more): a peer GPU
+// receives a line that is written in two pieces as two NVLink packets with one header each, which costs a fifth of the
+// link when 512-byte warp stores start in the middle of a line.
+template <int U = 8>
+__device__ __forceinline__ void warp_copy(char* dst, const char* src, size_t n, unsigned lane) {
   if (n == 0) return;
   size_t head = (16 - ((uintptr_t)dst & 15)) & 15;
   if (head > n) head = n;
-  if (tid < head) dst[tid] = (char)ld_cg_u8((const unsigned char*)src + tid);
-  dst += head; src += head; n -= head;
-  const size_t nvec = n >> 4;
-  if (nvec) {
-    uint4* d = reinterpret_cast<uint4*>(dst);
-    const unsigned sh = (unsigned)((uintptr_t)src & 15);
-    // Vectors in front of the first 128-byte line boundary of the destination go first, so that every store
-    // instruction of the main loops covers whole lines.  A peer GPU receives a line that is written in two pieces
-    // as two NVLink packets with one header each, which costs a fifth of the link when 512-byte warp stores start
-    // in the middle of a line.
-    size_t hv = ((128 - ((uintptr_t)dst & 127)) & 127) >> 4;
-    if (hv > nvec || nvec < 64) hv = 0;
-    if (sh == 0) {
-      const uint4* s = reinterpret_cast<const uint4*>(src);
-      if (tid < hv) st_v4(d + tid, ld_cg_v4(s + tid));
-      size_t i = hv + tid;
-      // 8 independent 16-byte loads in flight per thread (4 KB per warp) before the first store
-      for (; i + 7 * (size_t)nt < nvec; i += 8 * (size_t)nt) {
-        uint4 v[8];
-        #pragma unroll
-        for (int j = 0; j < 8; j++) v[j] = ld_cg_v4(s + i + j * (size_t)nt);
-        #pragma unroll
-        for (int j = 0; j < 8; j++) st_v4(d + i + j * (size_t)nt, v[j]);
-      }
-      for (; i + 3 * (size_t)nt < nvec; i += 4 * (size_t)nt) {
-        uint4 v0 = ld_cg_v4(s + i), v1 = ld_cg_v4(s + i + nt);
-        uint4 v2 = ld_cg_v4(s + i + 2 * nt), v3 = ld_cg_v4(s + i + 3 * nt);
-        st_v4(d + i, v0); st_v4(d + i + nt, v1);
-        st_v4(d + i + 2 * nt, v2); st_v4(d + i + 3 * nt, v3);
-      }
-      for (; i < nvec; i += nt) st_v4(d + i, ld_cg_v4(s + i));
-    } else {
-      const uint4* s = reinterpret_cast<const uint4*>(src - sh);
-      const unsigned bits = (sh & 3u) * 8u;
-      switch (sh >> 2) {
-        case 0: if (hv) copy_shifted<0>(d, s, hv, bits, tid, nt); copy_shifted<0>(d + hv, s + hv, nvec - hv, bits, tid, nt); break;
-        case 1: if (hv) copy_shifted<1>(d, s, hv, bits, tid, nt); copy_shifted<1>(d + hv, s + hv, nvec - hv, bits, tid, nt); break;
-        case 2: if (hv) copy_shifted<2>(d, s, hv, bits, tid, nt); copy_shifted<2>(d + hv, s + hv, nvec - hv, bits, tid, nt); break;
-        default: if (hv) copy_shifted<3>(d, s, hv, bits, tid, nt); copy_shifted<3>(d + hv, s + hv, nvec - hv, bits, tid, nt); break;
-      }
+  char* const d = dst + head;
+  const char* const from = src + head;
+  const long long nvec = (long long)((n - head) >> 4);
+  const unsigned tail = (unsigned)(n - head) & 15u;
+  unsigned char first = 0, last = 0;
+  if (lane < head) first = ld_cg_u8((const unsigned char*)src + lane);
+  if (lane < tail) last = ld_cg_u8((const unsigned char*)from + (nvec << 4) + lane);
+  bool ragged = true;                          // the bytes around the vectors are still to be stored
+  auto ends = [&]() {
+    if (ragged) {
+      if (lane < head) dst[lane] = (char)first;
+      if (lane < tail) d[(nvec << 4) + lane] = (char)last;
     }
+    ragged = false;
+  };
+  const unsigned sh = (unsigned)((uintptr_t)from & 15);
+  const uint4* const s = reinterpret_cast<const uint4*>(from - sh);
+  uint4* const o = reinterpret_cast<uint4*>(d);
+  // vector of lane 0 in the first round
+  long long base = nvec >= 64 ? -(long long)(((uintptr_t)d >> 4) & 7) : 0;
+  if (base < 0 && nvec - base > 4 * 32) {
+    copy_round<U, false>(o, s, base, nvec, sh, lane, ends);
+    base += U * 32;
   }
-  const size_t done = nvec << 4, tail = n - done;
-  if (tid < tail) dst[done + tid] = (char)ld_cg_u8((const unsigned char*)src + done + tid);
+  for (; base + U * 32 <= nvec; base += U * 32) copy_round<U, true>(o, s, base, nvec, sh, lane, ends);
+  if (nvec - base > 4 * 32) copy_round<U, false>(o, s, base, nvec, sh, lane, ends);
+  else if (nvec - base > 32) copy_round<4, false>(o, s, base, nvec, sh, lane, ends);
+  else if (nvec - base > 0) copy_round<1, false>(o, s, base, nvec, sh, lane, ends);
+  else ends();
 }
 
+// The same with all warps of a CTA, a piece each.  The caller synchronises.
 __device__ __forceinline__ void cta_copy(char* dst, const char* src, size_t n) {
-  group_copy(dst, src, n, threadIdx.x, blockDim.x);
+  const unsigned warps = blockDim.x >> 5, w = threadIdx.x >> 5;
+  const size_t per = ((n + warps - 1) / warps + 127) & ~(size_t)127, lo = w * per;
+  if (lo < n) warp_copy(dst + lo, src + lo, lo + per <= n ? per : n - lo, threadIdx.x & 31u);
 }
 
 // Index of the op that owns work item c: the largest i in [lo, n) with prefix[i] <= c (prefix is an exclusive scan

@@ -473,6 +473,21 @@ def test_functional_api_with_automatic_choice():
             assert torch.equal(got[s * n:(s + 1) * n], torch.arange(d * n, (d + 1) * n, dtype=torch.int32) + 1000 * s)
 
 
+@pytest.mark.parametrize("persistent", [False, True])
+@pytest.mark.parametrize("ts", [1, 2, 16])
+def test_copies_of_every_length_and_phase(ts, persistent):
+    """Blocks around the sizes at which the warp copy changes its way (bytes only, one vector, a line, one and several
+    rounds of 8 or 16 vectors per lane) at random phases of source and destination, with gaps that have to stay intact."""
+    edges = [0, 1, 7, 15, 16, 17, 31, 33, 47, 127, 129, 511, 513, 1007, 1023, 1024, 1025, 1040, 1151, 4095, 4097, 4112,
+             8176, 8191, 8192, 8193, 8208, 8320, 12289, 16383, 16400, 20000]
+    P = 8
+    for seed in range(3):
+        rng = np.random.default_rng(seed)
+        sizes = rng.choice(edges, (P, P)) if ts < 16 else rng.choice(edges, (P, P)) // 16
+        for algo, kw in (("spreadout", {}), ("rbruck", dict(r=2))):
+            run_case(P, algo, ts, sizes, packed=False, seed=seed, persistent=persistent, **kw)
+
+
 @pytest.mark.parametrize("device_counts", [False, True])
 @pytest.mark.parametrize("P,ts,shape", [(1, 4, "even"), (2, 1, "one"), (3, 8, "holes"), (8, 2, "zero"), (9, 4, "holes"),
                                         (16, 2, "one"), (23, 1, "holes"), (64, 4, "even"), (64, 1, "holes")])
