@@ -6,6 +6,7 @@
 // count patterns of such an exchange (examples/FFT_distribution.cpp:66-87) and leaves packing to the caller.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
 #include "api/ctx_internal.h"
@@ -31,6 +32,15 @@ struct TransposeArgs {
   int elem_size;                // 4, 8 or 16
   rbv_box box[kMaxProcs];
 };
+
+// Tiles of a box, at most (a lead of up to one line may add one along the destination-fastest dimension).
+long long tiles_of(const rbv_box& b, int elem_size) {
+  if (b.n0 <= 0 || b.n1 <= 0 || b.n2 <= 0) return 0;
+  if (b.t2 == 1) return (long long)b.n0 * b.n1 * ((b.n2 + kThreadsT - 1) / kThreadsT);
+  const int edge = elem_size == 16 ? TS : 64, line = 128 / elem_size;
+  const int nf = b.t1 == 1 ? b.n1 : b.n0, no = b.t1 == 1 ? b.n0 : b.n1;
+  return (long long)no * ((nf + line + edge - 1) / edge) * ((b.n2 + edge - 1) / edge);
+}
 
 // TF x TK tile: TF elements along the destination's contiguous dimension, TK along the source's (dimension 2).
 template <typename T, int TF, int TK>
@@ -117,6 +127,9 @@ __global__ void __launch_bounds__(kThreadsT) transpose_exchange_kernel(const __g
   if (a.elem_size == 8) move_boxes<unsigned long long, 64, 64>(a, reinterpret_cast<unsigned long long*>(tile_raw));
   else if (a.elem_size == 4) move_boxes<unsigned, 64, 64>(a, reinterpret_cast<unsigned*>(tile_raw));
   else move_boxes<uint4, TS, TS>(a, reinterpret_cast<uint4*>(tile_raw));
+  // One process: every box is stored by this very launch, so its end is the completion.  (Counting the CTAs' exits on
+  // one word cost a small grid more than moving its tiles.)
+  if (a.nproc == 1) return;
   // completion: last CTA signals every process, then waits for all of them (bounded)
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -163,6 +176,7 @@ extern "C" int rbv_transpose_exchange(rbv_ctx_t ctx, const void* src, unsigned l
   a.dst_off = dst_off;
   a.elem_size = elem_size;
   int grid = max_ctas > 0 ? max_ctas : c.sm_count() * 6;
+  if (c.nproc() == 1) grid = (int)std::max<long long>(1, std::min<long long>(grid, tiles_of(boxes[0], elem_size)));
   transpose_exchange_kernel<<<grid, kThreadsT, 0, static_cast<cudaStream_t>(stream)>>>(a);
   return (int)cudaGetLastError();
 }
