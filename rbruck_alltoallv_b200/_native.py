@@ -82,3 +82,11 @@ def cuda_lib():
             from ._cuda_decl import declare_cuda
             declare_cuda(_cuda)
         return _cuda
+
+
+def current_stream(device: int) -> int:
+    """Handle of torch's current stream on a device.  (``torch.cuda.current_stream`` makes a Stream object for it first,
+    which takes longer than many of the launches here.)"""
+    import torch
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    return raw(device) if raw is not None else torch.cuda.current_stream(device).cuda_stream

@@ -84,6 +84,10 @@ int rbv_ctx_info(rbv_ctx_t ctx, long long* o) {
 }
 void* rbv_ctx_heap(rbv_ctx_t ctx, int proc) { return ctx->c->peer_heap(proc); }
 int rbv_ctx_in_heap(rbv_ctx_t ctx, const void* p, size_t bytes) { return ctx->c->in_heap(p, bytes ? bytes : 1) ? 1 : 0; }
+void rbv_ctx_user_span(rbv_ctx_t ctx, void** out2) {
+  out2[0] = ctx->c->heap() + ctx->c->layout().user_off;
+  out2[1] = ctx->c->heap() + ctx->c->layout().total_bytes;
+}
 void* rbv_symm_alloc(rbv_ctx_t ctx, size_t bytes) { return ctx->c->symm_alloc(bytes); }
 int rbv_symm_free(rbv_ctx_t ctx, void* p) { return ctx->c->symm_free(p); }
 rbv_comm_t rbv_comm(rbv_ctx_t ctx, int local_rank) {

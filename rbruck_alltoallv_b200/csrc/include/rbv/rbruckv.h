@@ -64,6 +64,8 @@ int rbv_ctx_reset(rbv_ctx_t ctx);
 int rbv_ctx_info(rbv_ctx_t ctx, long long* out8); /* P, L, nproc, proc, device, seq, max_ctas, sm_count */
 void* rbv_ctx_heap(rbv_ctx_t ctx, int proc);
 int rbv_ctx_in_heap(rbv_ctx_t ctx, const void* ptr, size_t bytes); /* 1 if [ptr, ptr+bytes) lies in the symmetric heap */
+/* First byte and end of the part of this process's heap that rbv_symm_alloc hands out. */
+void rbv_ctx_user_span(rbv_ctx_t ctx, void** out2);
 void* rbv_symm_alloc(rbv_ctx_t ctx, size_t bytes);
 int rbv_symm_free(rbv_ctx_t ctx, void* ptr);
 rbv_comm_t rbv_comm(rbv_ctx_t ctx, int local_rank);

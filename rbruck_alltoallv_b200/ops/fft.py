@@ -95,7 +95,7 @@ class PencilTranspose:
         return boxes
 
     def _run(self, src, off, boxes, err):
-        st = C.c_void_p(torch.cuda.current_stream(src.device).cuda_stream)
+        st = _native.current_stream(src.device.index)
         rc = self.lib.rbv_transpose_exchange(self.comm._ctx, C.c_void_p(src.data_ptr()), off, self.esize, boxes,
                                              C.c_void_p(err.data_ptr()), 0, st)
         if rc:

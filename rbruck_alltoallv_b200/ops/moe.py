@@ -43,7 +43,7 @@ def grouped_gemm(A: torch.Tensor, B: torch.Tensor, group_start: torch.Tensor, gr
         out = torch.empty(M, n_out, dtype=torch.bfloat16, device=A.device)
     if error is None:
         error = torch.zeros(1, dtype=torch.int32, device=A.device)
-    st = torch.cuda.current_stream(A.device).cuda_stream
+    st = _native.current_stream(A.device.index)
     prev = None
     if pair is not None and ready is None:
         prev = lib.rbv_grouped_gemm_pair_enabled()
@@ -68,7 +68,7 @@ def quantize_rows_fp8(x: torch.Tensor, used: Optional[torch.Tensor] = None):
     rows, K = x.shape
     q = torch.empty(rows, K, dtype=torch.uint8, device=x.device)
     sc = torch.empty(K // 128, rows, dtype=torch.float32, device=x.device)
-    st = torch.cuda.current_stream(x.device).cuda_stream
+    st = _native.current_stream(x.device.index)
     rc = lib.rbv_quantize_used_rows_fp8(_p(x), rows, _p(used), K, x.stride(0), _p(q), _p(sc), C.c_void_p(st))
     if rc:
         raise RuntimeError(f"quantisation launch failed (CUDA error {rc})")
@@ -115,7 +115,7 @@ def grouped_gemm_fp8(Aq: torch.Tensor, a_scale_t: torch.Tensor, Bq: torch.Tensor
         out = torch.empty(M, n_out, dtype=torch.bfloat16, device=Aq.device)
     if error is None:
         error = torch.zeros(1, dtype=torch.int32, device=Aq.device)
-    st = torch.cuda.current_stream(Aq.device).cuda_stream
+    st = _native.current_stream(Aq.device.index)
     prev = None
     if pair is not None:
         prev = lib.rbv_grouped_gemm_pair_enabled()
@@ -143,7 +143,7 @@ def quantize_rows_mxfp8(x: torch.Tensor):
     rows, K = x.shape
     q = torch.empty(rows, K, dtype=torch.uint8, device=x.device)
     sf = torch.empty(K // 128, (rows + 127) // 128 * 128, dtype=torch.int32, device=x.device)
-    st = torch.cuda.current_stream(x.device).cuda_stream
+    st = _native.current_stream(x.device.index)
     rc = lib.rbv_quantize_rows_mxfp8(_p(x), rows, K, x.stride(0), _p(q), _p(sf), C.c_void_p(st))
     if rc:
         raise RuntimeError(f"MXFP8 quantisation launch failed (CUDA error {rc})")
@@ -228,7 +228,7 @@ def grouped_gemm_mxfp8(Aq: torch.Tensor, sfa: torch.Tensor, Bq: torch.Tensor, sf
         out = torch.empty(M, n_out, dtype=torch.bfloat16, device=Aq.device)
     if error is None:
         error = torch.zeros(1, dtype=torch.int32, device=Aq.device)
-    st = torch.cuda.current_stream(Aq.device).cuda_stream
+    st = _native.current_stream(Aq.device.index)
     rc = lib.rbv_grouped_gemm_mxfp8(_p(Aq), _p(sfa), M, _p(Bq), _p(sfb), _p(out), _p(group_start), _p(group_rows),
                                     G, N, K, out.stride(0), 1 if swiglu else 0, _p(error), int(max_ctas),
                                     C.c_void_p(st))
@@ -257,7 +257,7 @@ def grouped_gemm_mxfp8_swiglu_q(Aq: torch.Tensor, sfa: torch.Tensor, Bq: torch.T
     assert out_q.shape == (M, N // 2) and out_q.stride(1) == 1 and out_sf.shape == (N // 256, mp) and out_sf.is_contiguous()
     if error is None:
         error = torch.zeros(1, dtype=torch.int32, device=Aq.device)
-    st = torch.cuda.current_stream(Aq.device).cuda_stream
+    st = _native.current_stream(Aq.device.index)
     rc = lib.rbv_grouped_gemm_mxfp8_swiglu_q(_p(Aq), _p(sfa), M, _p(Bq), _p(sfb), _p(out_q), _p(out_sf),
                                              _p(group_start), _p(group_rows), G, N, K, out_q.stride(0), _p(error),
                                              int(max_ctas), C.c_void_p(st))
@@ -381,7 +381,7 @@ class MoEExpertParallel:
         assert T == self.T and H == self.H and x.dtype == torch.bfloat16 and x.is_contiguous()
         assert logits.shape == (T, self.E) and logits.dtype == torch.float32 and logits.is_contiguous()
         lib, ctx = self.lib, self.comm._ctx
-        st = C.c_void_p(torch.cuda.current_stream(self.dev).cuda_stream)
+        st = C.c_void_p(_native.current_stream(self.comm.device))
         if out is None:
             out = torch.empty_like(x)
         local = self.P == 1 and not self.overlap

@@ -17,6 +17,8 @@ from typing import List, Sequence
 import numpy as np
 import torch
 
+from .. import _native
+
 
 class UlyssesExchange:
     def __init__(self, comm, seq_local: int, heads: int, head_dim: int, dtype=torch.bfloat16, algo: str = "spreadout",
@@ -51,7 +53,7 @@ class UlyssesExchange:
         return [x] if isinstance(x, torch.Tensor) else list(x)
 
     def _reshard(self, seq_side, head_side, to_head: bool) -> None:
-        st = C.c_void_p(torch.cuda.current_stream(self._device).cuda_stream)
+        st = _native.current_stream(self.comm.device)
         rc = self.comm._lib.rbv_reshard_heads(self.comm._ctx, seq_side, head_side, self.s_l, self._piece_bytes,
                                               1 if to_head else 0, st)
         if rc:

@@ -66,12 +66,11 @@ class PreparedCall:
         self.grid, self.cooperative, self.items = int(info[0]), bool(info[1]), int(info[2])
 
     def launch(self, stream: Optional[torch.cuda.Stream] = None) -> None:
-        st = stream or torch.cuda.current_stream(self._dev)
-        rc = self._launch(self._ctx, self._h, C.c_void_p(st.cuda_stream))
+        rc = self._launch(self._ctx, self._h, stream.cuda_stream if stream else _native.current_stream(self._dev))
         if rc:
             raise CommError("launch failed: " + self._comm._lib.rbv_last_error().decode())
         if self._mirrored and self.kind != "static":     # the static kernel has copied them on itself
-            with torch.cuda.stream(st):
+            with torch.cuda.stream(stream or torch.cuda.current_stream(self._dev)):
                 for t, bt in self._mirrored:
                     t.reshape(-1).view(torch.uint8).copy_(bt, non_blocking=True)
 
@@ -134,6 +133,9 @@ class Communicator:
             self._enable_nvls()
         info = (C.c_longlong * 8)()
         self._lib.rbv_ctx_info(self._ctx, info)
+        span = (C.c_void_p * 2)()
+        self._lib.rbv_ctx_user_span(self._ctx, span)
+        self._heap_span = (int(span[0]), int(span[1]))
         self.max_ctas = int(info[6])
         self.sm_count = int(info[7])
 
@@ -290,7 +292,8 @@ class Communicator:
             def dev(a, dt):
                 if a is None:
                     return None
-                a = a.to(dt).contiguous().view(L, P)
+                if a.dtype != dt or not a.is_contiguous() or a.dim() != 2 or a.shape[0] != L or a.shape[1] != P:
+                    a = a.to(dt).contiguous().view(L, P)
                 keep.append(a)
                 return a
             sc, rc = dev(sendcounts, torch.int32), dev(recvcounts, torch.int32)
@@ -299,22 +302,27 @@ class Communicator:
                 raise ValueError("device-resident counts need explicit displacements")
             ptrs = (sc.data_ptr(), rc.data_ptr() if rc is not None else None, sd.data_ptr(), rd.data_ptr())
         else:
-            sc = np.ascontiguousarray(np.asarray(sendcounts, dtype=np.int32).reshape(L, P))
-            rc = None if recvcounts is None else np.ascontiguousarray(np.asarray(recvcounts, dtype=np.int32).reshape(L, P))
+            def host(a, dt):
+                if type(a) is np.ndarray and a.dtype == dt and a.shape == (L, P) and a.flags.c_contiguous:
+                    return a
+                return np.ascontiguousarray(np.asarray(a, dtype=dt).reshape(L, P))
+            sc = host(sendcounts, np.int32)
+            rc = None if recvcounts is None else host(recvcounts, np.int32)
             if sdispls is None:
                 sd = np.zeros((L, P), dtype=np.int64)
                 sd[:, 1:] = np.cumsum(sc[:, :-1], axis=1)
             else:
-                sd = np.ascontiguousarray(np.asarray(sdispls, dtype=np.int64).reshape(L, P))
+                sd = host(sdispls, np.int64)
             if rdispls is None:
                 if rc is None:
                     raise ValueError("rdispls or recvcounts is required")
                 rd = np.zeros((L, P), dtype=np.int64)
                 rd[:, 1:] = np.cumsum(rc[:, :-1], axis=1)
             else:
-                rd = np.ascontiguousarray(np.asarray(rdispls, dtype=np.int64).reshape(L, P))
+                rd = host(rdispls, np.int64)
             keep += [sc, rc, sd, rd]
-            ptrs = (sc.ctypes.data, rc.ctypes.data if rc is not None else None, sd.ctypes.data, rd.ctypes.data)
+            at = lambda a: a.__array_interface__["data"][0]
+            ptrs = (at(sc), at(rc) if rc is not None else None, at(sd), at(rd))
         sp = (C.c_void_p * L)(*[(t.data_ptr() if t is not None else None) for t in send_l])
         rp = (C.c_void_p * L)(*[t.data_ptr() for t in recv_l])
         keep += [sp, rp]
@@ -344,11 +352,11 @@ class Communicator:
         # through a symmetric bounce buffer (two extra local copies; the eager protocol needs none).
         recv_l = [recv] if isinstance(recv, torch.Tensor) else list(recv)
         bounce = None
-        st = stream or torch.cuda.current_stream(self.device)
         if not eager_max_bytes and not inplace:
-            outside = [not self._lib.rbv_ctx_in_heap(self._ctx, C.c_void_p(t.data_ptr()), t.numel() * t.element_size())
-                       for t in recv_l]
+            lo, hi = self._heap_span
+            outside = [not lo <= t.data_ptr() <= hi - max(t.nbytes, 1) for t in recv_l]
             if any(outside):
+                st = stream or torch.cuda.current_stream(self.device)
                 bounce = []
                 for t, out in zip(recv_l, outside):
                     if out:
@@ -368,7 +376,8 @@ class Communicator:
         self._lib.rbv_ctx_set_bulk(self._ctx, int(self._bulk if bulk is None else bulk))
         rcode = self._lib.rbv_alltoallv(self._ctx, algo_id, n, r, r2, b, b2, ts, sp, rp, p_sc, p_rc, p_sd, p_rd,
                                         1 if on_dev else 0, int(bytes_hint), 1 if inplace else 0, int(grid),
-                                        int(chunk_bytes), C.c_void_p(st.cuda_stream))
+                                        int(chunk_bytes),
+                                        stream.cuda_stream if stream else _native.current_stream(self.device))
         if rcode:
             raise CommError(f"alltoallv({algo}) failed with code {rcode}: {self._lib.rbv_last_error().decode()}")
         if bounce is not None:

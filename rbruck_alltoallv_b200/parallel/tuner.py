@@ -45,9 +45,11 @@ def block_stats(counts, type_size: int = 1):
     """(mean block bytes, coefficient of variation) of a count matrix."""
     import numpy as np
     a = np.asarray(counts, dtype=np.float64).ravel() * type_size
-    if a.size == 0 or a.mean() <= 0:
+    mean = float(a.sum()) / a.size if a.size else 0.0
+    if mean <= 0:
         return 0.0, 0.0
-    return float(a.mean()), float(a.std() / a.mean())
+    a -= mean
+    return mean, math.sqrt(float(a.dot(a)) / a.size) / mean
 
 
 def _key(P: int, nproc: int, cls: int, skew: int = 0) -> str:
