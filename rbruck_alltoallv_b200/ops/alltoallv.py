@@ -80,7 +80,9 @@ def _auto_choice(c, recv, sendcounts, kw, agree_on_max: bool):
         mean_block = kw["bytes_hint"] / (c.L * c.P)
     else:
         mean_block = None
-    choice = _tuner.choose(c.P, c.nproc, mean_block, cv) if mean_block is not None else dict(SAFE_CHOICE)
+    # (resolved on the host: with counts on the device a persistent call is no different from a one-shot one)
+    persistent = agree_on_max and host_counts
+    choice = _tuner.choose(c.P, c.nproc, mean_block, cv, persistent) if mean_block is not None else dict(SAFE_CHOICE)
     forced = env_overrides()
     if "algo" in forced and forced["algo"] != choice.get("algo"):
         choice = {"algo": forced["algo"], "protocol": choice.get("protocol", "rendezvous")}   # drop the other algorithm's knobs

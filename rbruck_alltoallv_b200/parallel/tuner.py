@@ -108,16 +108,19 @@ def robust_us(samples_ms) -> float:
     return float(t[:keep].mean()) * 1e3
 
 
-def default_choice(P: int, nproc: int, mean_block_bytes: float) -> dict:
+def default_choice(P: int, nproc: int, mean_block_bytes: float, persistent: bool = False) -> dict:
     """Built-in rule for configurations the table has no measurement for.  On a flat NVSwitch fabric every extra
     Bruck digit costs one more cross-GPU synchronisation and forwards data twice, so the single-hop spread-out
     order wins whenever ranks are on different GPUs; Bruck variants remain selectable explicitly.  Blocks up to
     64 KB go through the eager protocol (faster in every measured configuration: 1, 2, 4 and 8 GPUs), larger ones
-    through rendezvous."""
+    through rendezvous.  A persistent call of one process has its addresses resolved and no peer to hand a block to:
+    the eager cells are one more copy there (5 ranks, blocks up to 4 KB: 8.2 against 4.7 us)."""
+    if persistent and nproc == 1:
+        return {"algo": "spreadout", "protocol": "rendezvous"}
     return {"algo": "spreadout", "protocol": "eager" if mean_block_bytes <= (64 << 10) else "rendezvous"}
 
 
-def choose(P: int, nproc: int, mean_block_bytes: float, cv: float = 0.0) -> dict:
+def choose(P: int, nproc: int, mean_block_bytes: float, cv: float = 0.0, persistent: bool = False) -> dict:
     """The table's entry for this size and skew class; neighbours (other skew class first, then the adjacent size
     classes) stand in for classes that were not measured; then the built-in rule."""
     tab = load_table()
@@ -127,7 +130,7 @@ def choose(P: int, nproc: int, mean_block_bytes: float, cv: float = 0.0) -> dict
             hit = tab.get(_key(P, nproc, c, s))
             if hit:
                 return dict(hit["choice"])
-    return default_choice(P, nproc, mean_block_bytes)
+    return default_choice(P, nproc, mean_block_bytes, persistent)
 
 
 def _pow2_upto(limit: int) -> List[int]:

@@ -71,6 +71,8 @@ def test_default_choice_for_unmeasured_configurations():
     small = tuner.default_choice(16, 16, 1024)
     large = tuner.default_choice(16, 16, 4 << 20)
     assert small == {"algo": "spreadout", "protocol": "eager"}
+    assert tuner.default_choice(5, 1, 1024) == {"algo": "spreadout", "protocol": "eager"}
+    assert tuner.default_choice(5, 1, 1024, persistent=True) == {"algo": "spreadout", "protocol": "rendezvous"}
     assert large == {"algo": "spreadout", "protocol": "rendezvous"}
 
 
