@@ -21,11 +21,18 @@ from ..parallel import tuner as _tuner
 _ENV_INT = {"RBV_RADIX": "r", "RBV_RADIX2": "r2", "RBV_BATCH": "b", "RBV_BATCH2": "b2", "RBV_GROUP": "n"}
 
 
+_ENV_KEYS = [k.encode() for k in (*_ENV_INT, "RBV_ALGO", "RBV_PROTOCOL")]
+
+
 def env_overrides() -> dict:
     """Choices forced from the environment: ``RBV_ALGO`` (any algorithm name), ``RBV_RADIX`` / ``RBV_RADIX2``,
     ``RBV_BATCH`` / ``RBV_BATCH2``, ``RBV_GROUP`` (ranks per group of the two-layer algorithms) and ``RBV_PROTOCOL``
     (``eager`` or ``rendezvous``).  They take precedence over the tuner table in ``algo="auto"`` calls.  The
     reference's drivers take the same knobs as positional arguments (examples/rbruckv_example.cpp:23-44)."""
+    # (os.environ looks a missing name up by way of an exception, seven of them per call: its own table is asked first)
+    table = getattr(os.environ, "_data", None)
+    if isinstance(table, dict) and not any(k in table for k in _ENV_KEYS):
+        return {}
     out = {}
     if os.environ.get("RBV_ALGO"):
         out["algo"] = os.environ["RBV_ALGO"]

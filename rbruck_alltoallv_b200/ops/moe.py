@@ -18,7 +18,7 @@ from .. import _native
 
 
 def _p(t: Optional[torch.Tensor]):
-    return C.c_void_p(t.data_ptr()) if t is not None else None
+    return t.data_ptr() if t is not None else None     # (a pointer argument takes the number as it is)
 
 
 def grouped_gemm(A: torch.Tensor, B: torch.Tensor, group_start: torch.Tensor, group_rows: torch.Tensor,
@@ -51,7 +51,7 @@ def grouped_gemm(A: torch.Tensor, B: torch.Tensor, group_start: torch.Tensor, gr
     try:
         rc = lib.rbv_grouped_gemm_bf16_gated(_p(A), M, _p(B), _p(out), _p(group_start), _p(group_rows), G, N, K,
                                              out.stride(0), 1 if swiglu else 0, _p(error), int(max_ctas),
-                                             C.c_void_p(st), _p(ready), _p(ready_target), float(timeout_ms))
+                                             st, _p(ready), _p(ready_target), float(timeout_ms))
     finally:
         if prev is not None:
             lib.rbv_grouped_gemm_set_pair(prev)
@@ -69,7 +69,7 @@ def quantize_rows_fp8(x: torch.Tensor, used: Optional[torch.Tensor] = None):
     q = torch.empty(rows, K, dtype=torch.uint8, device=x.device)
     sc = torch.empty(K // 128, rows, dtype=torch.float32, device=x.device)
     st = _native.current_stream(x.device.index)
-    rc = lib.rbv_quantize_used_rows_fp8(_p(x), rows, _p(used), K, x.stride(0), _p(q), _p(sc), C.c_void_p(st))
+    rc = lib.rbv_quantize_used_rows_fp8(_p(x), rows, _p(used), K, x.stride(0), _p(q), _p(sc), st)
     if rc:
         raise RuntimeError(f"quantisation launch failed (CUDA error {rc})")
     return q, sc
@@ -124,7 +124,7 @@ def grouped_gemm_fp8(Aq: torch.Tensor, a_scale_t: torch.Tensor, Bq: torch.Tensor
         rc = lib.rbv_grouped_gemm_fp8(_p(Aq), _p(a_scale_t), M, _p(Bq), _p(b_scale), _p(out), _p(group_start),
                                       _p(group_rows), G, N, K, out.stride(0),
                                       (1 if swiglu else 0) | (2 if coarse else 0), _p(error), int(max_ctas),
-                                      C.c_void_p(st))
+                                      st)
     finally:
         if prev is not None:
             lib.rbv_grouped_gemm_set_pair(prev)
@@ -144,7 +144,7 @@ def quantize_rows_mxfp8(x: torch.Tensor):
     q = torch.empty(rows, K, dtype=torch.uint8, device=x.device)
     sf = torch.empty(K // 128, (rows + 127) // 128 * 128, dtype=torch.int32, device=x.device)
     st = _native.current_stream(x.device.index)
-    rc = lib.rbv_quantize_rows_mxfp8(_p(x), rows, K, x.stride(0), _p(q), _p(sf), C.c_void_p(st))
+    rc = lib.rbv_quantize_rows_mxfp8(_p(x), rows, K, x.stride(0), _p(q), _p(sf), st)
     if rc:
         raise RuntimeError(f"MXFP8 quantisation launch failed (CUDA error {rc})")
     return q, sf
@@ -231,7 +231,7 @@ def grouped_gemm_mxfp8(Aq: torch.Tensor, sfa: torch.Tensor, Bq: torch.Tensor, sf
     st = _native.current_stream(Aq.device.index)
     rc = lib.rbv_grouped_gemm_mxfp8(_p(Aq), _p(sfa), M, _p(Bq), _p(sfb), _p(out), _p(group_start), _p(group_rows),
                                     G, N, K, out.stride(0), 1 if swiglu else 0, _p(error), int(max_ctas),
-                                    C.c_void_p(st))
+                                    st)
     if rc:
         raise RuntimeError(f"MXFP8 grouped GEMM launch failed (CUDA error {rc})")
     return out
@@ -260,7 +260,7 @@ def grouped_gemm_mxfp8_swiglu_q(Aq: torch.Tensor, sfa: torch.Tensor, Bq: torch.T
     st = _native.current_stream(Aq.device.index)
     rc = lib.rbv_grouped_gemm_mxfp8_swiglu_q(_p(Aq), _p(sfa), M, _p(Bq), _p(sfb), _p(out_q), _p(out_sf),
                                              _p(group_start), _p(group_rows), G, N, K, out_q.stride(0), _p(error),
-                                             int(max_ctas), C.c_void_p(st))
+                                             int(max_ctas), st)
     if rc:
         raise RuntimeError(f"MXFP8 grouped GEMM launch failed (CUDA error {rc})")
     return out_q, out_sf
@@ -381,7 +381,7 @@ class MoEExpertParallel:
         assert T == self.T and H == self.H and x.dtype == torch.bfloat16 and x.is_contiguous()
         assert logits.shape == (T, self.E) and logits.dtype == torch.float32 and logits.is_contiguous()
         lib, ctx = self.lib, self.comm._ctx
-        st = C.c_void_p(_native.current_stream(self.comm.device))
+        st = _native.current_stream(self.comm.device)
         if out is None:
             out = torch.empty_like(x)
         local = self.P == 1 and not self.overlap

@@ -22,6 +22,7 @@ from .._cuda_decl import SITE_NAMES, STATUS_NAMES, Status
 from .plan import ALGO_ID, Plan
 
 _default_comm: Optional["Communicator"] = None
+_INT32, _INT64 = np.dtype(np.int32), np.dtype(np.int64)
 
 
 class CommError(RuntimeError):
@@ -303,23 +304,23 @@ class Communicator:
             ptrs = (sc.data_ptr(), rc.data_ptr() if rc is not None else None, sd.data_ptr(), rd.data_ptr())
         else:
             def host(a, dt):
-                if type(a) is np.ndarray and a.dtype == dt and a.shape == (L, P) and a.flags.c_contiguous:
+                if type(a) is np.ndarray and a.dtype is dt and a.shape == (L, P) and a.flags.c_contiguous:
                     return a
                 return np.ascontiguousarray(np.asarray(a, dtype=dt).reshape(L, P))
-            sc = host(sendcounts, np.int32)
-            rc = None if recvcounts is None else host(recvcounts, np.int32)
+            sc = host(sendcounts, _INT32)
+            rc = None if recvcounts is None else host(recvcounts, _INT32)
             if sdispls is None:
                 sd = np.zeros((L, P), dtype=np.int64)
                 sd[:, 1:] = np.cumsum(sc[:, :-1], axis=1)
             else:
-                sd = host(sdispls, np.int64)
+                sd = host(sdispls, _INT64)
             if rdispls is None:
                 if rc is None:
                     raise ValueError("rdispls or recvcounts is required")
                 rd = np.zeros((L, P), dtype=np.int64)
                 rd[:, 1:] = np.cumsum(rc[:, :-1], axis=1)
             else:
-                rd = host(rdispls, np.int64)
+                rd = host(rdispls, _INT64)
             keep += [sc, rc, sd, rd]
             at = lambda a: a.__array_interface__["data"][0]
             ptrs = (at(sc), at(rc) if rc is not None else None, at(sd), at(rd))
