@@ -36,13 +36,16 @@ constexpr int QHM = 128;                // weight rows per CTA: one scale block
 constexpr int QT = 128;                 // most tokens per tile
 constexpr int QU = 32;                  // a tile's token count is a multiple of this
 constexpr int QK = 128;                 // one 128-byte swizzle row of fp8
-constexpr int QSTAGES = 8, QSLOTS = 4;
+constexpr int QSLOTS = 4;
 constexpr int QW_TILE = QHM * QK;       // 16 KB of weights
 constexpr int QT_TILE = QT / 2 * QK;    // up to 8 KB of tokens
-constexpr int QSTAGE = QW_TILE + QT_TILE;
+// Pipeline: 8 stages with room for the tokens of a full tile; where no group has more than 64 rows, 10 with room for 64
+constexpr int QSTAGES = 8, QSTAGE = QW_TILE + QT_TILE;
+constexpr int QSMALL = 64, QSTAGES_SMALL = 10, QSTAGE_SMALL = QW_TILE + QSMALL / 2 * QK;
 constexpr int QSCALERS = 8;             // scaling / epilogue warps
 constexpr int QTHREADS = 64 + 32 * QSCALERS;
-constexpr size_t QSMEM = (size_t)QSTAGES * QSTAGE + 1024;
+constexpr size_t QSMEM = (size_t)QSTAGES_SMALL * QSTAGE_SMALL + 1024;
+static_assert(QSTAGES * QSTAGE <= QSTAGES_SMALL * QSTAGE_SMALL, "shared memory");
 
 // Token boxes of 16, 32 and 64 rows: a CTA's half of a tile is fetched with the smallest that covers it.
 struct Fp8TokMaps { CUtensorMap w, tok[3]; };
@@ -226,13 +229,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QTHREADS, 1)
 grouped_gemm_fp8_tok_kernel(const __grid_constant__ Fp8TokMaps maps, const __grid_constant__ Fp8TokParams p) {
   extern __shared__ uint8_t dyn_smem[];
   uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dyn_smem) + 1023) & ~uintptr_t(1023));
-  __shared__ __align__(8) uint64_t full_bar[QSTAGES];    // used in the rank-0 CTA: bytes of both CTAs' loads
-  __shared__ __align__(8) uint64_t empty_bar[QSTAGES];   // in each CTA: its stage has been read by the MMAs
+  __shared__ __align__(8) uint64_t full_bar[QSTAGES_SMALL];    // used in the rank-0 CTA: bytes of both CTAs' loads
+  __shared__ __align__(8) uint64_t empty_bar[QSTAGES_SMALL];   // in each CTA: its stage has been read by the MMAs
   __shared__ __align__(8) uint64_t tfull_bar[QSLOTS];    // in each CTA: TMEM slot holds a finished K block (or tile)
   __shared__ __align__(8) uint64_t tempty_bar[QSLOTS];   // used in the rank-0 CTA: all 16 scaling warps took the slot
   __shared__ uint32_t tmem_base_s;
   __shared__ int s_rows[kMoeMaxGroups], s_start[kMoeMaxGroups];
-  __shared__ int s_abort;
+  __shared__ int s_abort, s_most;                        // s_most: rows of the largest group
   __shared__ __align__(16) float s_scale[QSCALERS][2][64];
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -241,21 +244,28 @@ grouped_gemm_fp8_tok_kernel(const __grid_constant__ Fp8TokMaps maps, const __gri
   const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
 
   if (tid == 0) {
-    for (int s = 0; s < QSTAGES; s++) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+    for (int s = 0; s < QSTAGES_SMALL; s++) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
     for (int b = 0; b < QSLOTS; b++) { mbar_init(&tfull_bar[b], 1); mbar_init(&tempty_bar[b], 2 * QSCALERS); }
     s_abort = 0;
+    s_most = 0;
     mbar_fence_init();
   }
   if (warp == 1) { tmem_alloc_pair(&tmem_base_s, 512); tmem_relinquish_pair(); }
+  __syncthreads();
   pdl_trigger();
   pdl_wait();
-  for (int i = tid; i < p.G; i += blockDim.x) { s_rows[i] = p.group_rows[i]; s_start[i] = p.group_start[i]; }
+  for (int i = tid; i < p.G; i += blockDim.x) {
+    s_rows[i] = p.group_rows[i]; s_start[i] = p.group_start[i];
+    atomicMax(&s_most, s_rows[i]);
+  }
   tc_fence_before_sync();
   __syncthreads();
   cluster_sync_all();
   tc_fence_after_sync();
   const uint32_t tmem_base = tmem_base_s;
   const int num_kb = p.K / QK;
+  const int stages = s_most <= QSMALL ? QSTAGES_SMALL : QSTAGES;
+  const int stage_bytes = s_most <= QSMALL ? QSTAGE_SMALL : QSTAGE;
   volatile int* abort_flag = &s_abort;
   const uint32_t peer_abort = mapa_u32(smem_u32(&s_abort), rank ^ 1u);
 
@@ -277,12 +287,12 @@ grouped_gemm_fp8_tok_kernel(const __grid_constant__ Fp8TokMaps maps, const __gri
         const int t_row = tl.tok0 + (int)rank * half;
         for (int kb = 0; kb < num_kb; kb++) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag)) { ok = false; break; }
-          uint8_t* sw = tiles + (size_t)stage * QSTAGE;
+          uint8_t* sw = tiles + (size_t)stage * stage_bytes;
           if (leader) mbar_arrive_expect_tx(&full_bar[stage], bytes);
           const uint32_t bar0 = mapa_u32(smem_u32(&full_bar[stage]), 0);
           tma_load_2d_pair(sw, &maps.w, kb * QK, w_row, bar0);
           tma_load_2d_pair(sw + QW_TILE, tok, kb * QK, t_row, bar0);
-          if (++stage == QSTAGES) { stage = 0; phase ^= 1u; }
+          if (++stage == stages) { stage = 0; phase ^= 1u; }
         }
       }
       if (!ok) { s_abort = 1; st_cluster_u32(peer_abort, 1); atomicExch(p.error, 1); }
@@ -306,7 +316,7 @@ grouped_gemm_fp8_tok_kernel(const __grid_constant__ Fp8TokMaps maps, const __gri
             if (!mbar_wait(&tempty_bar[slot], ((it / QSLOTS) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
           if (!mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
           tc_fence_after_sync();
-          const uint8_t* sa = tiles + (size_t)stage * QSTAGE;
+          const uint8_t* sa = tiles + (size_t)stage * stage_bytes;
           const uint64_t adesc = umma_desc_sw128(sa);
           const uint64_t bdesc = umma_desc_sw128(sa + QW_TILE);
           const uint32_t d_tmem = tmem_base + (uint32_t)slot * QT;
@@ -316,7 +326,7 @@ grouped_gemm_fp8_tok_kernel(const __grid_constant__ Fp8TokMaps maps, const __gri
                          (uint32_t)(coarse ? (kb | kk) != 0 : kk != 0));
           umma_commit_pair(&empty_bar[stage]);
           if (!coarse || kb == num_kb - 1) { umma_commit_pair(&tfull_bar[slot]); it++; }
-          if (++stage == QSTAGES) { stage = 0; phase ^= 1u; }
+          if (++stage == stages) { stage = 0; phase ^= 1u; }
         }
       }
       if (!ok) { s_abort = 1; st_cluster_u32(peer_abort, 1); atomicExch(p.error, 2); }

@@ -42,13 +42,17 @@ constexpr int HM = 128;            // weight rows per CTA
 constexpr int PT = 256;            // most tokens per tile
 constexpr int PU = 32;             // tokens per unit: a tile's token count is a multiple of this
 constexpr int PK = 64;             // one 128-byte swizzle atom of bf16
-constexpr int PSTAGES = 6;
 constexpr int PW_BYTES = HM * PK * 2;        // 16 KB of weights
 constexpr int PT_BYTES = PT / 2 * PK * 2;    // up to 16 KB of tokens
-constexpr int PSTAGE_BYTES = PW_BYTES + PT_BYTES;
+// Pipeline: 6 stages with room for the tokens of a full tile; where no group has more than 64 rows, 10 stages with room for
+// 64.  The kernel then is a stream of weights, and what counts is how many of their bytes are on the way (160 instead of
+// 96 KB per SM: up / down GEMM of 64 tokens 316 / 171 -> 299 / 162 us, the layer 472 -> 440 us).
+constexpr int PSTAGES = 6, PSTAGE_BYTES = PW_BYTES + PT_BYTES;
+constexpr int PSMALL = 64, PSTAGES_SMALL = 10, PSTAGE_BYTES_SMALL = PW_BYTES + PSMALL / 2 * PK * 2;
 constexpr int PAIR_THREADS = 192;
 constexpr int PAIR_TMEM_COLS = 512;
-constexpr size_t PAIR_SMEM = (size_t)PSTAGES * PSTAGE_BYTES + 1024 /*alignment slack*/;
+constexpr size_t PAIR_SMEM = (size_t)PSTAGES_SMALL * PSTAGE_BYTES_SMALL + 1024 /*alignment slack*/;
+static_assert(PSTAGES * PSTAGE_BYTES <= PSTAGES_SMALL * PSTAGE_BYTES_SMALL, "shared memory");
 
 // Token boxes of 16, 32, 64 and 128 rows: a CTA's half of a tile is fetched with the smallest that covers it.
 struct PairMaps { CUtensorMap w, tok[4]; };
@@ -105,13 +109,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
 grouped_gemm_pair_kernel(const __grid_constant__ PairMaps maps, const __grid_constant__ PairParams p) {
   extern __shared__ uint8_t dyn_smem[];
   uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dyn_smem) + 1023) & ~uintptr_t(1023));
-  __shared__ __align__(8) uint64_t full_bar[PSTAGES];    // used in the rank-0 CTA: bytes of both CTAs' loads
-  __shared__ __align__(8) uint64_t empty_bar[PSTAGES];   // in each CTA: its stage has been read by the MMAs
+  __shared__ __align__(8) uint64_t full_bar[PSTAGES_SMALL];    // used in the rank-0 CTA: bytes of both CTAs' loads
+  __shared__ __align__(8) uint64_t empty_bar[PSTAGES_SMALL];   // in each CTA: its stage has been read by the MMAs
   __shared__ __align__(8) uint64_t tfull_bar[2];         // in each CTA: accumulator b is complete
   __shared__ __align__(8) uint64_t tempty_bar[2];        // used in the rank-0 CTA: both CTAs have drained accumulator b
   __shared__ uint32_t tmem_base_s;
   __shared__ int s_rows[kMoeMaxGroups], s_start[kMoeMaxGroups];
-  __shared__ int s_abort;
+  __shared__ int s_abort, s_most;                        // s_most: rows of the largest group
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t rank = cluster_ctarank();
@@ -119,21 +123,28 @@ grouped_gemm_pair_kernel(const __grid_constant__ PairMaps maps, const __grid_con
   const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
 
   if (tid == 0) {
-    for (int s = 0; s < PSTAGES; s++) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+    for (int s = 0; s < PSTAGES_SMALL; s++) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
     for (int b = 0; b < 2; b++) { mbar_init(&tfull_bar[b], 1); mbar_init(&tempty_bar[b], 8); }
     s_abort = 0;
+    s_most = 0;
     mbar_fence_init();
   }
   if (warp == 1) { tmem_alloc_pair(&tmem_base_s, PAIR_TMEM_COLS); tmem_relinquish_pair(); }
+  __syncthreads();
   pdl_trigger();
   pdl_wait();
-  for (int i = tid; i < p.G; i += blockDim.x) { s_rows[i] = p.group_rows[i]; s_start[i] = p.group_start[i]; }
+  for (int i = tid; i < p.G; i += blockDim.x) {
+    s_rows[i] = p.group_rows[i]; s_start[i] = p.group_start[i];
+    atomicMax(&s_most, s_rows[i]);
+  }
   tc_fence_before_sync();
   __syncthreads();
   cluster_sync_all();   // barriers of both CTAs are initialised before anything is signalled across
   tc_fence_after_sync();
   const uint32_t tmem_base = tmem_base_s;
   const int num_kb = p.K / PK;
+  const int stages = s_most <= PSMALL ? PSTAGES_SMALL : PSTAGES;
+  const int stage_bytes = s_most <= PSMALL ? PSTAGE_BYTES_SMALL : PSTAGE_BYTES;
   volatile int* abort_flag = &s_abort;
   const uint32_t peer_abort = mapa_u32(smem_u32(&s_abort), rank ^ 1u);
 
@@ -154,12 +165,12 @@ grouped_gemm_pair_kernel(const __grid_constant__ PairMaps maps, const __grid_con
         const int t_row = tl.tok0 + (int)rank * half;
         for (int kb = 0; kb < num_kb; kb++) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag)) { ok = false; break; }
-          uint8_t* sw = tiles + (size_t)stage * PSTAGE_BYTES;
+          uint8_t* sw = tiles + (size_t)stage * stage_bytes;
           if (leader) mbar_arrive_expect_tx(&full_bar[stage], bytes);
           const uint32_t bar0 = mapa_u32(smem_u32(&full_bar[stage]), 0);
           tma_load_2d_pair(sw, &maps.w, kb * PK, w_row, bar0);
           tma_load_2d_pair(sw + PW_BYTES, tok, kb * PK, t_row, bar0);
-          if (++stage == PSTAGES) { stage = 0; phase ^= 1u; }
+          if (++stage == stages) { stage = 0; phase ^= 1u; }
         }
       }
       if (!ok) { s_abort = 1; st_cluster_u32(peer_abort, 1); atomicExch(p.error, 1); }
@@ -182,14 +193,14 @@ grouped_gemm_pair_kernel(const __grid_constant__ PairMaps maps, const __grid_con
         for (int kb = 0; kb < num_kb; kb++) {
           if (!mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
           tc_fence_after_sync();
-          const uint8_t* sw = tiles + (size_t)stage * PSTAGE_BYTES;
+          const uint8_t* sw = tiles + (size_t)stage * stage_bytes;
           const uint64_t wdesc = umma_desc_sw128(sw);
           const uint64_t tdesc = umma_desc_sw128(sw + PW_BYTES);
           #pragma unroll
           for (int kk = 0; kk < PK / 16; kk++)
             umma_bf16_pair(d_tmem, wdesc + 2u * kk, tdesc + 2u * kk, idesc, (uint32_t)((kb | kk) != 0));
           umma_commit_pair(&empty_bar[stage]);   // frees this stage in both CTAs
-          if (++stage == PSTAGES) { stage = 0; phase ^= 1u; }
+          if (++stage == stages) { stage = 0; phase ^= 1u; }
         }
         if (ok) umma_commit_pair(&tfull_bar[b]);   // accumulator complete, both CTAs
       }
