@@ -30,6 +30,8 @@
 // 218 / 122 -> 178 / 105, 1000 tokens 268 / 154 -> 245 / 154, 2000 tokens 456 / 224 -> 423 / 195, 8192 tokens 2098 / 1052
 // -> 1534 / 712.  On the way: 128 tokens by 256 weight rows 531 / 270 at 2000 tokens, 192 by 256 455 / 238, two MMAs of
 // 128 tokens each instead of one of 256 443 / 205.
+// Short K makes the epilogue the bound (1024 / 2816, 4 experts of 616 rows: 88 us with four epilogue warps and tiles of 256
+// only, 70 with eight and the tile size below, 77 before).
 // Epilogues: bf16; SwiGLU to bf16; SwiGLU followed by the MXFP8 quantiser of the next GEMM's operand (32 tokens at a time
 // change hands through shared memory, so that eight lanes hold the 32 values that share a scale); and, for the down GEMM
 // of the MoE layer, bf16 rows stored straight into the buffers of the GPUs the tokens came from (the return all-to-all,
@@ -61,18 +63,23 @@ constexpr int XSUB = 128;               // tokens (columns) per accumulator slot
 constexpr int XU = 32;                  // a tile's token count is a multiple of this
 constexpr int XS = 64;                  // a tile starts at a multiple of this many tokens of its group
 constexpr int XK = 128;                 // bytes of K per pipeline stage (one 128-byte swizzle row, four scale blocks)
-constexpr int XSTAGES = 6;
 constexpr int XW_TILE = XHM * XK;       // 16 KB of weights
 constexpr int XT_TILE = XT / 2 * XK;    // up to 16 KB of tokens
 constexpr int XSF_TILE = 512;           // an atom: 128 scale words
-constexpr int XSTAGE = XW_TILE + XT_TILE + 4 * XSF_TILE;   // 34 KB
-constexpr int XTHREADS = 192;           // TMA warp, MMA warp, 4 epilogue warps
+// Pipeline: 6 stages with room for the tokens (and their three atoms) of a full tile; where no group has more than 64 rows,
+// 9 stages with room for 64 tokens and their one atom: the kernel then is a stream of weights, and what counts is how many
+// of their bytes are on the way.
+constexpr int XSTAGES = 6, XSTAGE = XW_TILE + XT_TILE + 4 * XSF_TILE;                              // 34 KB
+constexpr int XSMALL = 64, XSTAGES_SMALL = 9, XSTAGE_SMALL = XW_TILE + XSMALL / 2 * XK + 4 * XSF_TILE;   // 22 KB
+static_assert(XSTAGES * XSTAGE >= XSTAGES_SMALL * XSTAGE_SMALL, "shared memory");
+constexpr int XEPI = 8;                 // epilogue warps: two groups of four (one per TMEM lane quarter), every other 32 tokens each
+constexpr int XTHREADS = 64 + 32 * XEPI;   // and the TMA and the MMA warp
 constexpr int XACCS = 3;                // accumulator slots
 constexpr int XACC_COLS = XACCS * XSUB;
-constexpr int XSF_COLS = 16;            // TMEM columns of scales per stage: 4 for the weights, 12 for the tokens
-static_assert(XACC_COLS + XSTAGES * XSF_COLS <= 512, "TMEM");
-// quantising epilogue: two buffers of 32 tokens x 64 outputs; rows 80 floats apart, so that the even lanes' token and the
-// odd lanes' token fall into different halves of the banks
+constexpr int XSF_COLS = 16, XSF_COLS_SMALL = 8;   // TMEM columns of scales per stage: 4 for the weights, 12 (4) for the tokens
+static_assert(XACC_COLS + XSTAGES * XSF_COLS <= 512 && XACC_COLS + XSTAGES_SMALL * XSF_COLS_SMALL <= 512, "TMEM");
+// quantising epilogue: a buffer of 32 tokens x 64 outputs per group; rows 80 floats apart, so that the even lanes' token and
+// the odd lanes' token fall into different halves of the banks
 constexpr int XQ_LD = 80;
 constexpr int XQ_BUF = XU * XQ_LD * 4;  // 10 KB
 constexpr size_t XSMEM = (size_t)XSTAGES * XSTAGE + 2 * XQ_BUF + 1024;
@@ -101,12 +108,14 @@ struct XTile { int g, tok0, ntok, nt, n0; bool valid; };   // group, first token
 
 // Walks the tile schedule (groups in order, weight rows slow, tokens fast); `at(t)` wants non-decreasing t.
 struct MxWalk {
+  const int cap;           // most tokens of a tile, in units of XS
   int g = 0, before = 0;   // tiles of the groups in front of g
+  __device__ explicit MxWalk(int c) : cap(c) {}
   __device__ __forceinline__ XTile at(const MxParams& p, int t, const int* s_rows, const int* s_start) {
     XTile r; r.valid = false; r.g = r.tok0 = r.ntok = r.nt = r.n0 = 0;
     const int ntn = (p.N + XM - 1) / XM;     // N is a multiple of 128: the last tile may be half empty
     for (; g < p.G; g++) {
-      const int units = (s_rows[g] + XS - 1) / XS, ntm = (units + XT / XS - 1) / (XT / XS);
+      const int units = (s_rows[g] + XS - 1) / XS, ntm = (units + cap - 1) / cap;
       const int cnt = ntm * ntn;
       if (t - before < cnt) {
         const int n = (t - before) / ntm, m = (t - before) - n * ntm;
@@ -165,16 +174,16 @@ __device__ __forceinline__ void tmem_cp_scales_pair(uint32_t taddr, uint64_t sde
   asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(sdesc) : "memory");
 }
 
-// The four epilogue warps: barrier, and barrier with a vote.
-__device__ __forceinline__ void epi_barrier() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
-__device__ __forceinline__ bool epi_all(bool pred) {
+// The four epilogue warps of a group: barrier, and barrier with a vote.
+__device__ __forceinline__ void epi_barrier(int group) { asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory"); }
+__device__ __forceinline__ bool epi_all(int group, bool pred) {
   uint32_t all;
   asm volatile(
       "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.b32 p, %1, 0;\n\t"
-      "bar.red.and.pred q, 1, 128, p;\n\t"
+      "bar.red.and.pred q, %2, 128, p;\n\t"
       "selp.b32 %0, 1, 0, q;\n\t}"
-      : "=r"(all) : "r"((uint32_t)pred) : "memory");
+      : "=r"(all) : "r"((uint32_t)pred), "r"(1 + group) : "memory");
   return all != 0;
 }
 
@@ -194,13 +203,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(XTHREADS, 1)
 grouped_gemm_mxfp8_kernel(const __grid_constant__ MxMaps maps, const __grid_constant__ MxParams p) {
   extern __shared__ uint8_t dyn_smem[];
   uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dyn_smem) + 1023) & ~uintptr_t(1023));
-  __shared__ __align__(8) uint64_t full_bar[XSTAGES];    // rank-0 CTA: operand and scale bytes of both CTAs
-  __shared__ __align__(8) uint64_t empty_bar[XSTAGES];   // each CTA: its stage has been read by the MMAs
+  __shared__ __align__(8) uint64_t full_bar[XSTAGES_SMALL];    // rank-0 CTA: operand and scale bytes of both CTAs
+  __shared__ __align__(8) uint64_t empty_bar[XSTAGES_SMALL];   // each CTA: its stage has been read by the MMAs
   __shared__ __align__(8) uint64_t tfull_bar[XACCS];     // each CTA: the accumulator is complete
   __shared__ __align__(8) uint64_t tempty_bar[XACCS];    // rank-0 CTA: both CTAs have taken the accumulator
   __shared__ uint32_t tmem_base_s;
   __shared__ int s_rows[kMoeMaxGroups], s_start[kMoeMaxGroups];
-  __shared__ int s_abort, s_bad;
+  __shared__ int s_abort, s_bad, s_cap, s_most;          // s_most: rows of the largest group
+  __shared__ int s_tiles[3];                             // tiles of the schedule with at most 128, 192, 256 tokens each
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t rank = cluster_ctarank();
@@ -210,8 +220,10 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ MxMaps maps, const __grid_cons
 
   if (tid == 0) {
     s_bad = 0;
-    for (int s = 0; s < XSTAGES; s++) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-    for (int b = 0; b < XACCS; b++) { mbar_init(&tfull_bar[b], 1); mbar_init(&tempty_bar[b], 8); }
+    s_most = 0;
+    s_tiles[0] = s_tiles[1] = s_tiles[2] = 0;
+    for (int s = 0; s < XSTAGES_SMALL; s++) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+    for (int b = 0; b < XACCS; b++) { mbar_init(&tfull_bar[b], 1); mbar_init(&tempty_bar[b], 2 * XEPI); }
     s_abort = 0;
     mbar_fence_init();
   }
@@ -222,13 +234,32 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ MxMaps maps, const __grid_cons
   for (int i = tid; i < p.G; i += blockDim.x) {
     s_rows[i] = p.group_rows[i]; s_start[i] = p.group_start[i];
     if (s_rows[i] > 0 && (s_start[i] & 127)) s_bad = 1;   // the scale atoms of A would not coincide with the tiles
+    atomicMax(&s_most, s_rows[i]);
+    const int units = (s_rows[i] + XS - 1) / XS;
+    #pragma unroll
+    for (int c = 0; c < 3; c++) atomicAdd(&s_tiles[c], (units + c + 1) / (c + 2) * ((p.N + XM - 1) / XM));
   }
   tc_fence_before_sync();
+  __syncthreads();
+  if (tid == 0) {
+    // Rounds of tiles over the SM pairs, times what a K block of such a tile takes: 311 ns with 128 tokens, 380 with 190,
+    // 465 with 240, which is about 96 tokens plus its own.  (A few large tiles may leave most pairs idle in the last
+    // round, and the same groups in smaller ones fill it.)
+    int best = 0x7fffffff;
+    for (int c = 2; c >= 0; c--) {
+      const int cost = (s_tiles[c] + npairs - 1) / npairs * ((c + 2) * XS + 96);
+      if (cost < best) { best = cost; s_cap = c + 2; }
+    }
+  }
   __syncthreads();
   cluster_sync_all();
   tc_fence_after_sync();
   const uint32_t tmem_base = tmem_base_s;
   const int num_kb = s_bad ? 0 : p.K / XK;
+  const bool small = s_most <= XSMALL;
+  const int stages = small ? XSTAGES_SMALL : XSTAGES;
+  const int stage_bytes = small ? XSTAGE_SMALL : XSTAGE, sf_at = stage_bytes - 4 * XSF_TILE;   // scale atoms inside a stage
+  const uint32_t sf_cols = small ? XSF_COLS_SMALL : XSF_COLS;
   if (s_bad) {   // both CTAs see the same arrays: nobody does anything, the error is recorded once
     if (blockIdx.x == 0 && tid == 0) atomicExch(p.error, 5);
     npairs = 1 << 30;
@@ -246,7 +277,7 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ MxMaps maps, const __grid_cons
       int stage = 0; uint32_t phase = 0;
       bool ok = true;
       const int nb128 = p.N / 128;
-      MxWalk walk;
+      MxWalk walk(s_cap);
       for (int t = first_tile; ok; t += npairs) {
         const XTile tl = walk.at(p, t, s_rows, s_start);
         if (!tl.valid) break;
@@ -257,17 +288,17 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ MxMaps maps, const __grid_cons
         const int n_row = tl.n0 + (int)rank * XHM;
         for (int kb = 0; kb < num_kb; kb++) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag)) { ok = false; break; }
-          uint8_t* sw = tiles + (size_t)stage * XSTAGE;
+          uint8_t* sw = tiles + (size_t)stage * stage_bytes;
           if (leader) mbar_arrive_expect_tx(&full_bar[stage], bytes);
           const uint32_t bar0 = mapa_u32(smem_u32(&full_bar[stage]), 0);
           // (rows of a half-empty last tile belong to the next expert or lie outside: computed, never stored)
           tma_load_2d_pair(sw, &maps.w, kb * XK, tl.g * p.N + n_row, bar0);
           tma_load_2d_pair(sw + XW_TILE, tok, kb * XK, tl.tok0 + (int)rank * half, bar0);
-          tma_load_2d_pair(sw + XW_TILE + XT_TILE, &maps.sfw, 0, (tl.g * num_kb + kb) * nb128 + n_row / 128, bar0);
+          tma_load_2d_pair(sw + sf_at, &maps.sfw, 0, (tl.g * num_kb + kb) * nb128 + n_row / 128, bar0);
           for (int j = 0; j < atoms; j++)
-            tma_load_2d_pair(sw + XW_TILE + XT_TILE + (1 + j) * XSF_TILE, &maps.sft, 0,
+            tma_load_2d_pair(sw + sf_at + (1 + j) * XSF_TILE, &maps.sft, 0,
                              kb * p.a_row_blocks + tl.tok0 / 128 + j, bar0);
-          if (++stage == XSTAGES) { stage = 0; phase ^= 1u; }
+          if (++stage == stages) { stage = 0; phase ^= 1u; }
         }
       }
       if (!ok) { s_abort = 1; st_cluster_u32(peer_abort, 1); atomicExch(p.error, 1); }
@@ -278,7 +309,7 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ MxMaps maps, const __grid_cons
       int stage = 0; uint32_t phase = 0;
       bool ok = true;
       MxSlots slots;
-      MxWalk walk;
+      MxWalk walk(s_cap);
       for (int t = first_tile; ok; t += npairs) {
         const XTile tl = walk.at(p, t, s_rows, s_start);
         if (!tl.valid) break;
@@ -294,8 +325,8 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ MxMaps maps, const __grid_cons
         const int atoms = mx_tok_atoms(tl);
         const uint32_t sf_shift = (uint32_t)(tl.tok0 & 127) / 32;   // TMEM column of the tile's first token: 0 or 2
         auto copy_scales = [&](int st) {
-          const uint8_t* sf = tiles + (size_t)st * XSTAGE + XW_TILE + XT_TILE;
-          const uint32_t to = tmem_base + XACC_COLS + (uint32_t)st * XSF_COLS;
+          const uint8_t* sf = tiles + (size_t)st * stage_bytes + sf_at;
+          const uint32_t to = tmem_base + XACC_COLS + (uint32_t)st * sf_cols;
           tmem_cp_scales_pair(to, desc_rows16(sf));
           for (int j = 0; j < atoms; j++) tmem_cp_scales_pair(to + 4u + 4u * (uint32_t)j, desc_rows16(sf + (1 + j) * XSF_TILE));
         };
@@ -308,16 +339,16 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ MxMaps maps, const __grid_cons
             tc_fence_after_sync();
             copy_scales(stage);
           }
-          const int next = stage + 1 == XSTAGES ? 0 : stage + 1;
+          const int next = stage + 1 == stages ? 0 : stage + 1;
           const uint32_t next_phase = next ? phase : phase ^ 1u;
           copied = kb + 1 < num_kb && mbar_try_wait(&full_bar[next], next_phase);
           if (copied) {
             tc_fence_after_sync();
             copy_scales(next);
           }
-          const uint8_t* sw = tiles + (size_t)stage * XSTAGE;
+          const uint8_t* sw = tiles + (size_t)stage * stage_bytes;
           const uint64_t wdesc = umma_desc_sw128(sw);
-          const uint32_t tsfw = tmem_base + XACC_COLS + (uint32_t)stage * XSF_COLS;
+          const uint32_t tsfw = tmem_base + XACC_COLS + (uint32_t)stage * sf_cols;
           const uint64_t tdesc = umma_desc_sw128(sw + XW_TILE);
           #pragma unroll
           for (int kk = 0; kk < XK / 32; kk++)
@@ -331,16 +362,16 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ MxMaps maps, const __grid_cons
       if (!ok) { s_abort = 1; st_cluster_u32(peer_abort, 1); atomicExch(p.error, 2); }
     }
   } else {
-    // ---------------- epilogue (both CTAs): warps 2..5, TMEM lane quarter = warp % 4 ----------------
+    // ---------------- epilogue (both CTAs): warps 2..9, TMEM lane quarter = warp % 4, group = (warp - 2) / 4 ----------------
     const int q = warp & 3;
     const bool odd = (lane & 1) != 0;
-    float* const qbuf = reinterpret_cast<float*>(tiles + (size_t)XSTAGES * XSTAGE);
+    const int group = (warp - 2) >> 2;
+    float* const buf = reinterpret_cast<float*>(tiles + (size_t)XSTAGES * XSTAGE) + group * (XU * XQ_LD);
     __nv_bfloat16* C = static_cast<__nv_bfloat16*>(p.C);
     const uint32_t tempty0 = mapa_u32(smem_u32(&tempty_bar[0]), 0);
     bool ok = true;
-    unsigned chunk = 0;   // 32-token chunks so far: which of the two shared buffers
     MxSlots slots;
-    MxWalk walk;
+    MxWalk walk(s_cap);
     for (int t = first_tile; ok; t += npairs) {
       const XTile tl = walk.at(p, t, s_rows, s_start);
       if (!tl.valid) break;
@@ -355,12 +386,10 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ MxMaps maps, const __grid_cons
         if (p.epilogue == 3) {
           // SwiGLU, then the quantiser of the next GEMM's operand: 32 tokens x 64 outputs of this CTA go through shared
           // memory, after which 16 lanes hold a token's 64 outputs, four each, and 8 lanes the 32 that share a scale.
-          // The 64 (token, 4-wide) pieces of a warp are read before the other buffer is used again one barrier later.
-          float* buf = qbuf + (chunk++ & 1u) * (XU * XQ_LD);
           #pragma unroll
           for (int k = 0; k < 32; k += 2)
             buf[(k + (odd ? 1 : 0)) * XQ_LD + q * 16 + (lane >> 1)] = tokepi::swiglu_pair(r, k, odd);
-          epi_barrier();
+          epi_barrier(group);
           #pragma unroll
           for (int u = 0; u < 4; u++) {
             const int tok = u * 8 + q * 2 + (lane >> 4), l16 = lane & 15;
@@ -383,6 +412,7 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ MxMaps maps, const __grid_cons
               }
             }
           }
+          epi_barrier(group);   // read by all before the next tokens are written
         } else {
           __nv_bfloat16* rows = C + (size_t)(tl.tok0 + c) * p.ldc;
           if (p.epilogue == 1) {
@@ -402,24 +432,25 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ MxMaps maps, const __grid_cons
         // of two slots the one that the next tile wants, slot 1, goes first
         const int b = slots.count == 2 ? (i == 0 ? 1 : slots.first == 0 ? 0 : 2) : slots.first;
         const int s = b - slots.first;       // tokens s * 128 ...
-        // (the four epilogue warps meet at a named barrier when they quantise: they leave the loop together, see the vote)
+        // (the four warps of a group meet at a named barrier when they quantise: they leave the loop together, see the vote)
         const bool got_it = mbar_wait(&tfull_bar[b], slots.phase(b), abort_flag);
         slots.used(b);
-        if (p.epilogue == 3 ? !epi_all(got_it) : !got_it) { ok = false; break; }
+        if (p.epilogue == 3 ? !epi_all(group, got_it) : !got_it) { ok = false; break; }
         tc_fence_after_sync();
-        const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)b * XSUB;
+        // this group's tokens of the slot: 32 group ... and 64 + 32 group ...
+        const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * XSUB);
         const int n = min(tl.nt - s * XSUB, XSUB);
-        uint32_t r[XSUB / 32][32];
+        uint32_t r[XSUB / 64][32];
         #pragma unroll
-        for (int k = 0; k < XSUB / 32; k++)
-          if (k * 32 < n) tmem_ld32(taddr + k * 32, r[k]);
+        for (int k = 0; k < XSUB / 64; k++)
+          if (k * 64 + group * 32 < n) tmem_ld32(taddr + k * 64 + group * 32, r[k]);
         tmem_ld_wait();
         tc_fence_before_sync();
         __syncwarp();
-        if (lane == 0) mbar_arrive_cluster(tempty0 + 8u * (uint32_t)b);   // 4 warps x 2 CTAs
+        if (lane == 0) mbar_arrive_cluster(tempty0 + 8u * (uint32_t)b);   // 8 warps x 2 CTAs
         #pragma unroll
-        for (int k = 0; k < XSUB / 32; k++)
-          if (k * 32 < n) store_chunk(r[k], s * XSUB + k * 32);
+        for (int k = 0; k < XSUB / 64; k++)
+          if (k * 64 + group * 32 < n) store_chunk(r[k], s * XSUB + k * 64 + group * 32);
       }
     }
     if (!ok && lane == 0) { s_abort = 1; st_cluster_u32(peer_abort, 1); atomicExch(p.error, 3); }
