@@ -130,7 +130,8 @@ void rbv_ctx_set_eager(rbv_ctx_t ctx, unsigned long long max_block_bytes);
 void rbv_ctx_set_trace(rbv_ctx_t ctx, int on);       /* report phase time stamps after every call */
 void rbv_ctx_set_bulk(rbv_ctx_t ctx, int mode);      /* bulk-copy engine for large chunks: 0 off (default), 1 on, -1 by size */
 void rbv_ctx_set_cooperative(rbv_ctx_t ctx, int mode); /* -1 where a call needs it (default), 0 never, 1 always */
-void rbv_ctx_set_static(rbv_ctx_t ctx, int on);      /* 0: persistent calls keep the dynamic kernel */
+void rbv_ctx_set_static(rbv_ctx_t ctx, int on);      /* 0: persistent calls, and direct calls of one process, keep the
+                                                        dynamic kernel */
 /* For the next rbv_prepare* only: mirrors[L] (null entries: none) name where each local rank wants its received
  * blocks in the end, e.g. pinned host memory.  A call that runs the static kernel copies them there from the receive
  * buffers itself once everything has arrived, so the end of the launch is the end of the whole transfer; other calls
