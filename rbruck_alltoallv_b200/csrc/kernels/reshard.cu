@@ -4,7 +4,7 @@
 //
 // Bound by HBM: two bytes of traffic per byte moved.  The exchange through a packed buffer moves every byte twice (a
 // strided copy per rank, then the alltoallv), and for a few MB the launches of the per-rank copies dominate.  Measured on
-// one B200, bf16, 32 heads of 128: 8 ranks x 512 positions to heads 92 -> 23 us (host-bound: views and pointer arrays);
+// one B200, bf16, 32 heads of 128: 8 ranks x 512 positions to heads 92 -> 19 us (host-bound: views and pointer arrays);
 // 4 ranks x 4096 positions back 270 -> 43 us (6.2 TB/s).
 #include <cuda_runtime.h>
 
