@@ -326,6 +326,7 @@ class MoEExpertParallel:
         self.error = torch.zeros(4, dtype=i32, device=dev)
         self.place = torch.empty(tokens, 2, dtype=i32, device=dev)             # one rank: see _route_and_dispatch_local
         self.route_scratch = torch.zeros(self.E + 1, dtype=i32, device=dev)
+        self.xq8 = self.xs8 = None       # one rank, block-scaled fp8: the rows and scales that the dispatch delivers
         if self.P == 1 and self.fp8 and not self.mx and hidden % 128 == 0:
             self.xq8 = torch.empty(self.cap, hidden, dtype=torch.uint8, device=dev)
             self.xs8 = torch.empty(hidden // 128, self.cap, dtype=torch.float32, device=dev)

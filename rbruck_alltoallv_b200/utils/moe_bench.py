@@ -18,7 +18,8 @@ import numpy as np
 import torch
 import torch.distributed as dist
 
-from ..ops.moe import MoEExpertParallel, grouped_gemm, reference_forward
+from ..ops.moe import (MoEExpertParallel, grouped_gemm, grouped_gemm_fp8, grouped_gemm_mxfp8, quantize_rows_fp8,
+                       quantize_rows_mxfp8, reference_forward)
 from ..parallel.comm import Communicator
 
 
@@ -47,6 +48,17 @@ def _time(fn, steps, warmup):
         dist.all_reduce(tt, op=dist.ReduceOp.MAX)
         t = tt.cpu()
     return t.numpy()
+
+
+def first_gemm_operands(layer):
+    """((rows, scales), None) where the dispatch delivers the first GEMM's operand quantised, else ((rows, scales), the
+    pass that quantises the bf16 rows it delivered)."""
+    if layer.qdispatch:
+        return (layer.xq, layer.xs), None
+    if layer.xq8 is not None:
+        return (layer.xq8, layer.xs8), None
+    quantise = (lambda: quantize_rows_mxfp8(layer.xrecv)) if layer.mx else (lambda: quantize_rows_fp8(layer.xrecv, layer.totals))
+    return quantise(), quantise
 
 
 def main() -> int:
@@ -100,25 +112,18 @@ def main() -> int:
         res["check"] = "ok" if err <= tol * res["ref_scale"] + 1e-3 else "FAILED"
     t_all = _time(lambda: layer.forward(x, logits, out), a.steps, a.warmup)
     layer.check()
+    if a.mx or a.fp8:
+        (xq, xs), quantise = first_gemm_operands(layer)
+        if quantise is not None:
+            res["ms_quantize_x"] = float(np.median(_time(quantise, a.steps, a.warmup)))
     if a.mx:
-        from ..ops.moe import grouped_gemm_mxfp8, quantize_rows_mxfp8
-        if layer.qdispatch:      # the dispatch delivered quantised rows
-            xq, xs = layer.xq, layer.xs
-        else:
-            xq, xs = quantize_rows_mxfp8(layer.xrecv)
-            t_q = _time(lambda: quantize_rows_mxfp8(layer.xrecv), a.steps, a.warmup)
-            res["ms_quantize_x"] = float(np.median(t_q))
         hq, hs = (layer._hq, layer._hs) if getattr(layer, "_hq", None) is not None else quantize_rows_mxfp8(layer.h)
         t_g1 = _time(lambda: grouped_gemm_mxfp8(xq, xs, layer.w13_q, layer.w13_s, layer.group_start, layer.group_rows,
                                                 out=layer.h, swiglu=True, error=layer.error[1:2]), a.steps, a.warmup)
         t_g2 = _time(lambda: grouped_gemm_mxfp8(hq, hs, layer.w2_q, layer.w2_s, layer.group_start, layer.group_rows,
                                                 out=layer.y, error=layer.error[2:3]), a.steps, a.warmup)
     elif a.fp8:
-        from ..ops.moe import grouped_gemm_fp8, quantize_rows_fp8
-        xq, xs = quantize_rows_fp8(layer.xrecv)
-        hq, hs = quantize_rows_fp8(layer.h)
-        t_q = _time(lambda: quantize_rows_fp8(layer.xrecv), a.steps, a.warmup)
-        res["ms_quantize_x"] = float(np.median(t_q))
+        hq, hs = quantize_rows_fp8(layer.h, layer.totals)
         t_g1 = _time(lambda: grouped_gemm_fp8(xq, xs, layer.w13_q, layer.w13_s, layer.group_start, layer.group_rows,
                                               out=layer.h, swiglu=True, error=layer.error[1:2]), a.steps, a.warmup)
         t_g2 = _time(lambda: grouped_gemm_fp8(hq, hs, layer.w2_q, layer.w2_s, layer.group_start, layer.group_rows,

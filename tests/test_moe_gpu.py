@@ -602,3 +602,29 @@ def test_moe_layer_back_to_back_and_captured(fp8):
         assert torch.equal(o, layer.forward(want[i], ls[i]))
     del graph
     comm.close()
+
+
+def test_moe_bench_times_the_operands_of_the_layer(monkeypatch, capsys):
+    """The fp8 benchmark's first GEMM reads the rows that the layer's dispatch delivered: the same bytes and scales as the
+    layer's own first GEMM, and no time for a quantiser pass that the layer does not run."""
+    import json
+    import sys
+
+    from rbruck_alltoallv_b200.ops import moe
+    from rbruck_alltoallv_b200.utils import moe_bench
+    T, seen, gemm = 256, [], moe.grouped_gemm_fp8
+
+    def record(Aq, scales, *args, swiglu=False, **kw):
+        if swiglu:
+            seen.append(torch.cat([Aq[:2 * T].float(), scales[:, :2 * T].t()], dim=1))
+        return gemm(Aq, scales, *args, swiglu=swiglu, **kw)
+    monkeypatch.setattr(moe, "grouped_gemm_fp8", record)
+    monkeypatch.setattr(moe_bench, "grouped_gemm_fp8", record, raising=False)
+    monkeypatch.setattr(sys, "argv", ["moe_bench", "--fp8", "--tokens", str(T), "--hidden", "512", "--inter", "512",
+                                      "--experts-per-rank", "4", "--steps", "1", "--warmup", "1"])
+    assert moe_bench.main() == 0
+    res = json.loads(capsys.readouterr().out.strip().splitlines()[-1])
+    assert "ms_quantize_x" not in res
+    assert len(seen) == 7            # three passes of the layer, then warm-up and step with fine and with coarse scales
+    want = torch.unique(seen[0], dim=0)      # (a pass may place an expert's rows in another order)
+    assert all(torch.equal(torch.unique(rows, dim=0), want) for rows in seen[1:])
