@@ -111,7 +111,7 @@ def declare_moe(lib):
     lib.rbv_quantize_rows_mxfp8.argtypes = [vp, ll, i, i, vp, vp, vp]
     lib.rbv_quantize_rows_fp8.argtypes = [vp, ll, i, i, vp, vp, vp]
     lib.rbv_quantize_used_rows_fp8.argtypes = [vp, ll, vp, i, i, vp, vp, vp]
-    lib.rbv_moe_route_local.argtypes = [vp, vp, i, i, i, vp, vp, vp, vp, vp, vp, vp, vp, vp]
+    lib.rbv_moe_route_local.argtypes = [vp, vp, i, i, i, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp]
     lib.rbv_moe_dispatch_local.argtypes = [vp, vp, i, i, vp, vp, vp, vp, vp, i, vp, vp, ll, vp, vp]
     lib.rbv_moe_combine_local.argtypes = [vp, vp, i, i, vp, vp, vp, vp]
     lib.rbv_moe_route.argtypes = [vp, i, i, vp, vp, vp, vp]

@@ -160,15 +160,16 @@ int rbv_moe_combine_pushed(rbv_ctx_t ctx, void* out, int T, int H, const float* 
 
 /* One rank (every expert on this GPU): nothing is gathered and nobody is waited for.
  * rbv_moe_route_local is rbv_moe_route and rbv_moe_layout_aligned in one launch, plus place [T, 2]: the index of every
- * routed row among its expert's rows.  scratch [E + 1] ints, zeroed once, is left zero by every call.
+ * routed row among its expert's rows, and hist, hist_all [E]: rows per expert, as router and gather leave them.
+ * scratch [E + 1] ints, zeroed once, is left zero by every call.
  * rbv_moe_dispatch_local stores token t to rows slot[t][k] = dst_base[expert] + place[t][k] of `rows`; format 0: bf16,
  * 1: e4m3 with MXFP8 scale words in atom order [H / 128][capacity / 128][128] (as rbv_quantize_rows_mxfp8 makes them),
  * 2: e4m3 with fp32 scales [H / 128][capacity] (as rbv_quantize_rows_fp8).  ret (optional): token * 2 + k of every row.
  * rbv_moe_combine_local: out[t] = w[t][0] * y[slot[t][0]] + w[t][1] * y[slot[t][1]]; slot null: rows 2 t, 2 t + 1.
  * x, rows, out and y start at multiples of 16 bytes; H % 8 == 0 (formats 1 and 2: H % 128 == 0). */
 int rbv_moe_route_local(rbv_ctx_t ctx, const float* logits, int T, int E, int align, int* topk_idx, float* topk_w,
-                        int* place, int* scratch, int* dst_base, int* group_start, int* group_rows, int* totals,
-                        void* cuda_stream);
+                        int* place, int* scratch, int* hist, int* hist_all, int* dst_base, int* group_start,
+                        int* group_rows, int* totals, void* cuda_stream);
 int rbv_moe_dispatch_local(rbv_ctx_t ctx, const void* x, int T, int H, const int* topk_idx, const int* place,
                            const int* dst_base, int* slot, unsigned* ret, int format, void* rows, void* scales,
                            long long capacity_rows, int* error_flag, void* cuda_stream);

@@ -37,6 +37,7 @@ struct RouteLocalArgs {
   float* topk_w;            // [T, 2]
   int* place;               // [T, 2]: index of the row among its expert's rows
   int* scratch;             // [E + 1], zero on entry, left zero: rows per expert, CTAs that have finished
+  int *hist, *hist_all;     // [E] each: rows per expert, as the general path leaves them (its own and the gathered one)
   int *dst_base, *group_start, *group_rows, *totals;
   char* heap[kMaxProcs];    // for the failure note only
   unsigned long long ctrl_off;
@@ -88,7 +89,7 @@ __global__ void __launch_bounds__(kRouteWarps * 32) moe_route_local_kernel(const
     for (int e2 = 0; e2 < e; e2++) base += (s_rows[e2] + a.align - 1) / a.align * a.align;
     a.dst_base[e] = base;
     a.group_start[e] = base;
-    a.group_rows[e] = s_rows[e];
+    a.group_rows[e] = a.hist[e] = a.hist_all[e] = s_rows[e];
   }
   if (tid == 0) {
     a.scratch[a.E] = 0;
@@ -260,13 +261,14 @@ using namespace rbv;
 extern "C" {
 
 int rbv_moe_route_local(rbv_ctx_t ctx, const float* logits, int T, int E, int align, int* topk_idx, float* topk_w,
-                        int* place, int* scratch, int* dst_base, int* group_start, int* group_rows, int* totals,
-                        void* stream) {
+                        int* place, int* scratch, int* hist, int* hist_all, int* dst_base, int* group_start,
+                        int* group_rows, int* totals, void* stream) {
   if (!one_rank(ctx) || E < 2 || E > kMoeMaxExperts || align < 1 || T < 1) return (int)cudaErrorInvalidValue;
   const Context& c = *ctx->c;
   RouteLocalArgs a{};
   a.logits = logits; a.T = T; a.E = E; a.align = align;
   a.topk_idx = topk_idx; a.topk_w = topk_w; a.place = place; a.scratch = scratch;
+  a.hist = hist; a.hist_all = hist_all;
   a.dst_base = dst_base; a.group_start = group_start; a.group_rows = group_rows; a.totals = totals;
   a.heap[0] = c.heap(); a.ctrl_off = c.layout().ctrl_off; a.host_status = c.host_status_dev();
   moe_route_local_kernel<<<(T + kRouteWarps - 1) / kRouteWarps, kRouteWarps * 32, 0, static_cast<cudaStream_t>(stream)>>>(a);

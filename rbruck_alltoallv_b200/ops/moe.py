@@ -473,8 +473,9 @@ class MoEExpertParallel:
         if x.data_ptr() % 16:                 # a view that starts inside a 16-byte vector
             x = x.clone()
         self._check(lib.rbv_moe_route_local(ctx, _p(logits), T, self.E, 128 if self.mx else 1, _p(self.topk_idx),
-                                            _p(self.topk_w), _p(self.place), _p(self.route_scratch), _p(self.dst_base),
-                                            _p(self.group_start), _p(self.group_rows), _p(self.totals), st), "router")
+                                            _p(self.topk_w), _p(self.place), _p(self.route_scratch), _p(self.hist),
+                                            _p(self.hist_all), _p(self.dst_base), _p(self.group_start),
+                                            _p(self.group_rows), _p(self.totals), st), "router")
         if self.qdispatch:
             fmt, rows, scales = 1, self.xq, self.xs
         elif self.fp8 and not self.mx and H % 128 == 0:

@@ -628,3 +628,21 @@ def test_moe_bench_times_the_operands_of_the_layer(monkeypatch, capsys):
     assert len(seen) == 7            # three passes of the layer, then warm-up and step with fine and with coarse scales
     want = torch.unique(seen[0], dim=0)      # (a pass may place an expert's rows in another order)
     assert all(torch.equal(torch.unique(rows, dim=0), want) for rows in seen[1:])
+
+
+@pytest.mark.parametrize("fp8", [False, True, "mx"], ids=["bf16", "fp8", "mxfp8"])
+def test_moe_one_rank_histogram(fp8):
+    """`hist` and `hist_all` hold the rows per expert of the last pass, on one rank too."""
+    from rbruck_alltoallv_b200.ops.moe import MoEExpertParallel
+    from rbruck_alltoallv_b200.parallel.comm import Communicator
+    T, E = 77, 33                                   # more experts than a warp has lanes
+    comm = Communicator(nranks=1, heap_bytes=64 << 20, arena_bytes=1 << 20)
+    layer = MoEExpertParallel(comm, E, 256, 128, T, fp8=fp8)
+    for seed in range(2):
+        torch.manual_seed(seed)
+        logits = torch.randn(T, E, device="cuda")
+        layer.forward(torch.randn(T, 256, device="cuda").to(torch.bfloat16), logits)
+        want = torch.bincount(torch.topk(logits, 2, dim=1).indices.view(-1), minlength=E)
+        assert torch.equal(layer.hist.long(), want) and torch.equal(layer.hist_all.view(-1).long(), want)
+    layer.check()
+    comm.close()
