@@ -657,3 +657,33 @@ def test_persistent_calls_replay_from_a_cuda_graph():
             verify("direct after replays " + c.kind)
     finally:
         comm.close()
+
+
+def test_two_static_ctas_per_sm_keep_inside_their_blocks(monkeypatch):
+    """RBV_STATIC_OCC=2 copies with rounds of 128 vectors.  Block s starts at vector s of a 128-byte line and ends 128 vectors
+    behind that line's start, so that its only round is a full one whose first lanes have nothing to do."""
+    from rbruck_alltoallv_b200.parallel.comm import Communicator
+    monkeypatch.setenv("RBV_STATIC_OCC", "2")
+    P, ts, pitch = 8, 16, 160
+    comm = Communicator(nranks=P, heap_bytes=16 << 20, arena_bytes=1 << 20)
+    try:
+        counts = np.tile(128 - np.arange(P, dtype=np.int32)[:, None], (1, P))             # sender s: 128 - s vectors
+        sdispls = np.tile(np.arange(P, dtype=np.int64) * 128, (P, 1))
+        rdispls = np.tile(np.arange(P, dtype=np.int64) * (pitch + 1), (P, 1))
+        send = [torch.randint(0, 256, (128 * P * ts,), dtype=torch.uint8, device="cuda") for _ in range(P)]
+        recv = [comm.symm_empty(pitch * (P + 1) * ts, torch.uint8) for _ in range(P)]
+        assert all(t.data_ptr() % 128 == 0 for t in recv)
+        for t in recv:
+            t.fill_(oracle.CANARY)
+        call = comm.prepare(send, recv, counts, sdispls, np.ascontiguousarray(counts.T), rdispls, algo="spreadout", type_size=ts)
+        assert call.kind == "static"
+        call.launch()
+        comm.check()
+        for d in range(P):
+            want = torch.full_like(recv[d], oracle.CANARY)
+            for s in range(P):
+                n, to, at = (128 - s) * ts, s * (pitch + 1) * ts, d * 128 * ts
+                want[to:to + n] = send[s][at:at + n]
+            assert torch.equal(recv[d], want), d
+    finally:
+        comm.close()

@@ -38,3 +38,10 @@ def test_mpi_stand_in_under_tsan(tmp_path):
                          [ROOT / "tests" / "native" / "shim_tsan_main.cpp", ROOT / "baseline" / "mpi_shim" / "mpi_shim.cpp"],
                          ["-fsanitize=thread"], [ROOT / "baseline" / "mpi_shim"])
     assert "bad 0" in out
+
+
+def test_device_byte_copy_stays_inside_its_block(tmp_path):
+    """The warp copy of the alltoallv kernels with lanes as fibers: for every alignment and every size around the limits of
+    its rounds, each load touches the source block, each store lies inside the destination, and the bytes are right."""
+    out = _build_and_run(tmp_path, "warp_copy", [ROOT / "tests" / "native" / "warp_copy_main.cpp"], [], [CSRC])
+    assert " 0 bad" in out
