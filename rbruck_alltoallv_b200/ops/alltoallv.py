@@ -67,12 +67,19 @@ def agreed_block_stats(c, sendcounts, ts: int):
     return mean, float(np.sqrt(max(s2 / n - mean * mean, 0.0)) / mean)
 
 
-def _auto_choice(c, recv, sendcounts, kw, agree_on_max: bool):
+def _resolves_statically(kw) -> bool:
+    """Static resolution is left on, by the caller (``static=``) and by the environment."""
+    static = kw.get("static")
+    return os.environ.get("RBV_STATIC", "1") != "0" if static is None else bool(static)
+
+
+def _auto_choice(c, recv, sendcounts, kw, agree_on_max: bool, resolved: bool = True):
     """Resolves ``algo="auto"`` into keyword arguments for the communicator, using the tuner table.  The outcome is
     the same on every process: persistent calls (``agree_on_max``) agree on the size and skew class by a host-side
     reduction; one-shot calls of a multi-process communicator use the caller's ``mean_block_bytes=`` hint (which
     must be the same everywhere) or, without it, the spread-out order with the rendezvous protocol, which mixes
-    safely with itself whatever the counts are."""
+    safely with itself whatever the counts are.  ``resolved=False``: not the rule for calls that are resolved on the host
+    (:func:`prepare`)."""
     ts = kw.get("type_size") or (recv.element_size() if isinstance(recv, torch.Tensor) else recv[0].element_size())
     host_counts = not (isinstance(sendcounts, torch.Tensor) and sendcounts.is_cuda)
     kw = dict(kw)
@@ -88,7 +95,7 @@ def _auto_choice(c, recv, sendcounts, kw, agree_on_max: bool):
     else:
         mean_block = None
     # (resolved on the host: with counts on the device a persistent call is no different from a one-shot one)
-    persistent = agree_on_max and host_counts
+    persistent = agree_on_max and host_counts and resolved and _resolves_statically(kw)
     choice = _tuner.choose(c.P, c.nproc, mean_block, cv, persistent) if mean_block is not None else dict(SAFE_CHOICE)
     forced = env_overrides()
     if "algo" in forced and forced["algo"] != choice.get("algo"):
@@ -130,16 +137,32 @@ def alltoallv(send, recv, sendcounts, sdispls=None, recvcounts=None, rdispls=Non
 def prepare(send, recv, sendcounts, sdispls=None, recvcounts=None, rdispls=None, *, comm=None, algo: str = "auto",
             **kw):
     """Persistent call (``.launch()`` repeats it).  ``algo="auto"`` resolves algorithm AND protocol once, including
-    the collective agreement on the eager cell size.  Collective over the processes when counts are on the host."""
+    the collective agreement on the eager cell size.  Collective over the processes when counts are on the host.
+
+    With one process hosting every rank a call without a table entry is resolved on the host.  That refuses what the
+    eager protocol takes: a block larger than its receiver's ``recvcounts`` entry (there a ``truncate`` status of the
+    launch), and ``recvcounts`` that reach beyond a receive buffer which holds all blocks that are sent.  Such a call goes
+    through the eager protocol."""
     c = comm or _comm.get_default_comm()
+    asked = None
     if algo == "auto":
-        kw = _auto_choice(c, recv, sendcounts, kw, agree_on_max=True)
+        asked = kw
+        kw = _auto_choice(c, recv, sendcounts, asked, agree_on_max=True)
         algo = kw.pop("algo")
     else:
         for k in ("max_block_bytes", "mean_block_bytes", "block_cv"):
             kw.pop(k, None)
     kw.pop("stream", None)
-    return c.prepare(send, recv, sendcounts, sdispls, recvcounts, rdispls, algo=algo, **kw)
+    try:
+        return c.prepare(send, recv, sendcounts, sdispls, recvcounts, rdispls, algo=algo, **kw)
+    except _comm.CommError:
+        if asked is None or c.nproc > 1 or kw.get("eager_max_bytes"):
+            raise
+        kw = _auto_choice(c, recv, sendcounts, asked, agree_on_max=True, resolved=False)
+        if not kw.get("eager_max_bytes"):
+            raise
+    kw.pop("stream", None)
+    return c.prepare(send, recv, sendcounts, sdispls, recvcounts, rdispls, algo=kw.pop("algo"), **kw)
 
 
 def alltoall(send, recv, count: int, *, comm=None, algo: str = "auto", **kw) -> None:

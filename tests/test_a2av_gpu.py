@@ -687,3 +687,42 @@ def test_two_static_ctas_per_sm_keep_inside_their_blocks(monkeypatch):
             assert torch.equal(recv[d], want), d
     finally:
         comm.close()
+
+
+def test_automatic_persistent_calls_take_what_the_eager_protocol_takes():
+    """One process, no table entry: the call is resolved on the host, and what that refuses goes through the eager protocol.
+    A recvcount below the sendcount is a status of the launch; recvcounts beyond the end of a receive buffer (outside the
+    heap) that holds all blocks are no error.  Without static resolution the choice is the
+    eager protocol from the start."""
+    from rbruck_alltoallv_b200.ops import alltoallv as A
+    P, ts = 5, 4                                        # no row of the table has five ranks
+    comm = get_comm(P)
+    prob = oracle.make_problem(dist.uniform(P, 60, seed=5) + 4, ts, 5, packed=False)
+    send_h = oracle.fill_send(prob, 5)
+    want = oracle.expected_recv(prob, send_h)
+    send = [torch.from_numpy(b).cuda() for b in send_h]
+
+    def run(recv, rc, kind, **kw):
+        for t in recv:
+            t.fill_(oracle.CANARY)
+        call = A.prepare(send, recv, prob.counts, prob.sdispls, rc, prob.rdispls, comm=comm, type_size=ts, **kw)
+        assert call.kind == kind
+        call.launch()
+        return [t.cpu().numpy() for t in recv]
+    heap = [comm.symm_empty(len(w), torch.uint8) for w in want]
+    assert oracle.first_mismatch(run(heap, prob.recvcounts, "static"), want) is None
+    assert oracle.first_mismatch(run(heap, prob.recvcounts, "eager", static=False), want) is None
+    comm.check()
+    outside = [torch.empty(len(w), dtype=torch.uint8, device="cuda") for w in want]
+    wide = prob.recvcounts.copy()
+    wide[:, P - 1] += 1000
+    assert oracle.first_mismatch(run(outside, wide, "eager"), want) is None
+    comm.check()
+    short = prob.recvcounts.copy()
+    short[2, 1] -= 1                                    # rank 2 expects less from rank 1 than rank 1 sends
+    run(heap, short, "eager")
+    st = comm.status()
+    assert st["name"] == "truncate" and st["detail"] == (1, 2)
+    comm.reset()
+    assert oracle.first_mismatch(run(heap, prob.recvcounts, "static"), want) is None
+    comm.check()

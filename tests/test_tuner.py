@@ -147,3 +147,43 @@ def test_shipped_table_has_no_entry_that_the_native_reader_misreads():
         nat = tuner.native_choose(P, G, 2.0 ** cls * 1.2, 0.9 if sk else 0.0, path=path)
         assert nat["algo"] == ent["choice"]["algo"], key
         assert nat["protocol"] == ent["choice"].get("protocol", "rendezvous"), key
+
+
+def test_automatic_prepare_falls_back_to_what_the_eager_protocol_takes(monkeypatch):
+    """One process: a call that static resolution refuses goes through the eager protocol, as without the rule for
+    persistent calls; what the table sends to rendezvous, and what the eager protocol refuses too, stays refused."""
+    import numpy as np
+    import torch
+    from rbruck_alltoallv_b200.ops import alltoallv as A
+    from rbruck_alltoallv_b200.parallel.comm import CommError
+
+    class Comm:
+        P = L = 5
+        nproc, _side, arena_bytes = 1, None, 32 << 20
+        def __init__(self, takes):
+            self.takes, self.tried = takes, []
+        def max_block_bytes(self, counts, ts):
+            return int(np.max(counts)) * ts
+        def prepare(self, *args, algo, **kw):
+            self.tried.append("eager" if kw.get("eager_max_bytes") else "rendezvous")
+            assert "stream" not in kw
+            if self.tried[-1] not in self.takes:
+                raise CommError("refused by " + self.tried[-1])
+            return self.tried[-1]
+    monkeypatch.setattr(tuner, "_TABLE", {})
+    for var in ("RBV_ALGO", "RBV_PROTOCOL", "RBV_STATIC"):
+        monkeypatch.delenv(var, raising=False)
+    recv = [torch.empty(100, dtype=torch.float32) for _ in range(5)]
+    small, big = np.full((5, 5), 10, dtype=np.int32), np.full((5, 5), 1 << 20, dtype=np.int32)
+
+    def prepare(comm, counts, **kw):
+        return A.prepare(recv, recv, counts, comm=comm, stream=None, **kw), comm.tried
+    assert prepare(Comm(("rendezvous", "eager")), small) == ("rendezvous", ["rendezvous"])
+    assert prepare(Comm(("eager",)), small) == ("eager", ["rendezvous", "eager"])
+    assert prepare(Comm(("eager", "rendezvous")), small, static=False) == ("eager", ["eager"])
+    for comm, counts, tried in ((Comm(()), small, ["rendezvous", "eager"]), (Comm(("eager",)), big, ["rendezvous"])):
+        with pytest.raises(CommError, match="refused by " + tried[-1]):
+            prepare(comm, counts)
+        assert comm.tried == tried
+    monkeypatch.setenv("RBV_STATIC", "0")
+    assert prepare(Comm(("eager", "rendezvous")), small) == ("eager", ["eager"])
