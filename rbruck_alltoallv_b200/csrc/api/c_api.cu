@@ -165,11 +165,12 @@ void* rbv_prepare(rbv_ctx_t ctx, int algo, int n, int r, int r2, int b, int b2, 
                             rdispls, counts_on_device, bytes_hint, flags, grid, chunk_bytes, nullptr, nullptr, nullptr,
                             nullptr);
 }
-// 0 dynamic rendezvous kernel, 1 eager kernel, 2 static rendezvous kernel; out3 = grid, cooperative launch needed, items
+// 0 dynamic rendezvous kernel, 1 eager kernel, 2 static rendezvous kernel, 3 local kernel; out3 = grid, cooperative launch
+// needed, items listed in advance
 int rbv_prepared_info(void* prepared, long long* out3) {
   const Prepared* pc = static_cast<Prepared*>(prepared);
   if (out3) { out3[0] = pc->grid; out3[1] = pc->cooperative ? 1 : 0; out3[2] = pc->is_static ? pc->static_items : pc->ka.nitems; }
-  return pc->is_static ? 2 : (pc->eager ? 1 : 0);
+  return pc->is_local ? 3 : (pc->is_static ? 2 : (pc->eager ? 1 : 0));
 }
 int rbv_launch(rbv_ctx_t ctx, void* prepared, void* cuda_stream) {
   int rc = ctx->c->launch(*static_cast<Prepared*>(prepared), static_cast<cudaStream_t>(cuda_stream));

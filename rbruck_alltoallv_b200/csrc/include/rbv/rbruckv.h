@@ -101,8 +101,8 @@ void* rbv_prepare_global(rbv_ctx_t ctx, int algo, int n, int r, int r2, int b, i
                          int counts_on_device, long long bytes_hint, unsigned flags, int grid, size_t chunk_bytes,
                          const int* g_counts, const int* g_caps, const long long* g_rdispls,
                          const unsigned long long* g_recvoff);
-/* Which kernel a prepared call runs: 0 dynamic rendezvous, 1 eager, 2 static rendezvous;
- * out3 = grid, cooperative launch needed (0 / 1), work items. */
+/* Which kernel a prepared call runs: 0 dynamic rendezvous, 1 eager, 2 static rendezvous, 3 local (direct schedule among the
+ * ranks of one process); out3 = grid, cooperative launch needed (0 / 1), work items listed in advance. */
 int rbv_prepared_info(void* prepared, long long* out3);
 int rbv_launch(rbv_ctx_t ctx, void* prepared, void* cuda_stream);
 void rbv_prepared_free(rbv_ctx_t ctx, void* prepared);

@@ -52,7 +52,7 @@ class _Block:
 class PreparedCall:
     """A resolved collective; see :meth:`Communicator.prepare`."""
 
-    KINDS = {0: "rendezvous", 1: "eager", 2: "static"}
+    KINDS = {0: "rendezvous", 1: "eager", 2: "static", 3: "local"}
 
     def __init__(self, comm: "Communicator", handle, keep, mirrored=None):
         self._comm, self._h, self._keep = comm, C.c_void_p(handle), keep
@@ -62,7 +62,8 @@ class PreparedCall:
         self._dev = comm.device
         info = (C.c_longlong * 3)()
         #: which kernel runs the call: "static" (all counts resolved on the host, no metadata phase),
-        #: "rendezvous" (metadata exchanged by the kernel) or "eager"
+        #: "rendezvous" (metadata exchanged by the kernel), "eager" or "local" (counts on the device, every rank in this
+        #: process, a direct schedule: the kernel reads the counts where they are)
         self.kind = self.KINDS[comm._lib.rbv_prepared_info(self._h, info)]
         self.grid, self.cooperative, self.items = int(info[0]), bool(info[1]), int(info[2])
 

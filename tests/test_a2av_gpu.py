@@ -726,3 +726,19 @@ def test_automatic_persistent_calls_take_what_the_eager_protocol_takes():
     comm.reset()
     assert oracle.first_mismatch(run(heap, prob.recvcounts, "static"), want) is None
     comm.check()
+
+
+def test_persistent_calls_name_the_kernel_that_runs_them():
+    """Counts on the device, one process: the local kernel for a direct schedule; the kernel that exchanges metadata for a
+    schedule with relays, a traced call, and with static resolution switched off.  The bytes are the same."""
+    counts = dist.uniform(4, 300, seed=8)
+    kw = dict(device_counts=True, persistent=True, launches=2)
+    assert run_case(4, "spreadout", 4, counts, **kw).kind == "local"
+    assert run_case(4, "spreadout", 4, counts, static=False, **kw).kind == "rendezvous"
+    assert run_case(4, "rbruck", 4, counts, r=2, **kw).kind == "rendezvous"
+    comm = get_comm(4)
+    comm.enable_trace(True)
+    try:
+        assert run_case(4, "spreadout", 4, counts, **kw).kind == "rendezvous"
+    finally:
+        comm.enable_trace(False)
