@@ -305,11 +305,17 @@ class MoEExpertParallel:
         # MXFP8: rows are quantised by the dispatch itself and cross NVLink as e4m3 + scale words (half the bytes, no
         # quantiser pass on the owner); RBV_MOE_QDISPATCH=0 dispatches bf16 rows and quantises them afterwards
         self.qdispatch = self.mx and hidden % 128 == 0 and os.environ.get("RBV_MOE_QDISPATCH", "1") != "0"
+        # Block-scaled fp8 with one rank: the dispatch quantises the rows too, straight into what the GEMM reads
+        self.xq8 = self.xs8 = None
         if self.qdispatch:
             self.xrecv = None
             self.xq = comm.symm_empty((self.cap, hidden), torch.uint8)
             self.sfrow = comm.symm_empty((self.cap, hidden // 128), i32)
             self.xs = torch.full((hidden // 128, self.cap), 0x7f7f7f7f, dtype=i32, device=dev)   # atom order
+        elif self.P == 1 and self.fp8 and not self.mx:
+            self.xrecv = None
+            self.xq8 = torch.empty(self.cap, hidden, dtype=torch.uint8, device=dev)
+            self.xs8 = torch.empty(hidden // 128, self.cap, dtype=torch.float32, device=dev)
         else:
             self.xrecv = comm.symm_empty((self.cap, hidden), bf)
         self.h = torch.empty(self.cap, inter, dtype=bf, device=dev)
@@ -326,10 +332,6 @@ class MoEExpertParallel:
         self.error = torch.zeros(4, dtype=i32, device=dev)
         self.place = torch.empty(tokens, 2, dtype=i32, device=dev)             # one rank: see _route_and_dispatch_local
         self.route_scratch = torch.zeros(self.E + 1, dtype=i32, device=dev)
-        self.xq8 = self.xs8 = None       # one rank, block-scaled fp8: the rows and scales that the dispatch delivers
-        if self.P == 1 and self.fp8 and not self.mx and hidden % 128 == 0:
-            self.xq8 = torch.empty(self.cap, hidden, dtype=torch.uint8, device=dev)
-            self.xs8 = torch.empty(hidden // 128, self.cap, dtype=torch.float32, device=dev)
         # Streamed dispatch (bf16 path): rows travel expert by expert, every landed row bumps its expert's counter on
         # the owner, and the first grouped GEMM, launched on a second stream next to the dispatch, starts an expert as
         # soon as its rows are complete.  Opt-in (``overlap=True`` or RBV_MOE_OVERLAP=1): measured on B200 with the
@@ -357,7 +359,8 @@ class MoEExpertParallel:
         self.y2 = comm.symm_empty((2 * tokens, hidden), bf) if self.push else None      # results, by (token, k)
         self.y = None if self.push else comm.symm_empty((self.cap, hidden), bf)         # results, expert-sorted
         heap0 = self.lib.rbv_ctx_heap(comm._ctx, comm.proc)
-        self.xrecv_off = (self.xq if self.qdispatch else self.xrecv).data_ptr() - heap0
+        rows = self.xq if self.qdispatch else self.xrecv
+        self.xrecv_off = rows.data_ptr() - heap0 if rows is not None else 0
         self.sfrow_off = (self.sfrow.data_ptr() - heap0) if self.qdispatch else 0
         self.y_off = 0 if self.push else self.y.data_ptr() - heap0
         self.ready_off = self.ready.data_ptr() - heap0
@@ -478,7 +481,7 @@ class MoEExpertParallel:
                                             _p(self.group_rows), _p(self.totals), st), "router")
         if self.qdispatch:
             fmt, rows, scales = 1, self.xq, self.xs
-        elif self.fp8 and not self.mx and H % 128 == 0:
+        elif self.xq8 is not None:
             fmt, rows, scales = 2, self.xq8, self.xs8
         else:
             fmt, rows, scales = 0, self.xrecv, None

@@ -646,3 +646,22 @@ def test_moe_one_rank_histogram(fp8):
         assert torch.equal(layer.hist.long(), want) and torch.equal(layer.hist_all.view(-1).long(), want)
     layer.check()
     comm.close()
+
+
+def test_moe_fp8_one_rank_needs_no_bf16_receive_buffer():
+    """The dispatch of the one-rank fp8 layer stores quantised rows: the symmetric heap holds the layer's results and not
+    the bf16 rows as well."""
+    from rbruck_alltoallv_b200.ops.moe import MoEExpertParallel, reference_forward
+    from rbruck_alltoallv_b200.parallel.comm import Communicator
+    T, H, I, E = 1024, 1024, 256, 4
+    comm = Communicator(nranks=1, heap_bytes=2 * T * 2 * H * 2 + (1 << 20), arena_bytes=1 << 20)   # one [capacity, H] in bf16
+    layer = MoEExpertParallel(comm, E, H, I, T, seed=4, fp8=True)
+    assert layer.xrecv is None
+    torch.manual_seed(4)
+    x, logits = torch.randn(T, H, device="cuda").to(torch.bfloat16), torch.randn(T, E, device="cuda")
+    out = layer.forward(x, logits)
+    layer.check()
+    ref, _, _ = reference_forward(x, logits, layer.w13, layer.w2)
+    # e4m3 operands in two GEMMs against the unquantised weights: the bound of the layer's own test
+    assert (out.float() - ref).norm().item() <= 0.08 * ref.norm().item()
+    comm.close()
