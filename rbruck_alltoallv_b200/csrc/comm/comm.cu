@@ -6,6 +6,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <memory>
 #include <stdexcept>
 
 #include <cuda.h>
@@ -175,6 +176,31 @@ bool Context::in_heap(const void* p, size_t bytes) const {
   return c >= heap_ + lay_.user_off && c + bytes <= heap_ + lay_.total_bytes;
 }
 
+namespace {
+// One process: the warp that stores a chunk into a staging cell also executes the hop that forwards it.  That wants every
+// cell to be written once, and read at most once, after that and by a hop of the same block; `pred` stays empty otherwise.
+void find_chains(DevPlan* dp, int P) {
+  std::vector<int> writer((size_t)P * dp->plan.ncells, -1);
+  dp->pred.assign(dp->h_ops.size(), -1);
+  for (size_t i = 0; i < dp->h_ops.size(); i++) {
+    const Op& o = dp->h_ops[i];
+    bool ok = true;
+    if (o.src_cell >= 0) {
+      int& w = writer[(size_t)o.src * dp->plan.ncells + o.src_cell];
+      ok = w >= 0 && dp->h_ops[w].origin == o.origin && dp->h_ops[w].dest == o.dest;
+      dp->pred[i] = w;
+      w = -2;                       // read
+    }
+    if (o.dst_cell >= 0) {
+      int& w = writer[(size_t)o.dst * dp->plan.ncells + o.dst_cell];
+      ok = ok && w == -1;
+      w = (int)i;
+    }
+    if (!ok) { dp->pred.clear(); return; }
+  }
+}
+}  // namespace
+
 const DevPlan* Context::plan_for(const AlgoSpec& s) {
   auto key = std::make_tuple(s.algo, s.P, s.n, s.r, s.r2, s.b, s.b2);
   auto it = plans_.find(key);
@@ -195,6 +221,7 @@ const DevPlan* Context::plan_for(const AlgoSpec& s) {
       dp->nops = (int)ops.size();
       dp->h_ops = ops;
       for (const Op& o : dp->plan.ops) if (op_nparts(o)) dp->has_parts = true;
+      if (nproc_ == 1 && dp->plan.ncells > 0 && !dp->has_parts) find_chains(dp.get(), P_);
       if (dp->nops) {
         RBV_CUDA_THROW(cudaMalloc(&dp->d_ops, ops.size() * sizeof(Op)));
         RBV_CUDA_THROW(cudaMemcpy(dp->d_ops, ops.data(), ops.size() * sizeof(Op), cudaMemcpyHostToDevice));
@@ -713,133 +740,79 @@ int Context::prepare_static(const DevPlan* dp, int ts, const CallArgs& ca, const
     if (first_el) *first_el = f;
     return (unsigned long long)n * ts;
   };
-  // One process: the warp that stores a chunk into a staging cell also executes the hop that forwards it, which wants
-  // every cell to be written once, and read at most once and after that.
-  bool relay = nproc_ == 1 && ncells > 0 && !dp->has_parts;
-  if (relay) {
-    std::vector<unsigned char> state((size_t)P * ncells, 0);   // 0 empty, 1 written, 2 read
-    auto step = [&](int rank, int cell, unsigned char want) {
-      unsigned char& c = state[(size_t)rank * ncells + cell];
-      if (c++ != want) relay = false;
-    };
-    for (const Op& o : dp->h_ops) {
-      if (o.src_cell >= 0) step(o.src, o.src_cell, 1);
-      if (o.dst_cell >= 0) step(o.dst, o.dst_cell, 0);
-    }
+  const bool relay = !dp->pred.empty();   // one process: a warp forwards what it stored itself, see find_chains
+  // ---- the slice of every op of this process ----
+  struct Slice { unsigned long long bytes; long long first; unsigned n, wide, at, wide_at; };
+  const std::vector<Op>& ops = dp->h_ops;
+  std::vector<Slice> slices(ops.size());
+  double own_work = 0;
+  for (size_t i = 0; i < ops.size(); i++) {
+    slices[i].bytes = slice_bytes(ops[i], &slices[i].first);
+    own_work += (double)slices[i].bytes;
   }
-  constexpr unsigned kNoItem = ~0u;
-  std::vector<unsigned> stored(relay ? (size_t)P * ncells : 0, kNoItem);   // per cell: the item that stores its chunk 0
-  std::vector<unsigned> pred;                                             // per item: the item whose chunk it forwards
   // ---- chunk size: the same on every process (receivers count chunks), so it is derived from the busiest process ----
   unsigned long long chunk = opt.chunk_bytes;
+  bool small_chunks = false;
   if (!chunk) {
-    std::vector<double> work(nproc_, 0.0);
-    for (const Op& o : dp->plan.ops) work[o.src / L] += (double)slice_bytes(o, nullptr);
-    chunk = chunk_for(*std::max_element(work.begin(), work.end()), static_max_ctas_);
+    double most = own_work;
+    if (nproc_ > 1) {
+      std::vector<double> work(nproc_, 0.0);
+      for (const Op& o : dp->plan.ops) work[o.src / L] += (double)slice_bytes(o, nullptr);
+      most = *std::max_element(work.begin(), work.end());
+    }
+    chunk = chunk_for(most, static_max_ctas_);
     // What the resident warps have stored but not yet forwarded should still be in L2 when they read it, and what they
     // touch at one time lies closer together in any case.  Measured with one process and blocks up to 4 MB, chunks of 64,
     // 32, 16, 8, 4 KB: two-layer 150, 141, 126, 118, 130 us, direct 95, 96, 93, 91, 97 us.
-    if (nproc_ == 1) chunk = std::min<unsigned long long>(chunk, kLocalChunk);
+    if (nproc_ == 1 && chunk > kLocalChunk) { chunk = kLocalChunk; small_chunks = true; }
   }
   chunk = align_up(chunk, 16);
   const unsigned long long fpc = ncells > 0 ? lay_.flags_per_rank / (unsigned long long)ncells : 0;
   if (ncells > 0 && !relay) chunk = std::max<unsigned long long>(chunk, align_up((stride + fpc - 1) / fpc, 16));
   if (chunk > 0xffffffffull) chunk = 0xfffffff0ull;
   auto nchunks = [&](unsigned long long bytes) { return (bytes + chunk - 1) / chunk; };
+  for (Slice& sl : slices) sl.n = (unsigned)nchunks(sl.bytes);
+  // An item of 32 bytes per 8 KB makes a long table, slow to fill and to upload.  A wide item stands for 2, 4 or 8 chunks,
+  // which the kernel deals one by one, and the chunks that are left of a block have an item each.  The width is the one with
+  // the shortest table.  Wide items are dealt first, whatever round of the schedule they belong to; chains, the longest of
+  // which should not come last, keep plan order unless blocks are so long that little is left of them (32 ranks, radix 2,
+  // blocks up to 64 KB: 53 us in plan order, 56 us with wide items first).  Prepared and uploaded, an item per 8 KB / wide items:
+  // two-layer, 8 ranks, 4 MB 2510 / 65 us, direct 4 MB 527 / 55 us, direct, 64 ranks, 48 KB 609 / 212 us.
+  unsigned wide_shift = 0;
+  if (small_chunks && (ncells == 0 || relay)) {
+    size_t count[4] = {0, 0, 0, 0};
+    for (const Slice& sl : slices)
+      for (unsigned w = 0; w <= 3; w++) count[w] += (sl.n >> w) + (sl.n & ((1u << w) - 1));
+    for (unsigned w = 1; w <= 3; w++)
+      if (count[w] < count[wide_shift]) wide_shift = w;
+    if (relay && 4 * count[wide_shift] > count[0]) wide_shift = 0;
+  }
 
   // ---- items of this process: plan order.  Across GPUs the chunks of the ops of one key alternate, so that a rank
   // writes to all peers of a round at once (with one block after the other, two senders meet at one receiver while
   // another receiver idles as soon as block sizes differ).  Inside one GPU the copies are bound by HBM, where
-  // walking block after block measured 4-8 % faster than alternating (better DRAM page locality). ----
+  // walking block after block measured 4-8 % faster than alternating (better DRAM page locality).
+  // Chains: an item that stores a cell chunk leads to the one that forwards it.  The table holds the wide items that are
+  // dealt to the warps, then the others that are dealt, both in plan order, then those that others lead to. ----
   const bool alternate = nproc_ > 1;
-  std::vector<StaticItem> items;
-  const std::vector<Op>& ops = dp->h_ops;
-  auto stage_addr = [&](int proc, int lr, int cell) {
-    return reinterpret_cast<unsigned long long>(peer_[proc]) + lay_.stage_off + (unsigned long long)(lr * 2) * lay_.arena_bytes +
-           (unsigned long long)cell * stride;
-  };
-  for (size_t g0 = 0; g0 < ops.size();) {
-    size_t g1 = g0;
-    while (g1 < ops.size() && ops[g1].key == ops[g0].key) g1++;
-    unsigned long long maxn = 0;
-    for (size_t i = g0; i < g1; i++) maxn = std::max(maxn, nchunks(slice_bytes(ops[i], nullptr)));
-    // (outer, inner) = (chunk, op) when alternating, (op, chunk) otherwise
-    const unsigned long long n_outer = alternate ? maxn : (unsigned long long)(g1 - g0);
-    const unsigned long long n_inner = alternate ? (unsigned long long)(g1 - g0) : maxn;
-    for (unsigned long long outer = 0; outer < n_outer; outer++)
-      for (unsigned long long inner = 0; inner < n_inner; inner++) {
-        const unsigned long long k = alternate ? outer : inner;
-        const size_t i = g0 + (size_t)(alternate ? inner : outer);
-        const Op& o = ops[i];
-        long long f = 0;
-        const unsigned long long bytes = slice_bytes(o, &f);
-        if (k >= nchunks(bytes)) continue;
-        const int lsrc = o.src - first, dproc = o.dst / L, ldst = o.dst - dproc * L;
-        const unsigned long long off = k * chunk;
-        StaticItem it{};
-        unsigned from = kNoItem;
-        it.len = (unsigned)std::min<unsigned long long>(chunk, bytes - off);
-        it.dst_rank = o.dst;
-        unsigned fl = 0;
-        if (o.src_cell < 0) {
-          it.src = reinterpret_cast<unsigned long long>(ca.sendbufs[lsrc]) +
-                   (unsigned long long)(ca.sdispls[(size_t)lsrc * P + o.dest] + f) * ts + off;
-          it.wait_flag = kNoFlag;
-        } else {
-          it.src = stage_addr(proc_, lsrc, o.src_cell) + off;
-          it.wait_flag = (unsigned)((unsigned long long)lsrc * lay_.flags_per_rank + (unsigned long long)o.src_cell * fpc + k);
-          if (relay) {
-            it.wait_flag = kNoFlag;
-            from = stored[(size_t)lsrc * ncells + o.src_cell] + (unsigned)k;   // (the chunks of an op are consecutive items)
-          }
-          fl |= ITEM_SRC_STAGE;
-        }
-        if (o.dst_cell < 0) {
-          it.dst = reinterpret_cast<unsigned long long>(peer_[dproc]) + gro[o.dst] +
-                   (unsigned long long)(grd[(size_t)o.dst * P + o.origin] + f) * ts + off;
-          it.signal_flag = kNoFlag;
-        } else {
-          it.dst = stage_addr(dproc, ldst, o.dst_cell) + off;
-          it.signal_flag = (unsigned)((unsigned long long)ldst * lay_.flags_per_rank + (unsigned long long)o.dst_cell * fpc + k);
-          if (relay) {
-            it.signal_flag = kNoFlag;
-            if (k == 0) stored[(size_t)ldst * ncells + o.dst_cell] = (unsigned)items.size();
-          }
-          fl |= ITEM_DST_STAGE;
-        }
-        if (dproc != proc_) fl |= ITEM_REMOTE;
-        if (o.flags & kOpSelf) fl |= ITEM_SELF;
-        it.flags = (unsigned short)(fl | (std::min<unsigned>(op_key_index(o), 255u) << 8));
-        items.push_back(it);
-        if (relay) pred.push_back(from);
-      }
-    g0 = g1;
+  auto forwards = [&](size_t i) { return relay && dp->pred[i] >= 0; };
+  size_t wide = 0, dealt = 0, nitems = 0;
+  for (size_t i = 0; i < ops.size(); i++) {
+    Slice& sl = slices[i];
+    sl.wide = wide_shift ? sl.n >> wide_shift : 0;
+    sl.n -= sl.wide << wide_shift;
+    nitems += sl.wide + sl.n;
+    if (!forwards(i)) { wide += sl.wide; dealt += sl.wide + sl.n; }
   }
-  // Chains: an item that stores a cell chunk leads to the one that forwards it.  The heads keep plan order and are what
-  // the warps are dealt; the others lie behind them.
-  size_t heads = items.size();
-  if (relay) {
-    std::vector<unsigned> at(items.size());
-    heads = 0;
-    for (size_t i = 0; i < items.size(); i++)
-      if (pred[i] == kNoItem) at[i] = (unsigned)heads++;
-    unsigned tail = (unsigned)heads;
-    for (size_t i = 0; i < items.size(); i++)
-      if (pred[i] != kNoItem) {
-        at[i] = tail++;
-        items[pred[i]].signal_flag = at[i];
-        items[pred[i]].flags |= ITEM_NEXT;
-      }
-    std::vector<StaticItem> sorted(items.size());
-    for (size_t i = 0; i < items.size(); i++) sorted[at[i]] = items[i];
-    items.swap(sorted);
+  unsigned next_wide = 0, next_one = (unsigned)wide, next_tail = (unsigned)dealt;
+  for (size_t i = 0; i < ops.size(); i++) {
+    unsigned& w = forwards(i) ? next_tail : next_wide;
+    slices[i].wide_at = w;
+    w += slices[i].wide;
+    unsigned& o = forwards(i) ? next_tail : next_one;
+    slices[i].at = o;
+    o += slices[i].n;
   }
-
-  // chunks that land in the receive buffers of this process's ranks, from every process
-  std::vector<unsigned long long> expect(L, 0);
-  for (const Op& o : dp->plan.ops)
-    if (o.dst_cell < 0 && o.dst / L == proc_) expect[o.dst - first] += nchunks(slice_bytes(o, nullptr));
-
   // blocks to copy on to the caller's own buffers once everything has arrived (pieces of at most 64 KB, so that
   // the warps of the copying CTA share a large block)
   std::vector<DrainItem> drain;
@@ -860,23 +833,106 @@ int Context::prepare_static(const DevPlan* dp, int ts, const CallArgs& ca, const
       }
     }
 
-  // ---- device copy: [expect[L] | items | drain] ----
+  // ---- the table as it is uploaded: [expect[L] | items | drain] ----
   const size_t head = align_up(sizeof(unsigned long long) * L, 32);
-  const size_t items_bytes = std::max<size_t>(items.size(), 1) * sizeof(StaticItem);
+  const size_t items_bytes = std::max<size_t>(nitems, 1) * sizeof(StaticItem);
   const size_t bytes = head + items_bytes + drain.size() * sizeof(DrainItem);
-  std::vector<char> blob(bytes, 0);
-  std::memcpy(blob.data(), expect.data(), sizeof(unsigned long long) * L);
-  if (!items.empty()) std::memcpy(blob.data() + head, items.data(), items.size() * sizeof(StaticItem));
-  if (!drain.empty()) std::memcpy(blob.data() + head + items_bytes, drain.data(), drain.size() * sizeof(DrainItem));
+  const std::unique_ptr<char[]> blob(new char[bytes]);   // (every item is written below; a first touch of each page is enough)
+  StaticItem* const items = reinterpret_cast<StaticItem*>(blob.get() + head);
+  auto stage_addr = [&](int proc, int lr, int cell) {
+    return reinterpret_cast<unsigned long long>(peer_[proc]) + lay_.stage_off + (unsigned long long)(lr * 2) * lay_.arena_bytes +
+           (unsigned long long)cell * stride;
+  };
+  // op i as one item; its pieces differ in address, length, flags and successor
+  auto whole = [&](size_t i) {
+    const Op& o = ops[i];
+    const int lsrc = o.src - first, dproc = o.dst / L, ldst = o.dst - dproc * L;
+    StaticItem it{};
+    it.dst_rank = o.dst;
+    it.wait_flag = it.signal_flag = kNoFlag;
+    unsigned fl = 0;
+    if (o.src_cell < 0) {
+      it.src = reinterpret_cast<unsigned long long>(ca.sendbufs[lsrc]) +
+               (unsigned long long)(ca.sdispls[(size_t)lsrc * P + o.dest] + slices[i].first) * ts;
+    } else {
+      it.src = stage_addr(proc_, lsrc, o.src_cell);
+      if (!relay) it.wait_flag = (unsigned)((unsigned long long)lsrc * lay_.flags_per_rank + (unsigned long long)o.src_cell * fpc);
+      fl |= ITEM_SRC_STAGE;
+    }
+    if (o.dst_cell < 0) {
+      it.dst = reinterpret_cast<unsigned long long>(peer_[dproc]) + gro[o.dst] +
+               (unsigned long long)(grd[(size_t)o.dst * P + o.origin] + slices[i].first) * ts;
+    } else {
+      it.dst = stage_addr(dproc, ldst, o.dst_cell);
+      if (!relay) it.signal_flag = (unsigned)((unsigned long long)ldst * lay_.flags_per_rank + (unsigned long long)o.dst_cell * fpc);
+      fl |= ITEM_DST_STAGE;
+    }
+    if (dproc != proc_) fl |= ITEM_REMOTE;
+    if (o.flags & kOpSelf) fl |= ITEM_SELF;
+    it.flags = (unsigned short)(fl | (std::min<unsigned>(op_key_index(o), 255u) << 8));
+    return it;
+  };
+  // `size` bytes of op i from byte `off` on; k: the chunk that its flags belong to
+  auto piece = [&](StaticItem it, size_t i, unsigned long long off, unsigned long long size, unsigned k) {
+    it.src += off;
+    it.dst += off;
+    it.len = (unsigned)std::min<unsigned long long>(size, slices[i].bytes - off);
+    if (it.wait_flag != kNoFlag) it.wait_flag += k;
+    if (it.signal_flag != kNoFlag) it.signal_flag += k;
+    return it;
+  };
+  if (!alternate) {
+    const unsigned long long wide_bytes = chunk << wide_shift;
+    auto lead_to = [&](unsigned from, unsigned to) {
+      items[from].signal_flag = to;
+      items[from].flags |= ITEM_NEXT;
+    };
+    for (size_t i = 0; i < ops.size(); i++) {
+      const Slice& sl = slices[i];
+      if (!sl.bytes) continue;
+      const StaticItem it = whole(i);
+      for (unsigned k = 0; k < sl.wide; k++) items[sl.wide_at + k] = piece(it, i, k * wide_bytes, wide_bytes, 0);
+      for (unsigned k = 0; k < sl.n; k++) items[sl.at + k] = piece(it, i, sl.wide * wide_bytes + k * chunk, chunk, k);
+      if (!forwards(i)) continue;
+      const Slice& from = slices[dp->pred[i]];
+      for (unsigned k = 0; k < sl.wide; k++) lead_to(from.wide_at + k, sl.wide_at + k);
+      for (unsigned k = 0; k < sl.n; k++) lead_to(from.at + k, sl.at + k);
+    }
+  } else {
+    size_t at = 0;
+    std::vector<StaticItem> of_key;
+    for (size_t g0 = 0, g1; g0 < ops.size(); g0 = g1) {
+      unsigned maxn = 0;
+      of_key.clear();
+      for (g1 = g0; g1 < ops.size() && ops[g1].key == ops[g0].key; g1++) {
+        maxn = std::max(maxn, slices[g1].n);
+        of_key.push_back(whole(g1));
+      }
+      for (unsigned k = 0; k < maxn; k++)
+        for (size_t i = g0; i < g1; i++)
+          if (k < slices[i].n) items[at++] = piece(of_key[i - g0], i, k * chunk, chunk, k);
+    }
+  }
+
+  // chunks that land in the receive buffers of this process's ranks, from every process
+  std::vector<unsigned long long> expect(L, 0);   // (one process counts no arrivals)
+  for (const Op& o : dp->plan.ops)
+    if (nproc_ > 1 && o.dst_cell < 0 && o.dst / L == proc_) expect[o.dst - first] += nchunks(slice_bytes(o, nullptr));
+
+  std::memcpy(blob.get(), expect.data(), sizeof(unsigned long long) * L);
+  if (!drain.empty()) std::memcpy(blob.get() + head + items_bytes, drain.data(), drain.size() * sizeof(DrainItem));
   RBV_CUDA_THROW(cudaMalloc(&out->owned_items, bytes));
-  RBV_CUDA_THROW(cudaMemcpy(out->owned_items, blob.data(), bytes, cudaMemcpyHostToDevice));
+  RBV_CUDA_THROW(cudaMemcpy(out->owned_items, blob.get(), bytes, cudaMemcpyHostToDevice));
 
   StaticArgs& sa = out->sa;
   std::memset(&sa, 0, sizeof sa);
   sa.P = P; sa.L = L; sa.nproc = nproc_; sa.proc = proc_;
   sa.flags = trace_ ? (unsigned)CALL_TRACE : 0u;
-  sa.nitems = (unsigned)heads;
-  out->static_items = (unsigned)items.size();
+  sa.wide = (unsigned)(wide << wide_shift);
+  sa.nitems = sa.wide + (unsigned)(dealt - wide);
+  sa.wide_shift = wide_shift;
+  sa.chunk = (unsigned)chunk;
+  out->static_items = (unsigned)nitems;
   sa.expect = static_cast<const unsigned long long*>(out->owned_items);
   sa.items = reinterpret_cast<const StaticItem*>(static_cast<char*>(out->owned_items) + head);
   sa.drain = reinterpret_cast<const DrainItem*>(static_cast<char*>(out->owned_items) + head + items_bytes);
@@ -886,14 +942,14 @@ int Context::prepare_static(const DevPlan* dp, int ts, const CallArgs& ca, const
   for (int q = 0; q < nproc_; q++) sa.heap[q] = peer_[q];
   sa.host_status = host_status_dev_;
   sa.host_trace = host_trace_dev_;
-  std::memcpy(sa.inl, items.data(), std::min(items.size(), (size_t)kInlineItems) * sizeof(StaticItem));
+  std::memcpy(sa.inl, items, std::min(nitems, (size_t)kInlineItems) * sizeof(StaticItem));
   const int warps_per_cta = kThreads / 32;
   // One process: item c goes to warp c / grid of CTA c % grid (a2av_static.cu), so with one CTA per item (up to the
   // CTAs that are resident at once) a small call spreads over as many SMs as it has items instead of filling the 16
   // warps of a few.  Several processes: 16 items per CTA (see the kernel).
   const bool spread = static_spread_ && nproc_ == 1;
   int grid = opt.grid > 0 ? opt.grid
-                          : (int)(spread ? heads : (heads + warps_per_cta - 1) / warps_per_cta);
+                          : (int)std::min<size_t>(static_max_ctas_, spread ? sa.nitems : (dealt + warps_per_cta - 1) / warps_per_cta);
   out->grid = std::max(1, std::min(grid, static_max_ctas_));
   out->is_static = true;
   out->eager = false;
@@ -901,7 +957,7 @@ int Context::prepare_static(const DevPlan* dp, int ts, const CallArgs& ca, const
   // for, on every process.  With one round of items per warp that order cannot block as long as CTAs start in index
   // order; several rounds per warp need all CTAs resident.
   // (Where a warp forwards what it stored itself nobody waits.)
-  out->cooperative = ncells > 0 && !relay && items.size() > (size_t)out->grid * warps_per_cta;
+  out->cooperative = ncells > 0 && !relay && nitems > (size_t)out->grid * warps_per_cta;
   return 0;
 }
 

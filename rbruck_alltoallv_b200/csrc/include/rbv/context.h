@@ -21,6 +21,8 @@ struct DevPlan {
   Op* d_ops = nullptr;     // ops of this process's ranks
   std::vector<Op> h_ops;   // host copy of the same list
   bool has_parts = false;  // some block travels in slices (split_alltoallv)
+  std::vector<int> pred;   // one process: per op the op that stores the cell it reads (-1: none), empty where a cell is
+                           // not written once and read once
   unsigned* d_done = nullptr;
   int nops = 0;
   // eager protocol: the same ops retargeted at arrival / staging cells, followed by one unpack op per

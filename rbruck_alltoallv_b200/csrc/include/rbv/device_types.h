@@ -254,12 +254,15 @@ struct alignas(16) DrainItem {
 struct StaticArgs {
   int P, L, nproc, proc;
   unsigned flags;                       // CALL_TRACE
-  unsigned nitems;                      // items dealt to warps (those that others lead to with ITEM_NEXT lie behind them)
+  unsigned nitems;                      // chunks dealt to warps (items that others lead to with ITEM_NEXT lie behind those
+                                        // that are dealt)
   unsigned seq_hint, use_seq_hint;      // as in KernelArgs
-  const StaticItem* items;              // issue order; item c is handled by warp c mod (warps in the grid)
+  const StaticItem* items;              // issue order; dealt chunk c is handled by warp c mod (warps in the grid)
   const unsigned long long* expect;     // [L] chunks that land in each local rank's receive buffer per call
   const DrainItem* drain;               // copies made after the last arrival (receive buffers mirrored elsewhere)
-  unsigned ndrain, pad;
+  unsigned ndrain;
+  unsigned wide, wide_shift, chunk;     // the first `wide` of them are those of wide items, 1 << wide_shift chunks of `chunk`
+                                        // bytes each; the others have an item each
   unsigned long long timeout_ns;
   HeapLayout lay;
   char* heap[kMaxProcs];

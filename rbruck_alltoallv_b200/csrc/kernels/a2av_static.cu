@@ -50,7 +50,8 @@ __device__ void static_error(const StaticArgs& a, int code, int site, int d0, in
 
 // MINB = CTAs per SM the register budget is cut for: 1 keeps everything in registers (16 warps per SM), 2 trades a
 // few spilled words for twice the warps, hence twice the loads in flight per SM.
-template <int MINB>
+// WIDE: the table has items of several chunks (one process, long blocks).
+template <int MINB, bool WIDE>
 __global__ void __launch_bounds__(kThreads, MINB) a2av_static_kernel(const __grid_constant__ StaticArgs a) {
   __shared__ unsigned s_arrived[kMaxRanksStatic];
   __shared__ unsigned s_seq;
@@ -69,13 +70,27 @@ __global__ void __launch_bounds__(kThreads, MINB) a2av_static_kernel(const __gri
   TraceBlock* tb = reinterpret_cast<TraceBlock*>(a.heap[a.proc] + a.lay.trace_off);
   dev::WaitCfg wc{&my->abort_flag, a.timeout_ns};
 
+  // Chunk d of those dealt: item `at` from byte `from` on.
+  auto locate = [&](unsigned d, unsigned& at, unsigned& from) {
+    at = d;
+    from = 0;
+    if (WIDE && d < a.wide) {
+      at = d >> a.wide_shift;
+      from = (d - (at << a.wide_shift)) * a.chunk;
+    } else if (WIDE) {
+      at = (a.wide >> a.wide_shift) + (d - a.wide);
+    }
+  };
   // The first items travel in the kernel parameters: the source of such an item is requested from memory before
   // anything else happens (with a call number that has to be read from memory, the two trips to DRAM overlap).
-  if (gwarp < a.nitems && gwarp < (unsigned)kInlineItems) {
-    const StaticItem& f = a.inl[gwarp];
-    if (!(f.flags & ITEM_SRC_STAGE))
-      for (unsigned off = lane * 128u; off < f.len; off += 32u * 128u)
+  if (gwarp < a.nitems) {
+    unsigned at, from;
+    locate(gwarp, at, from);
+    if (at < (unsigned)kInlineItems && !(a.inl[at].flags & ITEM_SRC_STAGE)) {
+      const StaticItem& f = a.inl[at];
+      for (unsigned off = from + lane * 128u; off < (WIDE ? min(f.len, from + a.chunk) : f.len); off += 32u * 128u)
         asm volatile("prefetch.global.L2 [%0];" ::"l"(f.src + off));
+    }
   }
   // The CTA that completes the start count advances the call number for the next call; the count's result is only
   // looked at when the CTA is done, so the atomic's round trip is off the path of the data.
@@ -99,9 +114,13 @@ __global__ void __launch_bounds__(kThreads, MINB) a2av_static_kernel(const __gri
   bool alive = true;
   unsigned ready = 1u << a.proc;   // processes known to have entered this call
   unsigned next = kNoFlag;         // the item that forwards what this warp has just stored
+  unsigned from = 0;               // first byte of its chunk, the same in every item of a chain
   for (unsigned dealt = gwarp; next != kNoFlag || dealt < a.nitems;) {
-    const unsigned c = next != kNoFlag ? next : dealt;
-    if (next == kNoFlag) dealt += nwarps;
+    unsigned c = next;
+    if (c == kNoFlag) {
+      locate(dealt, c, from);
+      dealt += nwarps;
+    }
     next = kNoFlag;
     union { uint4 q[2]; StaticItem it; } u;
     if (c < (unsigned)kInlineItems) {
@@ -137,9 +156,9 @@ __global__ void __launch_bounds__(kThreads, MINB) a2av_static_kernel(const __gri
       if (r != dev::WAIT_OK) { ok = false; alive = false; }
     }
     if (ok && it.len) {
-      const char* src = reinterpret_cast<const char*>(it.src) + ((it.flags & ITEM_SRC_STAGE) ? (size_t)parity * a.lay.arena_bytes : 0);
-      char* dst = reinterpret_cast<char*>(it.dst) + ((it.flags & ITEM_DST_STAGE) ? (size_t)parity * a.lay.arena_bytes : 0);
-      dev::warp_copy<MINB == 1 ? 8 : 4>(dst, src, it.len, lane);
+      const char* src = reinterpret_cast<const char*>(it.src) + from + ((it.flags & ITEM_SRC_STAGE) ? (size_t)parity * a.lay.arena_bytes : 0);
+      char* dst = reinterpret_cast<char*>(it.dst) + from + ((it.flags & ITEM_DST_STAGE) ? (size_t)parity * a.lay.arena_bytes : 0);
+      dev::warp_copy<MINB == 1 ? 8 : 4>(dst, src, WIDE ? min(it.len - from, a.chunk) : it.len, lane);
     }
     __syncwarp();   // (also orders these stores before the loads of the warp's other lanes, when it forwards them)
     if (it.flags & ITEM_NEXT) {
@@ -201,15 +220,16 @@ __global__ void __launch_bounds__(kThreads, MINB) a2av_static_kernel(const __gri
 cudaError_t a2av_static_configure(int occupancy, int* max_ctas_per_sm) {
   int nb = 0;
   cudaError_t e = occupancy >= 2
-      ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, a2av_static_kernel<2>, kThreads, 0)
-      : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, a2av_static_kernel<1>, kThreads, 0);
+      ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, a2av_static_kernel<2, true>, kThreads, 0)
+      : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, a2av_static_kernel<1, true>, kThreads, 0);
   if (max_ctas_per_sm) *max_ctas_per_sm = nb;
   return e;
 }
 
 cudaError_t a2av_static_launch(const StaticArgs& args, int grid, int occupancy, bool cooperative, cudaStream_t stream) {
   void* params[] = {(void*)&args};
-  const void* fn = occupancy >= 2 ? (const void*)a2av_static_kernel<2> : (const void*)a2av_static_kernel<1>;
+  const void* fn = args.wide ? (occupancy >= 2 ? (const void*)a2av_static_kernel<2, true> : (const void*)a2av_static_kernel<1, true>)
+                             : (occupancy >= 2 ? (const void*)a2av_static_kernel<2, false> : (const void*)a2av_static_kernel<1, false>);
   if (cooperative) return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kThreads), params, 0, stream);
   return cudaLaunchKernel(fn, dim3(grid), dim3(kThreads), params, 0, stream);
 }

@@ -742,3 +742,18 @@ def test_persistent_calls_name_the_kernel_that_runs_them():
         assert run_case(4, "spreadout", 4, counts, **kw).kind == "rendezvous"
     finally:
         comm.enable_trace(False)
+
+
+@pytest.mark.parametrize("P,algo,kw,top", [(8, "spreadout", {}, 900_000), (8, "ttpl_bt_s1", dict(n=4, r=2), 500_000),
+                                           (8, "rbruck", dict(r=2), 400_000), (32, "spreadout", {}, 48_000)])
+def test_persistent_items_of_several_chunks(P, algo, kw, top):
+    """One process, blocks of many chunks: an item stands for several chunks, which are dealt one by one.  Blocks that end
+    inside, at the end of and before most chunks of an item, empty and single-byte ones; direct and chained."""
+    rng = np.random.default_rng(P + top)
+    counts = rng.integers(top // 2, top, (P, P))
+    counts[0, :5] = [0, 1, 8192, 8193, 65536]
+    counts[1, :4] = [65535, 65537, 3 * 65536, 8191]
+    call = run_case(P, algo, 1, counts, packed=False, seed=top, persistent=True, launches=2, big_arena=P == 8, **kw)
+    assert call.kind == "static"
+    hops = 1 if algo == "spreadout" else 2
+    assert call.items <= hops * (int(counts.sum()) // 16384 + P * P)     # far fewer than one per 8 KB chunk
