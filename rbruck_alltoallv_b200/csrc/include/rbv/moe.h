@@ -19,7 +19,8 @@ extern "C" {
  *   group_start / group_rows: device int32[G].  N % 256 == 0, K % 64 == 0.
  *   epilogue 0: C is [*, N];  epilogue 1 (SwiGLU): B rows interleave gate and up (2j = gate_j, 2j+1 = up_j) and
  *   C is [*, N/2] with C[:, j] = silu(gate_j) * up_j.
- *   error_flag: device int, set non-zero if a bounded wait inside the kernel ran out.
+ *   error_flag: device int, set non-zero if a bounded wait inside the kernel ran out, to 6 if a group reaches beyond the
+ *   a_rows rows of A (those rows are left out).
  * Returns 0 or a CUDA error code. */
 int rbv_grouped_gemm_bf16(const void* A, long long a_rows, const void* B, void* C, const int* group_start,
                           const int* group_rows, int G, int N, int K, int ldc, int epilogue, int* error_flag,
@@ -162,7 +163,8 @@ int rbv_moe_combine_pushed(rbv_ctx_t ctx, void* out, int T, int H, const float* 
  * rbv_moe_route_local is rbv_moe_route and rbv_moe_layout_aligned in one launch, plus place [T, 2]: the index of every
  * routed row among its expert's rows, and hist, hist_all [E]: rows per expert, as router and gather leave them.
  * scratch [E + 1] ints, zeroed once, is left zero by every call.
- * rbv_moe_dispatch_local stores token t to rows slot[t][k] = dst_base[expert] + place[t][k] of `rows`; format 0: bf16,
+ * rbv_moe_dispatch_local stores token t to rows slot[t][k] = dst_base[expert] + place[t][k] of `rows` (beyond its
+ * capacity: dropped, slot 0, error 4 << 8 | expert); format 0: bf16,
  * 1: e4m3 with MXFP8 scale words in atom order [H / 128][capacity / 128][128] (as rbv_quantize_rows_mxfp8 makes them),
  * 2: e4m3 with fp32 scales [H / 128][capacity] (as rbv_quantize_rows_fp8).  ret (optional): token * 2 + k of every row.
  * rbv_moe_combine_local: out[t] = w[t][0] * y[slot[t][0]] + w[t][1] * y[slot[t][1]]; slot null: rows 2 t, 2 t + 1.

@@ -111,7 +111,7 @@ grouped_gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __
   if (warp == 1) { tmem_alloc_pair(&tmem_base_s, 512); tmem_relinquish_pair(); }
   pdl_trigger();
   pdl_wait();
-  for (int i = tid; i < p.G; i += blockDim.x) { s_rows[i] = p.group_rows[i]; s_start[i] = p.group_start[i]; }
+  for (int i = tid; i < p.G; i += blockDim.x) { s_start[i] = p.group_start[i]; s_rows[i] = rows_inside(p.group_rows[i], s_start[i], p.a_rows, p.error); }
   tc_fence_before_sync();
   __syncthreads();
   cluster_sync_all();

@@ -91,7 +91,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_
     s_abort = 0;
     mbar_fence_init();
   }
-  for (int i = tid; i < p.G; i += blockDim.x) { s_rows[i] = p.group_rows[i]; s_start[i] = p.group_start[i]; }
+  for (int i = tid; i < p.G; i += blockDim.x) { s_start[i] = p.group_start[i]; s_rows[i] = rows_inside(p.group_rows[i], s_start[i], p.a_rows, p.error); }
   if (warp == 1) { tmem_alloc(&tmem_base_s, 512); tmem_relinquish(); }
   tc_fence_before_sync();
   __syncthreads();

@@ -255,7 +255,7 @@ grouped_gemm_fp8_tok_kernel(const __grid_constant__ Fp8TokMaps maps, const __gri
   pdl_trigger();
   pdl_wait();
   for (int i = tid; i < p.G; i += blockDim.x) {
-    s_rows[i] = p.group_rows[i]; s_start[i] = p.group_start[i];
+    s_start[i] = p.group_start[i]; s_rows[i] = rows_inside(p.group_rows[i], s_start[i], p.a_rows, p.error);
     atomicMax(&s_most, s_rows[i]);
   }
   tc_fence_before_sync();

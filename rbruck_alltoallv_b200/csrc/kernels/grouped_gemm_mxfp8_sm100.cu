@@ -91,6 +91,7 @@ struct MxParams {
   const int* group_start;
   const int* group_rows;
   int G, N, K, ldc;
+  long long a_rows;            // rows of A
   int a_row_blocks;            // ceil(a_rows / 128): scale atoms of A per K block
   void* C;
   uint32_t* sf_out;            // epilogue 3: scale words of the quantised output, [N / 256][a_row_blocks][128]
@@ -232,7 +233,7 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ MxMaps maps, const __grid_cons
   pdl_trigger();
   pdl_wait();
   for (int i = tid; i < p.G; i += blockDim.x) {
-    s_rows[i] = p.group_rows[i]; s_start[i] = p.group_start[i];
+    s_start[i] = p.group_start[i]; s_rows[i] = rows_inside(p.group_rows[i], s_start[i], p.a_rows, p.error);
     if (s_rows[i] > 0 && (s_start[i] & 127)) s_bad = 1;   // the scale atoms of A would not coincide with the tiles
     atomicMax(&s_most, s_rows[i]);
     const int units = (s_rows[i] + XS - 1) / XS;
@@ -605,7 +606,7 @@ static int launch_mxfp8(const void* A, const void* sfa, long long a_rows, const 
   if (!make_map_atoms(&maps.sfw, sfb, (unsigned long long)G * nkb * (unsigned long long)(N / 128))) return (int)cudaErrorUnknown;
   MxParams p;
   p.group_start = group_start; p.group_rows = group_rows; p.G = G; p.N = N; p.K = K; p.ldc = ldc;
-  p.a_row_blocks = (int)nrb;
+  p.a_rows = a_rows; p.a_row_blocks = (int)nrb;
   p.C = C; p.sf_out = static_cast<uint32_t*>(sf_out); p.error = error_flag; p.epilogue = epilogue;
   p.ret = ret; p.y2_off = y2_off;
   for (int q = 0; q < 16; q++) p.heap[q] = (ret && q < nheaps) ? static_cast<char*>(const_cast<void*>(heaps[q])) : nullptr;

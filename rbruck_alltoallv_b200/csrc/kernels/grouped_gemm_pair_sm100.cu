@@ -64,6 +64,7 @@ struct PairParams {
   int G;
   int N, K;
   int ldc;
+  long long a_rows;
   void* C;
   int* error;
   int epilogue;   // 0: C = bf16(acc); 1: C[:, j] = bf16(silu(acc[:, 2j]) * acc[:, 2j+1])
@@ -135,7 +136,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ PairMaps maps, const __grid_con
   pdl_trigger();
   pdl_wait();
   for (int i = tid; i < p.G; i += blockDim.x) {
-    s_rows[i] = p.group_rows[i]; s_start[i] = p.group_start[i];
+    s_start[i] = p.group_start[i]; s_rows[i] = rows_inside(p.group_rows[i], s_start[i], p.a_rows, p.error);
     atomicMax(&s_most, s_rows[i]);
   }
   tc_fence_before_sync();
@@ -327,7 +328,7 @@ static int launch_bf16_pair(const void* A, long long a_rows, const void* B, void
     if (!pair_make_map(&maps.tok[i], A, (unsigned long long)a_rows, (unsigned long long)K, 16u << i)) return (int)cudaErrorUnknown;
   PairParams p;
   p.group_start = group_start; p.group_rows = group_rows; p.G = G; p.N = N; p.K = K; p.ldc = ldc; p.C = C;
-  p.error = error_flag; p.epilogue = epilogue;
+  p.a_rows = a_rows; p.error = error_flag; p.epilogue = epilogue;
   p.ret = ret; p.y2_off = y2_off;
   for (int q = 0; q < 16; q++) p.heap[q] = (ret && q < nheaps) ? static_cast<char*>(const_cast<void*>(heaps[q])) : nullptr;
   int grid = max_ctas;

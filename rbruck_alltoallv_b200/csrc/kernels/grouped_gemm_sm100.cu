@@ -44,6 +44,7 @@ struct GemmParams {
   const int* group_rows;    // [G] rows of each group
   int G;
   int N, K;                 // B_g is N x K
+  long long a_rows;         // rows of A
   int ldc;                  // elements between rows of C
   void* C;                  // bf16
   int* error;               // set to non-zero when a wait ran out
@@ -120,7 +121,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
     s_abort = 0;
     mbar_fence_init();
   }
-  for (int i = tid; i < p.G; i += blockDim.x) { s_rows[i] = p.group_rows[i]; s_start[i] = p.group_start[i]; }
+  for (int i = tid; i < p.G; i += blockDim.x) { s_start[i] = p.group_start[i]; s_rows[i] = rows_inside(p.group_rows[i], s_start[i], p.a_rows, p.error); }
   if (warp == 1) { tmem_alloc(&tmem_base_s, TMEM_COLS); tmem_relinquish(); }
   tc_fence_before_sync();
   __syncthreads();
@@ -324,7 +325,7 @@ extern "C" int rbv_grouped_gemm_bf16_gated(const void* A, long long a_rows, cons
   if (!make_map(&mb, B, (unsigned long long)G * N, (unsigned long long)K, BN)) return (int)cudaErrorUnknown;
   GemmParams p;
   p.group_start = group_start; p.group_rows = group_rows; p.G = G; p.N = N; p.K = K; p.ldc = ldc; p.C = C;
-  p.error = error_flag; p.epilogue = epilogue;
+  p.a_rows = a_rows; p.error = error_flag; p.epilogue = epilogue;
   p.ready = ready; p.ready_target = ready ? ready_target : nullptr;
   p.timeout_ns = (unsigned long long)((timeout_ms > 0 ? timeout_ms : 2000.0) * 1e6);
   int grid = max_ctas;

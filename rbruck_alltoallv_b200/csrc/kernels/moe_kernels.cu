@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(kMoeThreads) moe_dispatch_kernel(const __grid_
     int pos = 0;
     if (lane == 0) pos = a.dst_base[e] + atomicAdd(&a.cursor[e], 1);
     pos = __shfl_sync(0xffffffffu, pos, 0);
-    if (lane == 0) a.slot[r] = pos;
+    if (lane == 0) a.slot[r] = pos < a.capacity_rows ? pos : 0;   // (a dropped row: some row that the combine can read)
     if (pos >= a.capacity_rows) { if (lane == 0) moe_fail(c, 4, e); continue; }
     const int owner = e / a.El;
     char* dst = c.heap[owner] + a.xrecv_off + (size_t)pos * row_bytes;
@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(kMoeThreads, 2) moe_dispatch_mx_kernel(const _
     int pos = 0;
     if (lane == 0) pos = a.dst_base[e] + atomicAdd(&a.cursor[e], 1);
     pos = __shfl_sync(0xffffffffu, pos, 0);
-    if (lane == 0) a.slot[r] = pos;
+    if (lane == 0) a.slot[r] = pos < a.capacity_rows ? pos : 0;   // (a dropped row: some row that the combine can read)
     if (pos >= a.capacity_rows) { if (lane == 0) moe_fail(c, 4, e); continue; }
     const int owner = e / a.El;
     if (a.ret_off && lane == 0)
@@ -468,7 +468,7 @@ __global__ void __launch_bounds__(kMoeThreads) moe_dispatch_streamed_kernel(cons
     const int e = a.topk_idx[r];
     const int pos = a.dst_base[e] + (i - a.loc_off[e]);
     const int owner = e / a.El;
-    if (lane == 0) a.slot[r] = pos;
+    if (lane == 0) a.slot[r] = pos < a.capacity_rows ? pos : 0;   // (a dropped row: some row that the combine can read)
     if (pos < a.capacity_rows)
       dev::warp_copy(c.heap[owner] + a.xrecv_off + (size_t)pos * row_bytes, a.x + (size_t)(r >> 1) * row_bytes, row_bytes, lane);
     else if (lane == 0) moe_fail(c, 4, e);

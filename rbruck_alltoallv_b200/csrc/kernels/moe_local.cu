@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(128) moe_dispatch_local_kernel(const __grid_co
   const bool fits[2] = {pos[0] < a.capacity, pos[1] < a.capacity};
   if (seg == 0 && lane < 2) {
     const int k = lane;
-    a.slot[2 * t + k] = k ? pos[1] : pos[0];
+    a.slot[2 * t + k] = (k ? fits[1] : fits[0]) ? (k ? pos[1] : pos[0]) : 0;   // (a dropped row: some row the combine can read)
     if (!(k ? fits[1] : fits[0])) atomicCAS(a.error, 0, (4 << 8) | ((k ? e.y : e.x) & 0xff));
     else if (a.ret) a.ret[k ? pos[1] : pos[0]] = (unsigned)(2 * t + k);
   }

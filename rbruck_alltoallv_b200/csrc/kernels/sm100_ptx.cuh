@@ -213,5 +213,14 @@ __host__ __device__ constexpr uint32_t umma_idesc(int M, int N, int ab_format /*
          ((uint32_t)(M >> 4) << 24);
 }
 
+// Rows of a group that lie inside A.  An expert may be routed more rows than its GPU has room for: the dispatch drops them,
+// but they are counted, and what lies behind the last row of A belongs to somebody else, in C and in the table of return
+// addresses too.  Recorded as error 6.
+__device__ __forceinline__ int rows_inside(int rows, int start, long long a_rows, int* error) {
+  const int inside = (int)max(0ll, min((long long)rows, a_rows - start));
+  if (inside < rows && error && blockIdx.x == 0) atomicCAS(error, 0, 6);
+  return inside;
+}
+
 }  // namespace sm100
 }  // namespace rbv

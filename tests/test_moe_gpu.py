@@ -665,3 +665,53 @@ def test_moe_fp8_one_rank_needs_no_bf16_receive_buffer():
     # e4m3 operands in two GEMMs against the unquantised weights: the bound of the layer's own test
     assert (out.float() - ref).norm().item() <= 0.08 * ref.norm().item()
     comm.close()
+
+
+@pytest.mark.parametrize("push", [True, False], ids=["push", "pull"])
+@pytest.mark.parametrize("fp8,pair", [(False, True), (False, False), (True, True), (True, False), ("mx", True)])
+def test_moe_layer_drops_what_does_not_fit(fp8, pair, push):
+    """More routed rows than the receive buffer holds: an error is recorded, tokens whose rows fit get their result, and
+    nothing behind the layer's buffers is touched."""
+    from rbruck_alltoallv_b200 import _native
+    from rbruck_alltoallv_b200.ops.moe import MoEExpertParallel
+    from rbruck_alltoallv_b200.parallel.comm import Communicator
+    T, H, I, E = 700, 512, 256, 4
+    lib = _native.cuda_lib()
+    comm = Communicator(nranks=1, heap_bytes=128 << 20, arena_bytes=1 << 20)
+    torch.manual_seed(1)
+    x, logits = torch.randn(T, H, device="cuda").to(torch.bfloat16), torch.randn(T, E, device="cuda")
+    before = lib.rbv_grouped_gemm_pair_enabled()
+    lib.rbv_grouped_gemm_set_pair(1 if pair else 0)
+    try:
+        whole = MoEExpertParallel(comm, E, H, I, T, seed=6, fp8=fp8, push_combine=push)
+        want = whole.forward(x, logits)
+        whole.check()
+        layer = MoEExpertParallel(comm, E, H, I, T, seed=6, fp8=fp8, push_combine=push, capacity_factor=0.4)
+        cap, spare = layer.cap, 2 * T
+        assert cap < 2 * T
+        room = {"h": torch.full((cap + spare, I), 7.0, dtype=torch.bfloat16, device="cuda")}
+        layer.h = room["h"][:cap]
+        if not layer.push:
+            room["y"] = comm.symm_empty((cap + spare, H), torch.bfloat16)
+            room["y"].fill_(7.0)
+            layer.y = room["y"][:cap]
+            layer.y_off = layer.y.data_ptr() - lib.rbv_ctx_heap(comm._ctx, 0)
+        if fp8 == "mx":
+            room["hq"] = torch.full((cap + spare, I), 7, dtype=torch.uint8, device="cuda")
+            layer._hq = room["hq"][:cap]
+            layer._hs = torch.empty(I // 128, cap, dtype=torch.int32, device="cuda")
+        out = layer.forward(x, logits)
+        torch.cuda.synchronize()
+        assert layer.error[0].item() >> 8 == 4
+        with pytest.raises(RuntimeError, match="dispatch"):
+            layer.check()
+        for name, t in room.items():
+            assert torch.all(t[cap:] == 7), name
+        rows = layer.dst_base.long()[layer.topk_idx.long()] + layer.place.long()
+        fits = (rows < cap).all(dim=1)
+        assert 0 < int(fits.sum()) < T
+        # the same products in the same order whatever the tile is; bf16 rounding at most
+        assert ((out[fits].float() - want[fits].float()).abs() <= 2.0 ** -7 * want[fits].float().abs() + 1e-3).all()
+    finally:
+        lib.rbv_grouped_gemm_set_pair(before)
+        comm.close()
