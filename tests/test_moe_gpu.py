@@ -715,3 +715,59 @@ def test_moe_layer_drops_what_does_not_fit(fp8, pair, push):
     finally:
         lib.rbv_grouped_gemm_set_pair(before)
         comm.close()
+
+
+def _fp8_pair_operands(rows, N, K, seed):
+    """Operands with so many unused rows behind the groups that the CTA-pair kernel with tokens as M takes them
+    (a_rows > 384 per group)."""
+    from rbruck_alltoallv_b200.ops import moe
+    torch.manual_seed(seed)
+    G, M = len(rows), 384 * len(rows) + 1 + sum(rows)
+    Aq, sa = moe.quantize_rows_fp8((torch.randn(M, K, device="cuda") * torch.rand(M, 1, device="cuda") * 3).to(torch.bfloat16))
+    Bq, sb = moe.quantize_weight_blocks_fp8(torch.randn(G, N, K, device="cuda") * 0.1)
+    gs, gr = _groups(rows, "cuda")
+    return M, Aq, sa, Bq, sb, gs, gr
+
+
+@pytest.mark.parametrize("coarse", [False, True])
+@pytest.mark.parametrize("rows,N", [([1], 128), ([100, 37, 0, 300], 128), ([0, 255, 256, 257], 384), ([513, 64], 256)])
+def test_grouped_gemm_fp8_pair_kernel_with_few_rows(rows, N, coarse):
+    """The kernel for many rows per group on small, ragged and empty groups and a single column tile, with scales per K block
+    and with scales that are constant along K.  Exact after quantisation: bf16 rounding plus fp32 sums of K = 512 products."""
+    from rbruck_alltoallv_b200.ops import moe
+    K = 512
+    M, Aq, sa, Bq, sb, gs, gr = _fp8_pair_operands(rows, N, K, sum(rows) + N)
+    if coarse:
+        sa, sb = sa[:1].expand_as(sa).contiguous(), sb[:, :, :1].expand_as(sb).contiguous()
+    A, B = moe.dequantize_rows_fp8(Aq, sa).double(), moe.dequantize_weight_blocks_fp8(Bq, sb).double()
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    out = torch.full((M, N), 7.0, dtype=torch.bfloat16, device="cuda")
+    moe.grouped_gemm_fp8(Aq, sa, Bq, sb, gs, gr, out=out, error=err, coarse=coarse, pair=True)
+    torch.cuda.synchronize()
+    assert err.item() == 0 and torch.all(out[sum(rows):] == 7.0)
+    r0 = 0
+    for g, n in enumerate(rows):
+        ref = A[r0:r0 + n] @ B[g].t()
+        slack = (A[r0:r0 + n].abs() @ B[g].abs().t()) * K * 2.0 ** -24
+        assert ((out[r0:r0 + n].double() - ref).abs() <= ref.abs() * 2.0 ** -8 + slack + 1e-6).all(), f"group {g}"
+        r0 += n
+
+
+def test_moe_layer_fp8_many_rows_per_expert():
+    """A layer whose buffer has more than 384 rows per expert: both GEMMs run the kernel for many rows, behind the one-rank
+    dispatch, passes in a row."""
+    from rbruck_alltoallv_b200.ops.moe import MoEExpertParallel, reference_forward
+    from rbruck_alltoallv_b200.parallel.comm import Communicator
+    T, H, I, E = 500, 512, 384, 2
+    comm = Communicator(nranks=1, heap_bytes=64 << 20, arena_bytes=1 << 20)
+    layer = MoEExpertParallel(comm, E, H, I, T, seed=8, fp8=True)
+    assert layer.cap > 384 * E
+    torch.manual_seed(8)
+    xs = [torch.randn(T, H, device="cuda").to(torch.bfloat16) for _ in range(3)]
+    logits = [torch.randn(T, E, device="cuda") for _ in range(3)]
+    outs = [layer.forward(x, l) for x, l in zip(xs, logits)]
+    layer.check()
+    for x, l, out in zip(xs, logits, outs):
+        ref, _, _ = reference_forward(x, l, layer.w13, layer.w2)
+        assert (out.float() - ref).norm().item() <= 0.08 * ref.norm().item()   # e4m3 operands, as the layer's own test
+    comm.close()
