@@ -47,6 +47,7 @@ Context::Context(int P, int nproc, int proc, int device, size_t user_bytes, size
   if (const char* e = std::getenv("RBV_COOPERATIVE")) cooperative_mode_ = std::atoi(e) != 0 ? 1 : 0;
   if (const char* e = std::getenv("RBV_STATIC_OCC")) static_occ_ = std::atoi(e) >= 2 ? 2 : 1;
   if (const char* e = std::getenv("RBV_STATIC_SPREAD")) static_spread_ = std::atoi(e) != 0;
+  if (const char* e = std::getenv("RBV_STATIC_CHAINS")) static_chains_ = std::atoi(e) != 0;
   if (const char* e = std::getenv("RBV_EAGER_SPREAD")) eager_spread_ = std::atoi(e);
   if (const char* e = std::getenv("RBV_SEQ_HINT")) seq_hints_ = std::atoi(e) != 0;
   int st_per_sm = 1;
@@ -740,7 +741,7 @@ int Context::prepare_static(const DevPlan* dp, int ts, const CallArgs& ca, const
     if (first_el) *first_el = f;
     return (unsigned long long)n * ts;
   };
-  const bool relay = !dp->pred.empty();   // one process: a warp forwards what it stored itself, see find_chains
+  const bool relay = static_chains_ && !dp->pred.empty();   // one process: a warp forwards what it stored, see find_chains
   // ---- the slice of every op of this process ----
   struct Slice { unsigned long long bytes; long long first; unsigned n, wide, at, wide_at; };
   const std::vector<Op>& ops = dp->h_ops;

@@ -205,6 +205,8 @@ class Context {
   int eager_spread_ = 0;           // eager calls with a prepared item table: one CTA per item (RBV_EAGER_SPREAD=1);
                                    // off: measured on 2 GPUs it cost 1-2 us per call (16.8 against 15.0 us)
   bool static_spread_ = true;      // few items: one per CTA over many SMs instead of 16 per CTA on few (RBV_STATIC_SPREAD=0)
+  bool static_chains_ = true;      // one process: a warp forwards what it stored (RBV_STATIC_CHAINS=0: flags between the
+                                   // hops, as across processes)
   int prepare_static(const DevPlan* dp, int type_size, const CallArgs& args, const CallOptions& opt, Prepared* out);
   std::string last_error_;
   std::map<std::tuple<int, int, int, int, int, int, int>, std::unique_ptr<DevPlan>> plans_;

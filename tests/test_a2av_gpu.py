@@ -757,3 +757,22 @@ def test_persistent_items_of_several_chunks(P, algo, kw, top):
     assert call.kind == "static"
     hops = 1 if algo == "spreadout" else 2
     assert call.items <= hops * (int(counts.sum()) // 16384 + P * P)     # far fewer than one per 8 KB chunk
+
+
+def test_static_kernel_raises_and_waits_for_chunk_flags(monkeypatch):
+    """What a relay of several processes runs, on one GPU: with chains switched off every hop waits for the flag of its chunk.
+    Blocks of several chunks, empty ones, both parities of the staging cells."""
+    from rbruck_alltoallv_b200.parallel.comm import Communicator
+    monkeypatch.setenv("RBV_STATIC_CHAINS", "0")
+    monkeypatch.setitem(_comms, (8, True), Communicator(nranks=8, heap_bytes=256 << 20, arena_bytes=24 << 20))
+    monkeypatch.delenv("RBV_STATIC_CHAINS")
+    try:
+        counts = dist.normal(8, 120_000, seed=2)
+        counts[2, 5] = counts[5, 2] = 0
+        for algo, kw in (("rbruck", dict(r=2)), ("tuna2", dict(r=3, b=1)), ("ttpl_bt_s1", dict(n=4, r=2)), ("merge", dict(n=4))):
+            for chunk in (16 << 10, 0):
+                call = run_case(8, algo, 4, counts, seed=3, persistent=True, launches=3, chunk_bytes=chunk, big_arena=True, **kw)
+                assert call.kind == "static"
+                assert call.cooperative == (call.items > call.grid * 16)     # somebody waits
+    finally:
+        _comms[(8, True)].close()
