@@ -7,8 +7,8 @@
 // the table until it is complete, walks an op list and counts arrivals; and a host that does not know the counts has to
 // give it one chunk size for every call.  Here the chunk follows from the bytes that the call moves, so that they spread
 // over all warps whatever the host knew.  Measured on one B200 (cold caches): counts on the device, 16 ranks, 17 MB in
-// blocks of up to 64 KB 29 -> 11.5 us; 1 MB in blocks of up to 16 KB among 8 ranks 12.7 -> 9.2 us.  Long blocks: 16
-// vectors per lane in flight 4.6 TB/s, 8 vectors 4.25.
+// blocks of up to 64 KB 29 -> 11.5 us; 1 MB in blocks of up to 16 KB among 8 ranks 12.7 -> 9.2 us; 256 MB in
+// blocks of up to 4 MB 124 -> 98 us (5.2 TB/s; 16 vectors per lane in flight move them 7 % faster than 8).
 #include <cuda_runtime.h>
 
 #include "kernels/primitives.cuh"
@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(kLocalThreads, 1) a2av_local_kernel(const __gr
   for (int w = 0; w < kLocalThreads / 32; w++) total += s_sum[w];
 
   // A chunk is one warp's unit of work: the bytes of the call over the warps of the grid, in a whole number of rounds of
-  // at most 64 KB, and at least 2 KB (one round of loads of a warp is 4 KB).
+  // at most 64 KB, and at least 2 KB (four vectors per lane; a warp's round of loads is 16, 8 KB).
   const unsigned nwarps = gridDim.x * (kLocalThreads / 32);
   unsigned long long chunk = a.chunk_bytes;
   if (!chunk) {

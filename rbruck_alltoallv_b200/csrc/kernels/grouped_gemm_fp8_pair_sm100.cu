@@ -357,11 +357,14 @@ extern "C" int rbv_grouped_gemm_fp8_pair(const void* A, const float* a_scale_t, 
                                          int G, int N, int K, int ldc, int epilogue, int* error_flag, int max_ctas,
                                          void* cuda_stream) {
   using namespace rbv;
-  // Few tokens per group: tokens as the N operand (grouped_gemm_fp8_tok_sm100.cu).  Only the device knows the groups'
-  // rows; the host knows the rows of A, of which the MoE layer, whose buffer is sized for twice the average load, uses
-  // half.  Measured on one B200, 8 experts, hidden 4096, FFN 14336, up / down GEMM, this kernel against that one:
-  // 25 rows per expert 314 / 222 against 170 / 100 us, 125 rows 333 / 222 against 274 / 144, 250 rows 410 / 261 against
-  // 405 / 188, 500 rows 669 / 372 against 757 / 368.
+  // Few tokens per group: tokens as the N operand (grouped_gemm_fp8_tok_sm100.cu).  Only the device knows the groups' rows;
+  // the host knows the rows of A and draws the line there.  Measured on one B200, 8 experts, hidden 4096, FFN 14336, up plus
+  // down GEMM in us, that kernel (tiles of up to 128 tokens) / this one (tiles of 256), by rows per expert:
+  //   64: 276 / 534    128: 334 / 545    150: 506 / 545    192: 498 / 553    250: 581 / 558
+  //   300: 756 / 1011  350: 883 / 1024   383: 938 / 1024   1500, 600, ... 20: 963 / 963   all 1536 in one expert: 494 / 410
+  // So with A sized to the rows in use the line costs 4 % where the groups just fit this kernel's tile.  The MoE layer sizes A
+  // for twice the average load: its experts get this kernel from 192 rows on, which is right up to 256 and not between 257 and
+  // 384.  Routing that sends everything to one or two experts costs that kernel 17 to 20 %; a_rows does not show it.
   if (a_rows <= 384ll * G)
     return rbv_grouped_gemm_fp8_tok(A, a_scale_t, a_rows, B, b_scale, C, group_start, group_rows, G, N, K, ldc, epilogue,
                                     error_flag, max_ctas, cuda_stream);

@@ -7,9 +7,12 @@
                                                                    # chunk-granular forwarding)
     python -m rbruck_alltoallv_b200.utils.profile_case a2av_dynamic  # the same spread-out exchange through the kernel
                                                                    # that exchanges metadata itself
+    python -m rbruck_alltoallv_b200.utils.profile_case a2av_local  # the same exchange with counts on the device (local kernel)
     python -m rbruck_alltoallv_b200.utils.profile_case a2av_small  # Zipf blocks <= 64 KB (latency regime)
     python -m rbruck_alltoallv_b200.utils.profile_case gemm1       # grouped SwiGLU GEMM, 2 experts x 2048 rows, 4096 -> 2 x 14336
     python -m rbruck_alltoallv_b200.utils.profile_case gemm2       # grouped down GEMM, 14336 -> 4096
+    python -m rbruck_alltoallv_b200.utils.profile_case gemm_fp8    # block-scaled fp8 up/gate GEMM, the same rows
+    python -m rbruck_alltoallv_b200.utils.profile_case gemm_fp8_few  # 8 experts x 128 rows, 4096 -> 2 x 4096 (tokens as N)
     python -m rbruck_alltoallv_b200.utils.profile_case gemm_mx     # MXFP8 up/gate GEMM, SwiGLU + quantiser epilogue
     python -m rbruck_alltoallv_b200.utils.profile_case moe_mx      # MoE layer with MXFP8 experts (quantising dispatch, pushed combine)
     python -m rbruck_alltoallv_b200.utils.profile_case transpose   # fused pencil transpose, 384^3 complex64
@@ -49,7 +52,11 @@ def _a2av(algo, small=False, **kw):
     recv = [comm.symm_empty(max(int(rc[i].sum()), 1), torch.float32) for i in range(P)]
     if kw.pop("eager", False):
         kw["eager_max_bytes"] = comm.max_block_bytes(sc, 4)
-    call = comm.prepare(send, recv, sc, None, rc, None, algo=algo, **kw)
+    args = (sc, None, rc, None)
+    if kw.pop("device", False):
+        sd, rd = (np.cumsum(a, axis=1, dtype=np.int64) - a for a in (sc, rc))
+        args = tuple(torch.from_numpy(a).cuda() for a in (sc, sd, rc, rd))
+    call = comm.prepare(send, recv, *args, algo=algo, **kw)
     for _ in range(4):
         call.launch()
     comm.check()
@@ -76,15 +83,16 @@ def _gemm(which):
     assert err.item() == 0
 
 
-def _gemm_fp8():
+def _gemm_fp8(G=2, rows=2048, I=14336):
     from ..ops.moe import grouped_gemm_fp8, quantize_rows_fp8, quantize_weight_blocks_fp8
-    G, rows, H, I = 2, 2048, 4096, 14336
-    gs = torch.tensor([0, rows], dtype=torch.int32, device="cuda")
-    gr = torch.tensor([rows, rows], dtype=torch.int32, device="cuda")
+    H = 4096
+    gs = torch.arange(G, dtype=torch.int32, device="cuda") * rows
+    gr = torch.full_like(gs, rows)
     err = torch.zeros(1, dtype=torch.int32, device="cuda")
     Aq, a_sc = quantize_rows_fp8(torch.randn(G * rows, H, device="cuda").to(torch.bfloat16))
     Bq, b_sc = quantize_weight_blocks_fp8((torch.randn(G, 2 * I, H, device="cuda") * 0.02).to(torch.bfloat16))
     out = torch.empty(G * rows, I, dtype=torch.bfloat16, device="cuda")
+    torch.cuda.empty_cache()
     for _ in range(4):
         grouped_gemm_fp8(Aq, a_sc, Bq, b_sc, gs, gr, out=out, swiglu=True, error=err)
     torch.cuda.synchronize()
@@ -128,6 +136,8 @@ def main() -> int:
         _a2av("rbruck", r=2)
     elif case == "a2av_dynamic":
         _a2av("spreadout", static=False)
+    elif case == "a2av_local":
+        _a2av("spreadout", device=True)
     elif case == "a2av_small":
         _a2av("rbruck", small=True, r=2)
     elif case == "gemm1":
@@ -136,6 +146,8 @@ def main() -> int:
         _gemm(2)
     elif case == "gemm_fp8":
         _gemm_fp8()
+    elif case == "gemm_fp8_few":
+        _gemm_fp8(G=8, rows=128, I=4096)
     elif case == "gemm_mx":
         _gemm_mx()
     elif case == "transpose":
