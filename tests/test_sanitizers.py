@@ -45,3 +45,19 @@ def test_device_byte_copy_stays_inside_its_block(tmp_path):
     its rounds, each load touches the source block, each store lies inside the destination, and the bytes are right."""
     out = _build_and_run(tmp_path, "warp_copy", [ROOT / "tests" / "native" / "warp_copy_main.cpp"], [], [CSRC])
     assert " 0 bad" in out
+
+
+def test_static_tables_deliver_every_block(tmp_path):
+    """Every schedule resolved for one, two and four processes against a stand-in for the CUDA runtime, and its items executed
+    on the host: chains, flags between hops, wide items, chunk sizes given and chosen."""
+    from rbruck_alltoallv_b200.parallel.plan import ALGOS
+    include = Path("/usr/local/cuda/include")
+    if not (include / "cuda_runtime.h").exists():
+        pytest.skip("needs the CUDA headers")
+    exe = tmp_path / "static_table"
+    b = subprocess.run(["g++", "-std=c++17", "-O1", "-g", f"-I{include}", f"-I{CSRC / 'include'}", f"-I{CSRC}",
+                        str(ROOT / "tests" / "native" / "static_table_main.cpp"), "-x", "c++", str(CSRC / "comm" / "comm.cu"),
+                        str(CSRC / "plan" / "plan.cpp"), "-o", str(exe)], capture_output=True, text=True)
+    assert b.returncode == 0, b.stderr[-2000:]
+    r = subprocess.run([str(exe), str(len(ALGOS))], capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0 and " 0 bad" in r.stdout, (r.stdout[-1500:], r.stderr[-1500:])
